@@ -66,7 +66,7 @@ struct DeviceBasis {
     unsigned short *ellPair = nullptr, *ellIdx = nullptr;
     double *ellVal = nullptr;
     int *ellOff = nullptr;
-    int ellChunks = 0, ellRows = 0;
+    int ellChunks = 0, ellGroups = 0;
     // row 0 of the Gaunt contraction (CSR rows (0, j), layout columns) and
     // the eigenvalue bounds of the quadrature Gram matrix of the moment basis
     int *r0off = nullptr;
@@ -324,20 +324,20 @@ cudaError_t build_device_basis(DeviceBasis &B, int n, int n2, int nq, int useGau
         if ((e = upload(&B.hoff, off)) != cudaSuccess) return e;
         if ((e = upload(&B.hidx, idx)) != cudaSuccess) return e;
         if ((e = upload(&B.hval, val)) != cudaSuccess) return e;
-        const int chunks = gaunt_ell_chunks(n), maxRows = 32 * chunks * 64;
-        std::vector<unsigned short> epair(chunks * 32), eidx((size_t)maxRows * 32);
-        std::vector<double> eval((size_t)maxRows * 32);
+        const int chunks = gaunt_ell_chunks(n), maxGroups = 16 * chunks;
+        std::vector<unsigned short> epair(chunks * 64), eidx((size_t)maxGroups * kEllGroup);
+        std::vector<double> eval((size_t)maxGroups * kEllGroup);
         std::vector<int> eoff(chunks + 1);
-        int rows2 = build_gaunt_ell(n, goff, gidx, gval, epair.data(), eidx.data(), eval.data(), eoff.data(),
-                                    maxRows);
-        if (rows2 < 0)
+        const int groups = build_gaunt_ell(n, goff, gidx, gval, epair.data(), eidx.data(), eval.data(), eoff.data(),
+                                           maxGroups);
+        if (groups < 0)
             return cudaErrorInvalidValue;
-        eidx.resize((size_t)rows2 * 32);
-        eval.resize((size_t)rows2 * 32);
+        eidx.resize((size_t)groups * kEllGroup);
+        eval.resize((size_t)groups * kEllGroup);
         for (auto &x : eidx)   // G columns in the layout's order
             x = (unsigned short)colH[x];
         B.ellChunks = chunks;
-        B.ellRows = rows2;
+        B.ellGroups = groups;
         // pairs (0, j) are the Gaunt table's rows j = 0 .. n-1 (row i n + j, i <= j)
         std::vector<int> r0off(n + 1);
         std::vector<unsigned short> r0idx;
@@ -441,7 +441,7 @@ NewtonProblem make_problem(const DeviceBasis &B)
     pb.ellVal = B.ellVal;
     pb.ellOff = B.ellOff;
     pb.ellChunks = B.ellChunks;
-    pb.ellRows = B.ellRows;
+    pb.ellGroups = B.ellGroups;
     pb.p0 = B.p0;
     pb.row0Off = B.r0off;
     pb.row0Idx = B.r0idx;
@@ -476,7 +476,7 @@ static NewtonProblem make_screen_problem(const DeviceBasis &B)
     pb.ellPair = pb.ellIdx = nullptr;
     pb.ellVal = nullptr;
     pb.ellOff = nullptr;
-    pb.ellChunks = pb.ellRows = 0;
+    pb.ellChunks = pb.ellGroups = 0;
     return pb;
 }
 
@@ -735,7 +735,7 @@ int cl_create(const cl_grid *grid, const cl_options *opts, const cl_angular *ang
     if (opts->moment_type == CL_MN && opts->precision == CL_FP64 && opts->contraction == CL_CONTRACT_PAIRS) {
         int pnt = 0, pnbk = 0;
         paired_counts(ang->n, ang->n2, gauntNewton, pnt, pnbk);
-        paired = newton_pair_supported(pnt, pnbk) ? 1 : 0;
+        paired = newton_pair_supported(pnt, pnbk, ang->n) ? 1 : 0;
     }
     // the flux kernel takes direction pairs for either closure
     const int fluxPaired = opts->contraction == CL_CONTRACT_PAIRS ? 1 : 0;
@@ -1503,7 +1503,7 @@ static int ensure_alt_basis(cl_ctx *ctx)
     if (ctx->opt.moment_type == CL_MN && ctx->opt.precision == CL_FP64 && !ctx->B.paired) {
         int pnt = 0, pnbk = 0;
         paired_counts(ctx->angN, ctx->angN2, ctx->angGaunt, pnt, pnbk);
-        paired = newton_pair_supported(pnt, pnbk) ? 1 : 0;
+        paired = newton_pair_supported(pnt, pnbk, ctx->angN) ? 1 : 0;
     }
     const int fluxPaired = ctx->B.fluxPaired ? 0 : 1;
     cudaError_t e = build_device_basis(ctx->B2, ctx->angN, ctx->angN2, ctx->angNq, ctx->angGaunt, ctx->aw.data(),

@@ -30,11 +30,19 @@ __device__ __constant__ const double kRegularizations[kNumReg] = {0.0, 1e-3, 1e-
 __device__ __forceinline__ void dmma16x8x8(double (&c)[4], double a0, double a1, double a2,
                                            double a3, double b0, double b1)
 {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
         "{%8,%9}, {%0,%1,%2,%3};\n"
         : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
         : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
+}
+
+// FP64 MMA m8n8k4: a A[g][t], b B[t][g], c0 C[g][2t], c1 C[g][2t+1].
+__device__ __forceinline__ void dmma8x8x4(double (&c)[2], double a, double b)
+{
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
 }
 
 // TF32 tensor-core MMA m16n8k8 with FP32 accumulation: the same fragment
@@ -82,6 +90,10 @@ __device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned
     asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}\n" ::"r"(smem_u32(bar)),
                  "r"(bytes)
                  : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long *bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned parity)
 {

@@ -2,6 +2,8 @@
 // dual-Newton kernel (device code in newton_kernel.cuh).
 #include "newton.cuh"
 
+#include "angular.h"
+
 #include <cfloat>
 #include <cmath>
 
@@ -9,10 +11,10 @@ namespace clb {
 
 int plan_newton(NewtonArgs &a)
 {
-    int nbMax = 8, ldPMax = 0, K2tot = 0, nMax = 1, ellRows = 0, ellChunks = 0;
+    int nbMax = 8, ldPMax = 0, K2tot = 0, nMax = 1, ellGroups = 0, ellChunks = 0;
     for (int p = 0; p < a.nprob; p++) {
         const NewtonProblem &pb = a.prob[p];
-        ellRows = pb.ellRows > ellRows ? pb.ellRows : ellRows;
+        ellGroups = pb.ellGroups > ellGroups ? pb.ellGroups : ellGroups;
         ellChunks = pb.ellChunks > ellChunks ? pb.ellChunks : ellChunks;
         nbMax = pb.nb > nbMax ? pb.nb : nbMax;
         ldPMax = pb.ldP > ldPMax ? pb.ldP : ldPMax;
@@ -25,7 +27,13 @@ int plan_newton(NewtonArgs &a)
     if (a.nw != kWarps && a.nw != 4)
         return -1;
     const int nw = a.nw;
-    a.T = 4 * nw;   // 16-slot m-tiles x four q-groups of 8 directions = warps
+    a.T = 4 * nw;
+    // fused contractions when every problem's G fits in 16 column tiles; in
+    // FP64 one warp per 8 slots x 8 quadrature rows of a 32-row chunk, mixed
+    // one per 16 slots x 8 rows
+    const int nt2 = K2tot / 8;
+    a.ntf = (nt2 <= 16) ? ((nt2 + 7) / 8) * 8 : 0;
+    a.warps = (a.ntf > 0 && !a.mixed) ? 2 * nw : nw;
     a.kq = 32;
     a.ntq = a.kq / 8;
     a.ldv = nbMax + 4;
@@ -47,37 +55,34 @@ int plan_newton(NewtonArgs &a)
     a.offInt = take((T * SI_N + 1) / 2);
     a.offFpart = take(T * a.ntq);
     a.offStat = take(kStatU64 + 1);
-    // the 4-warp shape reads the Gaunt table through L1 so that two CTAs fit
+    // the 16-slot shape reads the Gaunt table through L1 so that two CTAs fit
     a.stageEll = (nw == kWarps) ? 1 : 0;   // matches the kernel's compile-time choice
     if (!a.stageEll)
-        ellRows = ellChunks = 0;
-    a.offEllVal = take(ellRows * 32);
-    a.offEllIdx = take((ellRows * 32 + 3) / 4);
-    a.offEllPair = take((ellChunks * 32 + 3) / 4);
+        ellGroups = ellChunks = 0;
+    a.offEllVal = take(ellGroups * kEllGroup);
+    a.offEllIdx = take(ellGroups * kEllGroup / 4);
+    a.offEllPair = take(ellChunks * 64 / 4);
     a.offEllOff = take((ellChunks + 2) / 2);
     a.offExp = take(64);
-    a.offBar = take(4);
+    a.offBar = take(6);
 
     exp_consts_init(a.ex);
     const int unionBase = off;
     const int ntiles2 = (T / 16) * (K2tot / 8);
     a.tpw = (ntiles2 + nw - 1) / nw;
-    // fused contractions when every problem's G fits in 16 column tiles
-    // (one warp per 16 slots x 8 quadrature rows of a 32-row chunk)
-    const int nt2 = K2tot / 8;
-    a.ntf = (nt2 <= 16) ? ((nt2 + 7) / 8) * 8 : 0;
     a.ntExact = (a.ntf > 0 && a.nprob == 1) ? nt2 : 0;
     a.nbk = (a.ntf > 0 && a.nprob == 1) ? a.prob[0].nb / 8 : 0;
     if (a.mixed && a.ntExact == 0)
         return -2;
     if (nw != kWarps && (a.ntExact == 0 || a.nprob != 1 || !a.prob[0].paired || a.mixed || a.optType != 0 ||
-                         !newton_pair4_supported(a.ntExact, a.nbk)))
-        return -1;   // the 4-warp shape: single-order direction-pair Newton only
+                         !newton_pair4_supported(a.ntExact, a.nbk, a.prob[0].n)))
+        return -1;   // the 16-slot shape: single-order direction-pair Newton only
     // phase-B region
     int offG = unionBase;
+    a.strideH = nMax * a.ldh;   // ldh is even
     int offH = offG + ((T * a.ldG + 1) & ~1);
-    int offVec = offH + ((nw * kMaxN * a.ldh + 1) & ~1);
-    int endB = offVec + nw * 64;
+    int offVec = offH + a.warps * a.strideH;
+    int endB = offVec + a.warps * 64;
 
     // phase-A region
     const int maxDoubles = (232448 - 1024) / 8;   // opt-in limit minus static shared
@@ -101,6 +106,9 @@ int plan_newton(NewtonArgs &a)
             return -2;
         if (nw != kWarps)
             return -1;
+        a.warps = nw;
+        offVec = offH + a.warps * a.strideH;
+        endB = offVec + a.warps * 64;
     }
     for (int db = 1; db >= 0; db--) {
         int offP = unionBase;

@@ -35,7 +35,7 @@ struct NewtonProblem {
     const unsigned short *ellPair, *ellIdx;
     const double *ellVal;
     const int *ellOff;
-    int ellChunks, ellRows;
+    int ellChunks, ellGroups;
     double p0;                  // p[0] = Y_00 (fobj.cpp:305 divides by it)
     // Converged-evaluation test without the Hessian (Mn, FP64): row 0 of the
     // Gaunt contraction (CSR rows (0, j), j < n, G columns in the layout's
@@ -137,12 +137,15 @@ struct NewtonArgs {
     double condHMaxBfgs;        // optType 2: MOMOPT_COND_H_MAX_BFGS
     int cbStride;               // doubles per slot of cbScratch (kCbSlotDoubles or kBfgsSlotDoubles)
     double *cbScratch;          // optType 1, 2: per-slot working state, [grid][T][cbStride]
-    // launch shape, set before plan_newton(): warps per CTA (0 or 8: 32
-    // slots, three staged chunks, one CTA per SM; 4: 16 slots, two staged
-    // chunks, the Gaunt table read through L1, two CTAs per SM -- fused
-    // direction-pair instances only)
+    // launch shape, set before plan_newton(): a quarter of the slots per CTA
+    // (0 or 8: 32 slots, three staged chunks, one CTA per SM; 4: 16 slots,
+    // two staged chunks, the Gaunt table read through L1, two CTAs per SM --
+    // fused direction-pair instances only)
     int nw;
+    int warps;                  // filled by plan_newton(): warps per CTA (2 nw on the fused FP64
+                                // contractions, else nw)
     int stageEll;               // filled by plan_newton(): Gaunt table staged in shared memory
+    int strideH;                // doubles of one warp's Hessian scratch
 };
 
 // Fills the layout fields from the problems' sizes; returns 0, -1 when the
@@ -151,10 +154,11 @@ struct NewtonArgs {
 int plan_newton(NewtonArgs &a);
 // Sets the kernel's shared-memory attribute (call once, outside capture).
 cudaError_t prepare_newton(const NewtonArgs &a);
-// A fused instance exists for the direction-pair layout with these counts.
-bool newton_pair_supported(int nt, int nbk);
-// ... and in the 4-warp launch shape.
-bool newton_pair4_supported(int nt, int nbk);
+// A fused instance exists for the direction-pair layout with these counts
+// and n moments.
+bool newton_pair_supported(int nt, int nbk, int n);
+// ... and in the 16-slot launch shape.
+bool newton_pair4_supported(int nt, int nbk, int n);
 // Screening pass (Mn, FP64, direction pairs; a.prob[0] the gradient-column
 // layout of the problem): layout, instance check, shared-memory attribute,
 // launch and resident CTAs per SM.
@@ -173,6 +177,7 @@ int newton_ctas_per_sm(const NewtonArgs &a);
 bool newton_run_generic(const NewtonArgs &a, int grid, cudaStream_t s, int mode, int *occ, cudaError_t *err);
 bool newton_run_exact_mn_a(const NewtonArgs &a, int grid, cudaStream_t s, int mode, int *occ, cudaError_t *err);
 bool newton_run_exact_pair(const NewtonArgs &a, int grid, cudaStream_t s, int mode, int *occ, cudaError_t *err);
+bool newton_run_exact_pair_b(const NewtonArgs &a, int grid, cudaStream_t s, int mode, int *occ, cudaError_t *err);
 bool newton_run_exact_pair4(const NewtonArgs &a, int grid, cudaStream_t s, int mode, int *occ, cudaError_t *err);
 bool newton_run_exact_mn_b(const NewtonArgs &a, int grid, cudaStream_t s, int mode, int *occ, cudaError_t *err);
 bool newton_run_exact_ppn_a(const NewtonArgs &a, int grid, cudaStream_t s, int mode, int *occ, cudaError_t *err);

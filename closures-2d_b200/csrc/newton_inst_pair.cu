@@ -1,19 +1,23 @@
 // newton_inst_pair.cu -- Mn instances of the direction-pair layout, one per
-// (column tiles, k-steps) of the Gaunt orders 1-6 and the direct orders 1-4.
+// (column tiles, k-steps, moments) of the Gaunt orders 1-6 and the direct
+// orders 1-4.  The moment count is part of the key: the per-slot logic
+// is unrolled for exactly that many rows.
 #include "newton_kernel.cuh"
 
 namespace clb {
 
 namespace {
-// (tiles, k-steps) of the paired layouts: Gaunt N = 1..6 -> (2,2) (3,2)
-// (4,2) (7,3) (9,4) (13,4); direct N = 3, 4 -> (7,2) (16,3) (N = 1, 2 as Gaunt)
-constexpr int kPairShapes[][2] = {{2, 2}, {3, 2}, {4, 2}, {7, 2}, {7, 3}, {9, 4}, {13, 4}, {16, 3}};
+// (tiles, k-steps, n) of the paired layouts: Gaunt N = 1..6 -> (2,2,3) (3,2,6)
+// (4,2,10) (7,3,15) (9,4,21) (13,4,28); direct N = 3, 4 -> (7,2,10) (16,3,15)
+// (N = 1, 2 as Gaunt)
+constexpr int kPairShapes[][3] = {{2, 2, 3}, {3, 2, 6}, {4, 2, 10}, {7, 2, 10}, {7, 3, 15}, {9, 4, 21}, {13, 4, 28},
+                                  {16, 3, 15}};
 }  // namespace
 
-bool newton_pair_supported(int nt, int nbk)
+bool newton_pair_supported(int nt, int nbk, int n)
 {
     for (const auto &s : kPairShapes)
-        if (s[0] == nt && s[1] == nbk)
+        if (s[0] == nt && s[1] == nbk && s[2] == n)
             return true;
     return false;
 }
@@ -22,21 +26,19 @@ bool newton_run_exact_pair(const NewtonArgs &a, int grid, cudaStream_t s, int mo
 {
     if (a.momentType != 0 || a.mixed)
         return false;
-#define CLB_PAIR(NT_, NBK_)                                                                     \
-    if (a.ntExact == NT_ && a.nbk == NBK_) {                                                   \
-        *err = newton_run<1, NT_, 0, NT_, NBK_, 0, 1>(a, grid, s, mode, occ);                  \
+#define CLB_PAIR(NT_, NBK_, N_, NTE_, NBE_)                                                     \
+    if (a.ntExact == NT_ && a.nbk == NBK_ && a.prob[0].n == N_ && a.prob[0].K2e == 8 * NTE_ &&   \
+        a.prob[0].nbe == 8 * NBE_) {                                                            \
+        *err = newton_run<1, NT_, 0, NT_, NBK_, 0, 16 * NTE_ + NBE_, 16, N_>(a, grid, s, mode, occ); \
         return true;                                                                           \
     }
-    CLB_PAIR(2, 2)
-    CLB_PAIR(3, 2)
-    CLB_PAIR(4, 2)
-    CLB_PAIR(7, 2)
-    CLB_PAIR(7, 3)
-    CLB_PAIR(9, 4)
-    CLB_PAIR(13, 4)
-    CLB_PAIR(16, 3)
+    CLB_PAIR(2, 2, 3, 1, 1)
+    CLB_PAIR(3, 2, 6, 2, 1)
+    CLB_PAIR(4, 2, 10, 2, 1)
+    CLB_PAIR(7, 2, 10, 4, 1)
+    CLB_PAIR(7, 3, 15, 4, 2)
 #undef CLB_PAIR
-    return false;
+    return newton_run_exact_pair_b(a, grid, s, mode, occ, err);
 }
 
 }  // namespace clb

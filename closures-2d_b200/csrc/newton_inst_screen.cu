@@ -13,7 +13,7 @@ int plan_screen(NewtonArgs &a)
     const NewtonProblem &pb = a.prob[0];
     if (a.nprob != 1 || !pb.paired || a.momentType != 0 || a.mixed || a.optType != 0)
         return -1;
-    a.nw = kWarps;
+    a.nw = a.warps = kWarps;
     a.T = 32;
     a.kq = 32;
     a.ntq = a.kq / 8;
@@ -39,7 +39,7 @@ int plan_screen(NewtonArgs &a)
     a.stageEll = 0;
     a.offEllVal = a.offEllIdx = a.offEllPair = a.offEllOff = off;
     a.offExp = take(64);
-    a.offBar = take(4);
+    a.offBar = take(6);
     a.offEg = take(4 * a.ldv);   // the representative start and results
     a.offE = 0;
     exp_consts_init(a.ex);

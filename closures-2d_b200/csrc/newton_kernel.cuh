@@ -57,10 +57,11 @@ __device__ __forceinline__ void record_error(int *err, int code, int idx)
 // loads: lane i writes L_ij there at step j, and 1/L_jj on the diagonal.
 // On return h[k] = L_lane,k for k <= lane.  LAPACK-style info: 0, or j+1 at
 // the first non-positive or NaN pivot (dpotrf semantics).
-__device__ __forceinline__ int chol_regs(double (&h)[kMaxN], double *Ls, int ldl, int n, int lane)
+template <int NM>
+__device__ __forceinline__ int chol_regs(double (&h)[NM], double *Ls, int ldl, int n, int lane)
 {
 #pragma unroll
-    for (int j = 0; j < kMaxN; j++) {
+    for (int j = 0; j < NM; j++) {
         if (j < n) {
             const double *Lj = Ls + j * ldl;
             double s0 = h[j], s1 = 0.0, s2 = 0.0, s3 = 0.0;
@@ -95,12 +96,50 @@ __device__ __forceinline__ int chol_regs(double (&h)[kMaxN], double *Ls, int ldl
     return 0;
 }
 
+// The same factorisation column by column (right-looking), for the instances
+// with ten or more moments: lane i >= j forms L_ij = h[j] / L_jj and writes it
+// to row j of Lt (L transposed: Lt[j * ld + i] = L_ij, 1 / L_jj on the
+// diagonal), and every lane takes column j off its row, h[k] -= L_ij L_kj, with
+// the L_kj from one row of Lt (16-byte broadcasts).  The updates are
+// independent, so a column costs its pivot (shuffle, reciprocal root) and one
+// trip through shared memory rather than a chain of dot products: 28
+// columns alone in a warp take 10.4k cycles in the form above.
+// On return h[k] = L_lane,k for k <= lane; false at a non-positive or NaN
+// pivot.
+template <int NM>
+__device__ __forceinline__ bool chol_cols(double (&h)[NM], double *Lt, int ld, int lane)
+{
+    bool spd = true;
+#pragma unroll
+    for (int j = 0; j < NM; j++) {
+        const double d = __shfl_sync(0xffffffffu, h[j], j);
+        spd = spd && d > 0.0;
+        const double r = rsqrt(d);
+        const double l = h[j] * r;
+        h[j] = l;
+        double *c = Lt + j * ld;
+        if (lane >= j && lane < NM)
+            c[lane] = (lane == j) ? r : l;
+        __syncwarp();
+#pragma unroll
+        for (int k = (j + 1) & ~1; k < NM; k += 2) {
+            const double2 lk = *reinterpret_cast<const double2 *>(c + k);
+            if (k > j)
+                h[k] = fma(-l, lk.x, h[k]);
+            if (k + 1 < NM)
+                h[k + 1] = fma(-l, lk.y, h[k + 1]);
+        }
+    }
+    return spd;
+}
+
 // Column `lane` of L^-1 into v[]: Linv_ic = -(sum_{k=c}^{i-1} L_ik Linv_kc) / L_ii,
 // rows in order, row i of L and 1/L_ii read from Ls as left by chol_regs.
-__device__ __forceinline__ void invert_regs(const double *Ls, int ldl, double (&v)[kMaxN], int n, int lane)
+template <int NM>
+__device__ __forceinline__ void invert_regs(const double *Ls, int ldl, double (&v)[NM], int n, int lane)
 {
 #pragma unroll
-    for (int i = 0; i < kMaxN; i++) {
+    for (int i = 0; i < NM; i++) {
         v[i] = 0.0;
         if (i < n) {
             const double *Li = Ls + i * ldl;
@@ -133,12 +172,13 @@ __device__ __forceinline__ void invert_regs(const double *Ls, int ldl, double (&
 // The two substitutions (nonnegative terms only) run interleaved; factor rows
 // come from h[] (lane i: L_ik) and Ls (1/L_kk on the diagonal, as left by
 // chol_regs).  Used where it is tight: Hessians of smooth cells.
-__device__ __forceinline__ double cmp_bound(const double (&h)[kMaxN], const double *Ls, int ldl, int n, int lane)
+template <int NM>
+__device__ __forceinline__ double cmp_bound(const double (&h)[NM], const double *Ls, int ldl, int n, int lane)
 {
     const double rl = (lane < n) ? Ls[lane * ldl + lane] : 0.0;
     double accF = 0.0, accB = 0.0;
 #pragma unroll
-    for (int s = 0; s < kMaxN; s++) {
+    for (int s = 0; s < NM; s++) {
         if (s < n) {
             const int kf = s, kb = n - 1 - s;
             const double xf = __shfl_sync(0xffffffffu, (1.0 + accF) * rl, kf);
@@ -222,6 +262,38 @@ __device__ double rcond_warp(const double *Hs, int n, int ldh, double *vec, doub
     if (est != 0.0)
         return (1.0 / est) / anorm;
     return 0.0;
+}
+
+// The condition estimate of A = L L^T from L (rows in Hs, 1 / L_ii on the
+// diagonal): column `lane` of L^-1 into v[], its rows into Hs, and 0 where the
+// bound ||A^-1||_1 <= ||L^-1||_1 ||L^-1||_inf already shows cond <= COND_H_MAX
+// (the Higham estimate never exceeds ||A^-1||_1; a factor-2 margin covers
+// rounding), so that the estimate cannot trigger regularisation and is not
+// needed; else that estimate.
+template <int NM>
+__device__ __forceinline__ double cond_by_inverse(const NewtonArgs &a, double *Hs, int ldh, double *vec,
+                                                  double (&v)[NM], int n, double anorm, int lane)
+{
+    const bool act = lane < n;
+    invert_regs(Hs, ldh, v, n, lane);
+    __syncwarp();
+    double colsum = 0.0;
+#pragma unroll
+    for (int i = 0; i < NM; i++) {
+        if (i < n && act)
+            Hs[i * ldh + lane] = v[i];
+        colsum += fabs(v[i]);
+    }
+    __syncwarp();
+    double rs = 0.0;   // unrolled: the loads issue together, the sum keeps its order
+#pragma unroll
+    for (int c = 0; c < NM; c++)
+        if (act && c <= lane)
+            rs += fabs(Hs[lane * ldh + c]);
+    const double bound = anorm * warp_max(colsum) * warp_max(rs);
+    if (bound <= 0.5 * a.condHMax)
+        return 0.0;
+    return 1.0 / rcond_warp(Hs, n, ldh, vec, anorm, lane);
 }
 
 struct Layout {
@@ -476,29 +548,40 @@ __device__ __forceinline__ void hessian_from_contractions(const NewtonArgs &a, c
     const int n = pb.n, ldh = a.ldh;
     const int npairs = n * (n + 1) / 2;
     if (a.useGaunt) {
+        // two pairs per lane, four entries of each per step: one 16-byte load
+        // brings the eight G columns, four the coefficients; each pair's sum
+        // runs through its entries in order
+        const uint4 *eidx = reinterpret_cast<const uint4 *>(L.ellIdx) + lane;
+        const double2 *eval = reinterpret_cast<const double2 *>(L.ellVal) + lane;
+        int g = L.ellOff[0];
         for (int c = 0; c < pb.ellChunks; c++) {
-            const unsigned short pr = L.ellPair[c * 32 + lane];
-            const int e1 = L.ellOff[c + 1];
-            int e = L.ellOff[c];
-            double v = 0.0;
-            // loads of four entries issued ahead of their (in-order) sum
-            for (; e + 4 <= e1; e += 4) {
-                const int i0 = L.ellIdx[e * 32 + lane], i1 = L.ellIdx[(e + 1) * 32 + lane];
-                const int i2 = L.ellIdx[(e + 2) * 32 + lane], i3 = L.ellIdx[(e + 3) * 32 + lane];
-                const double w0 = L.ellVal[e * 32 + lane], w1 = L.ellVal[(e + 1) * 32 + lane];
-                const double w2 = L.ellVal[(e + 2) * 32 + lane], w3 = L.ellVal[(e + 3) * 32 + lane];
-                const double g0 = Gs[i0], g1 = Gs[i1], g2 = Gs[i2], g3 = Gs[i3];
-                v += w0 * g0;
-                v += w1 * g1;
-                v += w2 * g2;
-                v += w3 * g3;
+            const unsigned p0 = L.ellPair[c * 64 + lane], p1 = L.ellPair[c * 64 + 32 + lane];
+            const int g1 = L.ellOff[c + 1];
+            double v0 = 0.0, v1 = 0.0;
+            for (; g < g1; g++) {
+                const uint4 ix = eidx[g * 32];
+                const double2 a0 = eval[g * 128], a1 = eval[g * 128 + 32];
+                const double2 b0 = eval[g * 128 + 64], b1 = eval[g * 128 + 96];
+                const double x0 = Gs[ix.x & 0xffff], x1 = Gs[ix.x >> 16], x2 = Gs[ix.y & 0xffff], x3 = Gs[ix.y >> 16];
+                const double y0 = Gs[ix.z & 0xffff], y1 = Gs[ix.z >> 16], y2 = Gs[ix.w & 0xffff], y3 = Gs[ix.w >> 16];
+                v0 = fma(a0.x, x0, v0);
+                v1 = fma(b0.x, y0, v1);
+                v0 = fma(a0.y, x1, v0);
+                v1 = fma(b0.y, y1, v1);
+                v0 = fma(a1.x, x2, v0);
+                v1 = fma(b1.x, y2, v1);
+                v0 = fma(a1.y, x3, v0);
+                v1 = fma(b1.y, y3, v1);
             }
-            for (; e < e1; e++)
-                v += L.ellVal[e * 32 + lane] * Gs[L.ellIdx[e * 32 + lane]];
-            if (pr != 0xFFFF) {
-                int i = pr >> 8, j = pr & 255;
-                Hs[i * ldh + j] = v;
-                Hs[j * ldh + i] = v;
+            if (p0 != 0xFFFF) {
+                const int i = p0 >> 8, j = p0 & 255;
+                Hs[i * ldh + j] = v0;
+                Hs[j * ldh + i] = v0;
+            }
+            if (p1 != 0xFFFF) {
+                const int i = p1 >> 8, j = p1 & 255;
+                Hs[i * ldh + j] = v1;
+                Hs[j * ldh + i] = v1;
             }
         }
     } else {
@@ -605,16 +688,20 @@ __device__ __forceinline__ double hessian_row0(const NewtonArgs &a, const Newton
 }
 
 // Newton logic for one slot after its evaluation (warp-wide).  `range`: the
-// evaluation is Mn in FP64 (the exponent-range test applies).
+// evaluation is Mn in FP64 (the exponent-range test applies).  NX is n where
+// the instance fixes it (else 0) and NM >= n bounds the unrolled loops over
+// rows and columns: with n fixed they are straight-line code without a guard
+// per row.
+template <int NM, int NX>
 __device__ void slot_logic(const NewtonArgs &a, const NewtonProblem &pb, Layout &L, int s, int lane,
                            int warp, bool range)
 {
-    const int n = pb.n;
+    const int n = NX ? NX : pb.n;
     const int ldv = a.ldv, ldG = a.ldG, ldh = a.ldh;
     const bool act = lane < n;
     int *si = L.ints + s * SI_N;
     double *sc = L.scal + s * SC_N;
-    double *Hs = L.H + warp * (kMaxN * ldh);
+    double *Hs = L.H + warp * a.strideH;
     double *vec = L.vec + warp * 64;
     const double *Gs = L.G + s * ldG;
 
@@ -720,10 +807,10 @@ __device__ void slot_logic(const NewtonArgs &a, const NewtonProblem &pb, Layout 
     const double fH = (a.momentType == 0) ? Hs[0] / (pb.p0 * pb.p0) - au : fsum;
 
     // row `lane` of H in registers; utils_norm1 = max absolute row sum
-    double h[kMaxN], v[kMaxN];
+    double h[NM];
     double rowsum = 0.0;
 #pragma unroll
-    for (int k = 0; k < kMaxN; k++) {
+    for (int k = 0; k < NM; k++) {
         h[k] = (act && k < n) ? Hs[lane * ldh + k] : 0.0;
         rowsum += fabs(h[k]);
     }
@@ -749,68 +836,100 @@ __device__ void slot_logic(const NewtonArgs &a, const NewtonProblem &pb, Layout 
             return;
         }
     }
-    __syncwarp();
-    int info = chol_regs(h, Hs, ldh, n, lane);
-    if (info == 0 && convTest && anorm * cmp_bound(h, Hs, ldh, n, lane) <= 0.5 * a.condHMax) {
-        converge(a, pb, L, s, ui, ai, gi, lane);
-        return;
-    }
-    double condest = 0.0;
-    if (info == 0) {
-        // column `lane` of L^-1 in v[], rows of L^-1 in Hs
-        invert_regs(Hs, ldh, v, n, lane);
+    double di;
+    if constexpr (NX >= 10) {
+        // Ten or more moments: the direction by the two triangular solves of
+        // dpotrs, the comparison-matrix bound's substitutions beside the
+        // first of them; L^-1 only where neither that bound nor the exponent
+        // range settles the condition test.
         __syncwarp();
-        double colsum = 0.0;
+        const bool spd = chol_cols(h, Hs, ldh, lane);   // Hs: L transposed
+        const double rl = act ? Hs[lane * ldh + lane] : 0.0;
+        double accY = 0.0, accF = 0.0, accB = 0.0, accZ = 0.0;
 #pragma unroll
-        for (int i = 0; i < kMaxN; i++) {
-            if (i < n && act)
-                Hs[i * ldh + lane] = v[i];
-            colsum += fabs(v[i]);
+        for (int s2 = 0; s2 < NM; s2++) {
+            const int kb = NM - 1 - s2;
+            const double y = __shfl_sync(0xffffffffu, (gi - accY) * rl, s2);
+            const double xf = __shfl_sync(0xffffffffu, (1.0 + accF) * rl, s2);
+            const double xb = __shfl_sync(0xffffffffu, (1.0 + accB) * rl, kb);
+            if (lane > s2) {   // h[k] holds L_lane,k only for k <= lane
+                accY = fma(h[s2], y, accY);
+                accF = fma(fabs(h[s2]), xf, accF);
+            }
+            if (lane < kb)
+                accB = fma(fabs(Hs[lane * ldh + kb]), xb, accB);
         }
-        __syncwarp();
-        double rs = 0.0;   // unrolled: the loads issue together, the sum keeps its order
+        const double bound = warp_max(act ? (1.0 + accF) * rl : 0.0) * warp_max(act ? (1.0 + accB) * rl : 0.0);
+        const bool small = anorm * bound <= 0.5 * a.condHMax;   // (false for NaN)
+        if (spd && convTest && small) {
+            converge(a, pb, L, s, ui, ai, gi, lane);
+            return;
+        }
+        const double yl = (gi - accY) * rl;
 #pragma unroll
-        for (int c = 0; c < kMaxN; c++)
+        for (int i = NM - 1; i >= 0; i--) {
+            const double zi = __shfl_sync(0xffffffffu, (yl - accZ) * rl, i);
+            if (lane < i)
+                accZ = fma(Hs[lane * ldh + i], zi, accZ);
+        }
+        di = act ? -(yl - accZ) * rl : 0.0;
+        double condest = 0.0;
+        if (spd && !small &&
+            !(range && a.momentType == 0 && pb.gramLo > 0.0 && exponent_range_bound(a, pb, ai, lane))) {
+            double v[NM];
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < NM; k++)   // L by rows, 1 / L_kk on the diagonal
+                if (act && k <= lane)
+                    Hs[lane * ldh + k] = (k == lane) ? rl : h[k];
+            __syncwarp();
+            condest = cond_by_inverse(a, Hs, ldh, vec, v, n, anorm, lane);
+        }
+        if (iter >= si[SI_MAXITER] || !spd || sc[SC_T] == 0.0 || condest > a.condHMax) {
+            __syncwarp();
+            regularize(a, pb, L, s, lane, ldv, ui, ai);
+            return;
+        }
+    } else {
+        __syncwarp();
+        const int info = chol_regs(h, Hs, ldh, n, lane);
+        if (info == 0 && convTest && anorm * cmp_bound(h, Hs, ldh, n, lane) <= 0.5 * a.condHMax) {
+            converge(a, pb, L, s, ui, ai, gi, lane);
+            return;
+        }
+        double v[NM];
+        double condest = 0.0;
+        if (info == 0)
+            condest = cond_by_inverse(a, Hs, ldh, vec, v, n, anorm, lane);
+        if (iter >= si[SI_MAXITER] || info != 0 || sc[SC_T] == 0.0 || condest > a.condHMax) {
+            __syncwarp();
+            regularize(a, pb, L, s, lane, ldv, ui, ai);
+            return;
+        }
+        // d = -L^-T (L^-1 g): rows of L^-1 from Hs, columns from registers
+        __syncwarp();
+        vec[lane] = gi;
+        __syncwarp();
+        double y = 0.0;
+#pragma unroll
+        for (int c = 0; c < NM; c++)
             if (act && c <= lane)
-                rs += fabs(Hs[lane * ldh + c]);
-        // ||A^-1||_1 <= ||L^-1||_1 ||L^-1||_inf, and the Higham estimate never
-        // exceeds ||A^-1||_1: when the bound already shows cond <= COND_H_MAX
-        // (with a factor-2 margin for rounding) the estimate cannot trigger
-        // regularisation and is not needed.
-        const double bound = anorm * warp_max(colsum) * warp_max(rs);
-        if (!(bound <= 0.5 * a.condHMax)) {
-            double rc = rcond_warp(Hs, n, ldh, vec, anorm, lane);
-            condest = 1.0 / rc;
-        }
-    }
-    if (iter >= si[SI_MAXITER] || info != 0 || sc[SC_T] == 0.0 || condest > a.condHMax) {
+                y = fma(Hs[lane * ldh + c], vec[c], y);
         __syncwarp();
-        regularize(a, pb, L, s, lane, ldv, ui, ai);
-        return;
-    }
-    // d = -L^-T (L^-1 g): rows of L^-1 from Hs, columns from registers
-    __syncwarp();
-    vec[lane] = gi;
-    __syncwarp();
-    double y = 0.0;
+        vec[32 + lane] = y;
+        __syncwarp();
+        double z = 0.0;
 #pragma unroll
-    for (int c = 0; c < kMaxN; c++)
-        if (act && c <= lane)
-            y = fma(Hs[lane * ldh + c], vec[c], y);
-    __syncwarp();
-    vec[32 + lane] = y;
-    __syncwarp();
-    double z = 0.0;
-#pragma unroll
-    for (int i = 0; i < kMaxN; i += 2) {
-        if (i < n) {
-            const double2 yi = *reinterpret_cast<const double2 *>(vec + 32 + i);
-            z = fma(v[i], yi.x, z);
-            if (i + 1 < n)
-                z = fma(v[i + 1], yi.y, z);
+        for (int i = 0; i < NM; i += 2) {
+            if (i < n) {
+                const double2 yi = *reinterpret_cast<const double2 *>(vec + 32 + i);
+                z = fma(v[i], yi.x, z);
+                if (i + 1 < n)
+                    z = fma(v[i + 1], yi.y, z);
+            }
         }
+        di = act ? -z : 0.0;
     }
-    const double di = act ? -z : 0.0;
     bool gammaOk = true;
     if (a.tolGamma > 0.0)
         gammaOk = modcfl(di, n, lane, a.momentType) <= a.tolGamma;
@@ -896,10 +1015,11 @@ __device__ double cb_solve_t(const double *Tg, double y, int n, int lane)
 // Columns held per lane (lane j: m[i] = M_ij) replaced by those of T^-1 M:
 // forward substitution by rows, row i of T (stride kMaxN) read by every lane
 // (one broadcast), rd[i] = 1/T_ii.
-__device__ __forceinline__ void cb_trsv_cols(const double *Tg, const double *rd, double (&m)[kMaxN], int n)
+template <int NM>
+__device__ __forceinline__ void cb_trsv_cols(const double *Tg, const double *rd, double (&m)[NM], int n)
 {
 #pragma unroll
-    for (int i = 0; i < kMaxN; i++) {
+    for (int i = 0; i < NM; i++) {
         if (i < n) {
             const double *Ti = Tg + i * kMaxN;
             double a0 = m[i], a1 = 0.0, a2 = 0.0, a3 = 0.0;
@@ -1299,14 +1419,15 @@ __device__ bool bfgs_after_step(const NewtonArgs &a, const NewtonProblem &pb, La
 }
 
 // Newton logic of one change-of-basis slot after its evaluation.
+template <int NM, int NX>
 __device__ void slot_logic_cb(const NewtonArgs &a, const NewtonProblem &pb, Layout &L, int s, int lane, int warp)
 {
-    const int n = pb.n;
+    const int n = NX ? NX : pb.n;
     const int ldv = a.ldv, ldG = a.ldG, ldh = a.ldh;
     const bool act = lane < n;
     int *si = L.ints + s * SI_N;
     double *sc = L.scal + s * SC_N;
-    double *Hs = L.H + warp * (kMaxN * ldh);
+    double *Hs = L.H + warp * a.strideH;
     double *Wi = cb_linv(a, s);   // rows of L^-1, stride kMaxN
     double *APs = cb_ap(a, s), *AMs = cb_am(a, s), *DMs = cb_dm(a, s);
     double *vec = L.vec + warp * 64;
@@ -1381,14 +1502,14 @@ __device__ void slot_logic_cb(const NewtonArgs &a, const NewtonProblem &pb, Layo
     vec[lane] = gi;
     __syncwarp();
     // X = T^-1 [H_M | g_M]: lane j < n a column of H_M, lane n the gradient
-    double m[kMaxN];
+    double m[NM];
 #pragma unroll
-    for (int k = 0; k < kMaxN; k++)
+    for (int k = 0; k < NM; k++)
         m[k] = (k < n) ? (act ? Hs[lane * ldh + k] : (lane == n ? vec[k] : 0.0)) : 0.0;
     cb_trsv_cols(Tg, rd, m, n);
     __syncwarp();
 #pragma unroll
-    for (int k = 0; k < kMaxN; k++) {
+    for (int k = 0; k < NM; k++) {
         if (k < n) {
             if (act)
                 Hs[k * ldh + lane] = m[k];
@@ -1399,24 +1520,24 @@ __device__ void slot_logic_cb(const NewtonArgs &a, const NewtonProblem &pb, Layo
     __syncwarp();
     // H_P = T^-1 X^T: lane j takes row j of X (a column of X^T)
 #pragma unroll
-    for (int k = 0; k < kMaxN; k++)
+    for (int k = 0; k < NM; k++)
         m[k] = (act && k < n) ? Hs[lane * ldh + k] : 0.0;
     cb_trsv_cols(Tg, rd, m, n);
     double rowsum = 0.0;
 #pragma unroll
-    for (int k = 0; k < kMaxN; k++)
+    for (int k = 0; k < NM; k++)
         rowsum += (k < n) ? fabs(m[k]) : 0.0;
     const double anorm = warp_max(act ? rowsum : 0.0);
     __syncwarp();
     int info = chol_regs(m, Hs, ldh, n, lane);
     double condest = 0.0;
-    double v[kMaxN];
+    double v[NM];
     if (info == 0) {
         invert_regs(Hs, ldh, v, n, lane);
         __syncwarp();
         double colsum = 0.0;
 #pragma unroll
-        for (int i = 0; i < kMaxN; i++) {
+        for (int i = 0; i < NM; i++) {
             if (i < n && act)
                 Wi[i * kMaxN + lane] = v[i];   // rows of L^-1
             colsum += fabs(v[i]);
@@ -1466,19 +1587,19 @@ __device__ void slot_logic_cb(const NewtonArgs &a, const NewtonProblem &pb, Layo
     }
     // T <- T L: lane i forms row i
     {
-        double t[kMaxN], tn[kMaxN];
+        double t[NM], tn[NM];
 #pragma unroll
-        for (int k = 0; k < kMaxN; k++) {
+        for (int k = 0; k < NM; k++) {
             t[k] = (act && k <= lane) ? Tg[lane * kMaxN + k] : 0.0;
             tn[k] = 0.0;
         }
 #pragma unroll
-        for (int k = 0; k < kMaxN; k++) {
+        for (int k = 0; k < NM; k++) {
             if (k < n) {
                 const double *Lk = Hs + k * ldh;
                 const double lkk = 1.0 / Lk[k];
 #pragma unroll
-                for (int j = 0; j < kMaxN; j++)
+                for (int j = 0; j < NM; j++)
                     if (j <= k)
                         tn[j] = fma(t[k], (j == k) ? lkk : Lk[j], tn[j]);
             }
@@ -1486,7 +1607,7 @@ __device__ void slot_logic_cb(const NewtonArgs &a, const NewtonProblem &pb, Layo
         __syncwarp();
         double tdiag = 1.0;
 #pragma unroll
-        for (int k = 0; k < kMaxN; k++) {
+        for (int k = 0; k < NM; k++) {
             if (act && k <= lane)
                 Tg[lane * kMaxN + k] = tn[k];
             if (k == lane)
@@ -1565,6 +1686,22 @@ __device__ void slot_logic_cb(const NewtonArgs &a, const NewtonProblem &pb, Layo
 // buffers keep one chunk in flight while two are read.
 constexpr unsigned long long kWaitNs = 2000000000ull;   // bound on any wait for a staged chunk
 
+// The weighted exponentials of a direction pair: their sum (even column
+// tiles) and difference (odd ones).  Roundings spelled out, so that the
+// screening pass and K1 form the same bits whatever a compiler would contract.
+__device__ __forceinline__ void pair_weights(double &sum, double &diff, double x, double y, double w)
+{
+    const double yw = __dmul_rn(y, w);
+    sum = __fma_rn(x, w, yw);
+    diff = __fma_rn(x, w, -yw);
+}
+
+// The part of f of two pairs (x, y) with weights w0, w1.
+__device__ __forceinline__ double pair_f(double x0, double x1, double y0, double y1, double w0, double w1)
+{
+    return __dadd_rn(__fma_rn(x0, w0, __dmul_rn(x1, w1)), __fma_rn(y0, w0, __dmul_rn(y1, w1)));
+}
+
 // PAIR (Mn, FP64): the chunk's rows are one direction q of each (phi,
 // phi + pi) pair and the columns are grouped by degree parity.  GEMM1 forms
 // the even and odd half sums S_e, S_o of alpha . p(q); the pair's exponents
@@ -1573,20 +1710,17 @@ constexpr unsigned long long kWaitNs = 2000000000ull;   // bound on any wait for
 // the A operand of the even column tiles and their difference for the odd
 // ones.  Each MMA so serves two directions.
 //
-// NW (warps per CTA) sets the launch shape: NW = 8 runs T = 32 slots (two
-// 16-slot m-tiles, q-group = warp / 2) with three chunk buffers, one CTA per
-// SM; NW = 4 runs T = 16 slots (one m-tile, q-group = warp) with two chunk
-// buffers, small enough for two CTAs per SM, so that one CTA's phase B runs
-// while the other's phase A keeps the tensor pipe busy.  Each slot's sums
-// are the same MMAs in the same order in both shapes.
-template <int NTF, int PPN, int NT, int NBK, int MIX, int PAIR = 0, int NW = 8>
+// Runs T = 32 slots on 8 warps (two 16-slot m-tiles, q-group = warp / 2) with
+// three chunk buffers: the mixed-precision instances, whose split-TF32 tiles
+// exist only 16 rows high, and the screening pass.  The FP64 instances run
+// phase_a_rows8.
+template <int NTF, int PPN, int NT, int NBK, int MIX, int PAIR = 0>
 __device__ __forceinline__ bool phase_a_fused(const NewtonArgs &a, const NewtonProblem &pb, Layout &L, int tid,
                                               int lane, int warp, unsigned &mbPhase)
 {
     static_assert(!PAIR || (PPN == 0 && MIX == 0), "direction pairs: Mn in FP64");
-    static_assert(NW == 8 || NW == 4, "launch shapes: 8 warps (32 slots) or 4 warps (16 slots)");
-    constexpr int MT = NW / 4;                  // 16-slot m-tiles: T = 16 MT
-    constexpr int DEPTH = (NW == 8) ? 3 : 2;    // staged chunk buffers
+    constexpr int MT = 2;       // 16-slot m-tiles: T = 16 MT
+    constexpr int DEPTH = 3;    // staged chunk buffers
     const int g = lane >> 2, t4 = lane & 3;
     const int kq = a.kq, ldv = a.ldv, ldG = a.ldG;
     const int nb = pb.nb, ldP = pb.ldP, K2p = pb.K2p;
@@ -1701,18 +1835,10 @@ __device__ __forceinline__ bool phase_a_fused(const NewtonArgs &a, const NewtonP
             }
             fast_exp_n<8>(x, sv, L.exptab, invL, L1, L2);
 #pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const double ww = (h & 1) ? w1 : w0;
-                x[h] *= ww;
-                x[4 + h] *= ww;
-            }
-            facc0 += (x[0] + x[1]) + (x[4] + x[5]);
-            facc1 += (x[2] + x[3]) + (x[6] + x[7]);
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                e[h] = x[h] + x[4 + h];
-                eg[h] = x[h] - x[4 + h];
-            }
+            for (int h = 0; h < 4; h++)
+                pair_weights(e[h], eg[h], x[h], x[4 + h], (h & 1) ? w1 : w0);
+            facc0 += pair_f(x[0], x[1], x[4], x[5], w0, w1);
+            facc1 += pair_f(x[2], x[3], x[6], x[7], w0, w1);
         } else if constexpr (PPN == 0) {
             fast_exp_n<4>(e, cs, L.exptab, invL, L1, L2);
             e[0] *= w0;
@@ -1790,39 +1916,19 @@ __device__ __forceinline__ bool phase_a_fused(const NewtonArgs &a, const NewtonP
         }
     };
     int bc = 0;   // buffer of chunk c
-    if constexpr (DEPTH == 3) {
-        for (int c = 0; c + 1 < nchunks; c++) {
-            const int bn = (bc == 2) ? 0 : bc + 1, bf = (bn == 2) ? 0 : bn + 1;
-            const bool okWait = wait_chunk(bn);
-            // chunk c + 1 visible to all; every warp is done with chunk c - 1 (buffer bf)
-            if (__syncthreads_or(!okWait))
-                return abandon();
-            if (c + 2 < nchunks)
-                load_chunk(c + 2, bf);
-            double cs[4], co[4];
-            gemm1(L.P + bn * chunkDoubles, cs, co);
-            gemm2(L.P + bc * chunkDoubles);
-            weights(L.P + bn * chunkDoubles, cs, co, e, eg);
-            bc = bn;
-        }
-    } else {
-        // two buffers: chunk c + 2 goes into chunk c's buffer once every
-        // warp has finished its GEMM2 on chunk c
-        for (int c = 0; c + 1 < nchunks; c++) {
-            const int bn = bc ^ 1;
-            const bool okWait = wait_chunk(bn);
-            if (__syncthreads_or(!okWait))
-                return abandon();
-            double cs[4], co[4];
-            gemm1(L.P + bn * chunkDoubles, cs, co);
-            gemm2(L.P + bc * chunkDoubles);
-            weights(L.P + bn * chunkDoubles, cs, co, e, eg);
-            if (c + 2 < nchunks) {
-                __syncthreads();
-                load_chunk(c + 2, bc);
-            }
-            bc = bn;
-        }
+    for (int c = 0; c + 1 < nchunks; c++) {
+        const int bn = (bc == 2) ? 0 : bc + 1, bf = (bn == 2) ? 0 : bn + 1;
+        const bool okWait = wait_chunk(bn);
+        // chunk c + 1 visible to all; every warp is done with chunk c - 1 (buffer bf)
+        if (__syncthreads_or(!okWait))
+            return abandon();
+        if (c + 2 < nchunks)
+            load_chunk(c + 2, bf);
+        double cs[4], co[4];
+        gemm1(L.P + bn * chunkDoubles, cs, co);
+        gemm2(L.P + bc * chunkDoubles);
+        weights(L.P + bn * chunkDoubles, cs, co, e, eg);
+        bc = bn;
     }
     gemm2(L.P + bc * chunkDoubles);   // the last chunk (waited for by the last iteration)
     if constexpr (MIX) {
@@ -1868,13 +1974,284 @@ __device__ __forceinline__ bool phase_a_fused(const NewtonArgs &a, const NewtonP
     return true;
 }
 
-template <int TPW, int NTF, int PPN, int NT, int NBK, int MIX, int PAIR = 0, int NW = 8>
-__global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) newton_kernel(const __grid_constant__ NewtonArgs a)
+// What phase_a_rows8 needs of the launch and the problem.
+struct PhaseA {
+    int offAlpha, offScal, offFpart, offP, offG, offExp, offBar;   // doubles into shared memory
+    int ldv, ldG, ntq, nb, ldP, K2p, nchunks;
+    const double *P;       // the problem's basis
+    const short *binv;     // direction pairs: moment of each basis column
+    double invL, L1, L2;
+    int *err;
+};
+
+// The FP64 contractions in 8-slot row tiles (DMMA m8n8k4): warp w owns the 8
+// slots mt = w / 4 and the q-group qg = w % 4, so T slots take T / 2 warps.
+// On this chip an m16n8k8 FP64 MMA is, bit for bit, the chain of fused
+// multiply-adds over k, and runs at the FP64 pipe's rate in either shape (64
+// cycles per m16n8k8, 16 per m8n8k4 per scheduler, measured); the half-height
+// tile halves a warp's accumulators, so sixteen warps fit on an SM instead of
+// eight.  Both phases are bound by latency (with eight warps: issue 27 %
+// active, FP64 pipe 29 %), so warps in flight are what they lack.  Each sum
+// has the same terms in the same order as with 16-slot tiles.
+//
+// PAIR (Mn): 0, or 16 * (even column tiles) + even k-steps of the
+// direction-pair layout, whose parity split the unrolled loops then know.
+//
+// Chunks arrive by one bulk copy each and are handed back per warp (an
+// "empty" mbarrier per buffer, one arrival per warp), so warps drift up to a
+// chunk apart and one warp's exponentials run under another's MMAs; the CTA
+// meets only after the last chunk.  A tile with no slot in use (`active`
+// false) takes part in the handing back only.  phases: the parities of the
+// next phase of the full (bits 0-2) and empty (bits 3-5) mbarriers.
+//
+// A function of its own, so that its registers are not allocated under the
+// pressure of phase B (inlined, the chunk loop reloaded spilled operands).
+template <int NTF, int PPN, int NT, int NBK, int PAIR, int NW>
+__device__ __noinline__ bool phase_a_rows8(const PhaseA x, bool active, unsigned phases)
 {
-    static_assert(NW == 8 || NTF > 0, "the 4-warp shape runs the fused contractions only");
-    constexpr int kThreads = NW * 32, kWarps = NW;
+    static_assert(!PAIR || PPN == 0, "direction pairs: Mn");
+    static_assert(NW == 16 || NW == 8, "32 or 16 slots per CTA");
     extern __shared__ __align__(16) double sm[];
-    __shared__ int ctl[4];   // [0] problem, [1] done, [2] exhausted, [3] next slot of phase B
+    constexpr int DEPTH = (NW == 16) ? 3 : 2;    // staged chunk buffers
+    constexpr int kq = 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int mt = warp >> 2, qg = warp & 3;     // a tile's four warps on four schedulers
+    const int r0 = mt * 8 + g;
+    const int ldG = x.ldG, nb = (NBK > 0) ? 8 * NBK : x.nb, ldP = x.ldP;
+    constexpr int NTL = (NT > 0) ? NT : NTF;
+    constexpr int KSL = (NBK > 0) ? NBK : 4;
+    constexpr int NTE = PAIR / 16, NBE = PAIR % 16;
+    const int NTH = (NT > 0) ? NT - (PPN ? NBK : 0) : x.K2p / 8;
+    const int NT2 = (NT > 0) ? NT : NTH + (PPN ? nb / 8 : 0);
+    const int nchunks = x.nchunks;
+    const int chunkDoubles = kq * ldP + kq;
+    double *const sP = sm + x.offP;
+    const double *const exptab = sm + x.offExp;
+    double acc[NTL][2];
+#pragma unroll
+    for (int j = 0; j < NTL; j++)
+        acc[j][0] = acc[j][1] = 0.0;
+    double facc = 0.0;
+    const double invL = x.invL, L1 = x.L1, L2 = x.L2;
+    const unsigned chunkBytes = (unsigned)chunkDoubles * 8u;
+    unsigned long long *full = reinterpret_cast<unsigned long long *>(sm + x.offBar), *empty = full + 3;
+    unsigned pending = 0;   // thread 0: buffers with a copy issued and not yet waited for
+    auto load_chunk = [&](int c, int buf) {
+        mbar_expect_tx(&full[buf], chunkBytes);
+        bulk_copy_g2s(sP + buf * chunkDoubles, x.P + (size_t)c * chunkDoubles, chunkBytes, &full[buf]);
+        pending |= 1u << buf;
+    };
+    auto wait_full = [&](int buf) -> bool {
+        const bool ok = mbar_wait_bounded(&full[buf], (phases >> buf) & 1u, kWaitNs);
+        phases ^= 1u << buf;
+        pending &= ~(1u << buf);
+        return ok;
+    };
+    auto release = [&](int buf) {
+        __syncwarp();
+        if (lane == 0)
+            mbar_arrive(&empty[buf]);
+    };
+    const int offA = basis_row(qg * 8 + g, ldP) + t4;        // GEMM1 B row
+    const int qb = qg * 8 + 2 * t4;                          // GEMM2 B rows qb, qb + 1
+    const int wOff = basis_wgap(qb, ldP);
+    const int offB = basis_row(qb, ldP) + g;
+    // this slot's multipliers, columns 8 ks + t4 and 8 ks + t4 + 4
+    const double *const al = sm + x.offAlpha + r0 * x.ldv;
+    double aA[2 * KSL];
+#pragma unroll
+    for (int k2 = 0; k2 < 2 * KSL; k2++) {
+        const int c = k2 * 4 + t4;
+        if constexpr (PAIR != 0) {
+            const int k = x.binv[c];
+            aA[k2] = (k >= 0) ? al[k] : 0.0;
+        } else {
+            aA[k2] = (NBK > 0 || k2 * 4 < nb) ? al[c] : 0.0;
+        }
+    }
+    double e[2], eg[2];
+    // S of the chunk at Pc: cs (PAIR: even half sums), co (odd ones)
+    auto gemm1 = [&](const double *Pc, double (&cs)[2], double (&co)[2]) {
+        cs[0] = cs[1] = co[0] = co[1] = 0.0;
+        const double *B1 = Pc + offA;
+#pragma unroll
+        for (int k2 = 0; k2 < 2 * KSL; k2++) {
+            if (PAIR && k2 >= 2 * NBE)
+                dmma8x8x4(co, aA[k2], B1[k2 * 4]);
+            else if (NBK > 0 || k2 * 4 < nb)
+                dmma8x8x4(cs, aA[k2], B1[k2 * 4]);
+        }
+    };
+    // its weights: e (Hessian weights; PAIR: pair sums) and eg (PPn gradient
+    // weights; PAIR: pair differences)
+    auto weights = [&](const double *Pc, const double (&cs)[2], const double (&co)[2]) {
+        const double w0 = Pc[wOff], w1 = Pc[wOff + 1];
+        if constexpr (PAIR != 0) {
+            double sv[4], y[4];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                sv[h] = cs[h] + co[h];
+                sv[2 + h] = cs[h] - co[h];
+            }
+            fast_exp_n<4>(y, sv, exptab, invL, L1, L2);
+            pair_weights(e[0], eg[0], y[0], y[2], w0);
+            pair_weights(e[1], eg[1], y[1], y[3], w1);
+            facc += pair_f(y[0], y[1], y[2], y[3], w0, w1);
+        } else if constexpr (PPN == 0) {
+            fast_exp_n<2>(e, cs, exptab, invL, L1, L2);
+            e[0] *= w0;
+            e[1] *= w1;
+            facc += e[0] + e[1];
+            eg[0] = eg[1] = 0.0;
+        } else {
+            // fobj.cpp:408-434 and :196-210 (PPn)
+            const double dl = sm[x.offScal + r0 * SC_N + SC_DELTA];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const double ww = h ? w1 : w0;
+                const double k = 0.5 * cs[h];
+                const double s2 = sqrt(k * k + dl);
+                double G = k + s2;
+                if (k < 0)
+                    G = -dl / (k - sqrt(k * k + dl));
+                e[h] = 0.5 * ww * (G / s2);
+                eg[h] = ww * G;
+                facc += ww * (k * G - 0.5 * dl + dl * log(G));
+            }
+        }
+    };
+    // G += E . Phess of the chunk at Pc; k-slots 0-3 are the rows 2 t4, 4-7
+    // the rows 2 t4 + 1, as in the 16-slot tiles.  Row by row: no MMA waits
+    // for the one before it.
+    auto gemm2 = [&](const double *Pc) {
+        const double *B2 = Pc + offB;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+#pragma unroll
+            for (int nt = 0; nt < NTL; nt++) {
+                if (NT > 0 || nt < NT2) {
+                    const bool hess = (PPN == 0) || nt < NTH;
+                    const int col = hess ? nb + nt * 8 : (nt - NTH) * 8;
+                    const bool useE = PAIR ? (nt < NTE) : hess;
+                    dmma8x8x4(acc[nt], useE ? e[h] : eg[h], B2[col + h * ldP]);
+                }
+            }
+        }
+    };
+    if (tid == 0)
+        for (int c = 0; c < DEPTH && c < nchunks; c++)
+            load_chunk(c, c);
+    bool ok = wait_full(0);
+    double cs[2], co[2];
+    if (active && ok) {
+        gemm1(sP, cs, co);
+        weights(sP, cs, co);
+    }
+    int bc = 0;   // buffer of chunk c
+    for (int c = 0; c < nchunks; c++) {
+        const int bp = (bc == 0) ? DEPTH - 1 : bc - 1, bn = (bc == DEPTH - 1) ? 0 : bc + 1;
+        const double *Pc = sP + bc * chunkDoubles, *Pn = sP + bn * chunkDoubles;
+        const bool next = c + 1 < nchunks;
+        // the buffer of chunk c - 1, once every warp has handed it back,
+        // takes chunk c - 1 + DEPTH
+        if (c > 0) {
+            if (tid == 0 && c - 1 + DEPTH < nchunks) {
+                ok = mbar_wait_bounded(&empty[bp], (phases >> (3 + bp)) & 1u, kWaitNs) && ok;
+                if (ok)
+                    load_chunk(c - 1 + DEPTH, bp);
+            }
+            phases ^= 8u << bp;   // one phase per chunk, waited for or not
+        }
+        if constexpr (DEPTH == 3) {
+            // chunk c + 1 is there already: one block of code in which its
+            // exponentials fill the gaps of chunk c's MMAs
+            if (next) {
+                ok = wait_full(bn) && ok;
+                if (!__all_sync(0xffffffffu, ok))
+                    break;
+                if (active) {
+                    gemm1(Pn, cs, co);
+                    gemm2(Pc);
+                    weights(Pn, cs, co);
+                }
+            } else if (active) {
+                gemm2(Pc);
+            }
+            release(bc);
+        } else {
+            // two buffers: chunk c's goes back before chunk c + 1 is needed
+            if (active)
+                gemm2(Pc);
+            release(bc);
+            if (next) {
+                ok = wait_full(bn) && ok;
+                if (!__all_sync(0xffffffffu, ok))
+                    break;
+                if (active) {
+                    gemm1(Pn, cs, co);
+                    weights(Pn, cs, co);
+                }
+            }
+        }
+        bc = bn;
+    }
+    // every warp is done with the staged basis (the G region overlaps it)
+    if (__syncthreads_or(!ok)) {
+        // a copy never arrived: wait (bounded) for those still in flight so
+        // that none lands in shared memory after the CTA has exited
+        if (tid == 0) {
+            record_error(x.err, -5, -1);
+            for (int b = 0; b < DEPTH; b++)
+                if (pending & (1u << b))
+                    mbar_wait_bounded(&full[b], (phases >> b) & 1u, kWaitNs);
+        }
+        return false;
+    }
+    // the four q-groups' partial sums of G, in q-group order
+    double *const G = sm + x.offG + r0 * ldG + 2 * t4;
+#pragma unroll 1
+    for (int step = 0; step < 4; step++) {
+        if (qg == step && active) {
+#pragma unroll
+            for (int nt = 0; nt < NTL; nt++) {
+                if (NT > 0 || nt < NT2) {
+                    double2 *G0 = reinterpret_cast<double2 *>(G + nt * 8);
+                    if (step == 0) {
+                        *G0 = make_double2(acc[nt][0], acc[nt][1]);
+                    } else {
+                        double2 v = *G0;
+                        v.x += acc[nt][0];
+                        v.y += acc[nt][1];
+                        *G0 = v;
+                    }
+                }
+            }
+        }
+        if (step < 3)
+            __syncthreads();
+    }
+    facc += __shfl_xor_sync(0xffffffffu, facc, 1);
+    facc += __shfl_xor_sync(0xffffffffu, facc, 2);
+    if (t4 == 0 && active)
+        sm[x.offFpart + r0 * x.ntq + qg] = facc;
+    __syncthreads();
+    return true;
+}
+
+template <int TPW, int NTF, int PPN, int NT, int NBK, int MIX, int PAIR, int NW, int NX>
+__global__ void __launch_bounds__(NW * 32, (NTF > 0 && !MIX && NW == 8) ? 2 : 1)
+    newton_kernel(const __grid_constant__ NewtonArgs a)
+{
+    // fused FP64 contractions: 8-slot tiles, 16 warps (32 slots) or 8 warps
+    // (16 slots, two CTAs per SM); the mixed and general ones: 8 warps, 32 slots
+    constexpr bool R8 = NTF > 0 && !MIX;
+    static_assert(R8 ? (NW == 16 || NW == 8) : NW == 8, "launch shapes");
+    constexpr int kThreads = NW * 32, kWarps = NW;
+    constexpr int NM = NX ? NX : (NBK > 0 && 8 * NBK < kMaxN) ? 8 * NBK : kMaxN;   // n <= nb = 8 NBK
+    extern __shared__ __align__(16) double sm[];
+    // [0] problem, [1] done, [2] exhausted, [3] next slot of phase B, [4] problems whose first share is taken
+    __shared__ int ctl[5];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t4 = lane & 3;
     const int T = a.T, MT = a.T / 16, kq = a.kq, ldv = a.ldv, ldE = a.ldE, ldG = a.ldG;
@@ -1894,31 +2271,37 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) newton_kernel(const 
         ctl[0] = 0;
         ctl[1] = 0;
         ctl[2] = 0;
-    }
-    if (tid == 0) {
-        for (int b = 0; b < 3; b++)
+        ctl[4] = 0;
+        for (int b = 0; b < 3; b++) {
             mbar_init(&L.bar[b], 1);
+            mbar_init(&L.bar[3 + b], kWarps);
+        }
         mbar_init_fence();
     }
     __syncthreads();
     int loadedProb = -1;
-    unsigned mbPhase = 0;   // parity of the next phase of each chunk mbarrier
+    unsigned mbPhase = 0;   // parity of the next phase of each chunk mbarrier (full; empty three bits up)
 
     for (;;) {
-        // ---- refill idle slots from the work counter of the current problem
-        if (tid == 0) {
+        // ---- refill idle slots from the work counter of the current problem:
+        // warp 0, lane s for slot s.  A launch with fewer vectors than slots
+        // spreads them over the CTAs (quota per CTA): the first quota of each
+        // CTA are the vectors blockIdx.x + k * gridDim.x, so that the longest
+        // chains, listed first, fall to different CTAs; the work counter hands
+        // out the rest.
+        if (warp == 0) {
+            int *si = L.ints + lane * SI_N;
+            const bool mine = lane < T;
             int p = ctl[0];
-            int nIdle = 0, nActive = 0;
-            for (int s = 0; s < T; s++) {
-                if (L.ints[s * SI_N + SI_STATE] == S_HELP)   // helpers serve one round
-                    L.ints[s * SI_N + SI_STATE] = S_IDLE;
-                if (L.ints[s * SI_N + SI_STATE] == S_IDLE)
-                    nIdle++;
-                else
-                    nActive++;
+            int st = mine ? si[SI_STATE] : -1;
+            if (st == S_HELP) {   // helpers serve one round
+                st = S_IDLE;
+                si[SI_STATE] = S_IDLE;
             }
+            unsigned idle = __ballot_sync(0xffffffffu, st == S_IDLE);
+            int nActive = T - __popc(idle);
             bool exhausted = ctl[2] != 0;
-            while (nIdle > 0) {
+            while (idle) {
                 if (exhausted) {
                     if (nActive == 0 && p + 1 < a.nprob) {
                         p++;
@@ -1930,46 +2313,60 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) newton_kernel(const 
                 const NewtonProblem &pb = a.prob[p];
                 const bool list = pb.cellList && *pb.countDev >= 0;
                 const int count = list ? *pb.countDev : pb.count;
-                unsigned base = atomicAdd(pb.queue, (unsigned)nIdle);
-                if (base >= (unsigned)count) {
-                    exhausted = true;
-                    continue;
+                const int quota = (count + (int)gridDim.x - 1) / (int)gridDim.x;
+                const int cap = min(T, quota);
+                int item = -1;   // this lane's vector
+                const int rank = __popc(idle & ((1u << lane) - 1u));
+                const bool isIdle = (idle >> lane) & 1u;
+                if (nActive == 0 && ctl[4] <= p) {
+                    // the CTA's first vectors of this problem
+                    const int at = (int)blockIdx.x + rank * (int)gridDim.x;
+                    if (isIdle && rank < cap && at < count)
+                        item = at;
+                    __syncwarp();
+                    if (lane == 0)
+                        ctl[4] = p + 1;
+                    __syncwarp();
+                    if (cap == quota)   // quota <= T: the CTAs took everything
+                        exhausted = true;
+                } else {
+                    const int want = __popc(idle);
+                    unsigned base = 0;
+                    if (lane == 0)
+                        base = atomicAdd(pb.queue, (unsigned)want);
+                    base = __shfl_sync(0xffffffffu, base, 0);
+                    const long long at = (long long)cap * gridDim.x + base + rank;
+                    if (isIdle && at < count)
+                        item = (int)at;
+                    if ((long long)cap * gridDim.x + base + want > count)
+                        exhausted = true;
                 }
-                int take = min(nIdle, count - (int)base);
-                int c = 0;
-                for (int s = 0; s < T && c < take; s++) {
-                    if (L.ints[s * SI_N + SI_STATE] == S_IDLE) {
-                        L.ints[s * SI_N + SI_CELL] = list ? pb.cellList[(int)base + c] : pb.first + (int)base + c;
-                        L.ints[s * SI_N + SI_STATE] = S_NEW;
-                        c++;
-                    }
+                if (item >= 0) {
+                    si[SI_CELL] = list ? pb.cellList[item] : pb.first + item;
+                    si[SI_STATE] = S_NEW;
                 }
-                nIdle -= take;
-                nActive += take;
-                if (nIdle > 0)
-                    exhausted = true;
+                const unsigned got = __ballot_sync(0xffffffffu, item >= 0);
+                nActive += __popc(got);
+                idle &= ~got;
             }
             // idle slots once the work counter is exhausted: lend them to
-            // slots whose line search is backtracking (plain Newton)
-            if (a.optType == 0 && exhausted && nIdle > 0) {
-                for (int s = 0; s < T && nIdle > 0; s++) {
-                    if (L.ints[s * SI_N + SI_STATE] != S_TRIAL || !(L.scal[s * SC_N + SC_T] < 1.0))
-                        continue;
-                    int k = 0;
-                    for (int h = 0; h < T && nIdle > 0; h++) {
-                        if (L.ints[h * SI_N + SI_STATE] == S_IDLE) {
-                            L.ints[h * SI_N + SI_STATE] = S_HELP;
-                            L.ints[h * SI_N + SI_CELL] = s;
-                            L.ints[h * SI_N + SI_ITER] = ++k;
-                            nIdle--;
-                        }
-                    }
+            // slots whose line search is backtracking (plain Newton), the
+            // first such slot first
+            if (a.optType == 0 && exhausted && idle) {
+                __syncwarp();
+                const unsigned back = __ballot_sync(0xffffffffu, st == S_TRIAL && L.scal[lane * SC_N + SC_T] < 1.0);
+                if (back && ((idle >> lane) & 1u)) {
+                    si[SI_STATE] = S_HELP;
+                    si[SI_CELL] = __ffs(back) - 1;
+                    si[SI_ITER] = 1 + __popc(idle & ((1u << lane) - 1u));
                 }
             }
-            ctl[0] = p;
-            ctl[2] = exhausted ? 1 : 0;
-            ctl[1] = (nActive == 0) ? 1 : 0;
-            ctl[3] = 0;
+            if (lane == 0) {
+                ctl[0] = p;
+                ctl[2] = exhausted ? 1 : 0;
+                ctl[1] = (nActive == 0) ? 1 : 0;
+                ctl[3] = 0;
+            }
         }
         __syncthreads();
         if (ctl[1])
@@ -1980,9 +2377,9 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) newton_kernel(const 
             // (or read it from global memory through L1 where the launch
             // shape leaves no room for it)
             loadedProb = ctl[0];
-            // (a compile-time choice: the 8-warp shape's table pointers stay
+            // (a compile-time choice: the 32-slot shape's table pointers stay
             // shared-memory pointers, which the loads in phase B rely on)
-            if constexpr (NW != 8) {
+            if constexpr (R8 && NW == 8) {
                 if (a.useGaunt) {
                     L.ellVal = const_cast<double *>(pb.ellVal);
                     L.ellIdx = const_cast<unsigned short *>(pb.ellIdx);
@@ -1990,11 +2387,11 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) newton_kernel(const 
                     L.ellOff = const_cast<int *>(pb.ellOff);
                 }
             } else if (a.useGaunt) {
-                for (int i = tid; i < pb.ellRows * 32; i += kThreads) {
+                for (int i = tid; i < pb.ellGroups * 256; i += kThreads) {
                     L.ellVal[i] = pb.ellVal[i];
                     L.ellIdx[i] = pb.ellIdx[i];
                 }
-                for (int i = tid; i < pb.ellChunks * 32; i += kThreads)
+                for (int i = tid; i < pb.ellChunks * 64; i += kThreads)
                     L.ellPair[i] = pb.ellPair[i];
                 for (int i = tid; i <= pb.ellChunks; i += kThreads)
                     L.ellOff[i] = pb.ellOff[i];
@@ -2010,8 +2407,39 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) newton_kernel(const 
         __syncthreads();
 
         // ---- phase A: evaluation contractions over the quadrature
-        if constexpr (NTF > 0) {
-            if (!phase_a_fused<NTF, PPN, NT, NBK, MIX, PAIR, NW>(a, pb, L, tid, lane, warp, mbPhase))
+        if constexpr (R8) {
+            const int s8 = (warp >> 2) * 8 + (lane & 7);
+            const bool active = __any_sync(0xffffffffu, L.ints[s8 * SI_N + SI_STATE] != S_IDLE);
+            PhaseA x;
+            x.offAlpha = a.offAlpha;
+            x.offScal = a.offScal;
+            x.offFpart = a.offFpart;
+            x.offP = a.offP;
+            x.offG = a.offG;
+            x.offExp = a.offExp;
+            x.offBar = a.offBar;
+            x.ldv = ldv;
+            x.ldG = ldG;
+            x.ntq = a.ntq;
+            x.nb = pb.nb;
+            x.ldP = pb.ldP;
+            x.K2p = pb.K2p;
+            x.nchunks = pb.nqp / 32;
+            x.P = pb.P;
+            x.binv = pb.binv;
+            x.invL = a.ex.invL;
+            x.L1 = a.ex.L1;
+            x.L2 = a.ex.L2;
+            x.err = a.err;
+            if (!phase_a_rows8<NTF, PPN, NT, NBK, PAIR, NW>(x, active, mbPhase))
+                return;   // a staged chunk never arrived (error recorded)
+            // each buffer's barriers went through a phase per chunk it held
+            constexpr int DEPTH = (NW == 16) ? 3 : 2;
+            for (int b = 0; b < DEPTH; b++)
+                if (((x.nchunks - b + DEPTH - 1) / DEPTH) & 1)
+                    mbPhase ^= 9u << b;
+        } else if constexpr (NTF > 0) {
+            if (!phase_a_fused<NTF, PPN, NT, NBK, MIX, PAIR>(a, pb, L, tid, lane, warp, mbPhase))
                 return;   // a staged chunk never arrived (error recorded)
         } else {
         const int nb = pb.nb, ldP = pb.ldP, K2p = pb.K2p;
@@ -2159,9 +2587,9 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) newton_kernel(const 
             int st = L.ints[s * SI_N + SI_STATE];
             if (st == S_NEWTON || st == S_TRIAL) {
                 if (a.optType != 0)
-                    slot_logic_cb(a, pb, L, s, lane, warp);
+                    slot_logic_cb<NM, NX>(a, pb, L, s, lane, warp);
                 else
-                    slot_logic(a, pb, L, s, lane, warp, PPN == 0 && MIX == 0);
+                    slot_logic<NM, NX>(a, pb, L, s, lane, warp, PPN == 0 && MIX == 0);
             }
         }
         if constexpr (NTF > 0)
@@ -2374,7 +2802,7 @@ __global__ void __launch_bounds__(256, 2) screen_kernel(const __grid_constant__ 
             if (L.ints[s * SI_N + SI_STATE] == S_NEW)
                 init_slot(a, pb, L, s, lane, ldv);
         __syncthreads();
-        if (!phase_a_fused<8, 0, NT, NBK, 0, 1, 8>(a, pb, L, tid, lane, warp, mbPhase))
+        if (!phase_a_fused<8, 0, NT, NBK, 0, 1>(a, pb, L, tid, lane, warp, mbPhase))
             return;   // a staged chunk never arrived (error recorded)
         for (;;) {
             int s = 0;
@@ -2445,10 +2873,10 @@ cudaError_t screen_run(const NewtonArgs &a, int grid, cudaStream_t stream, int m
 
 // One kernel instance: mode 0 launches it, 1 sets its shared-memory limit,
 // 2 writes its resident CTAs per SM to *occ.
-template <int TPW, int NTF, int PPN, int NT, int NBK, int MIX = 0, int PAIR = 0, int NW = 8>
+template <int TPW, int NTF, int PPN, int NT, int NBK, int MIX = 0, int PAIR = 0, int NW = (NTF > 0 && !MIX) ? 16 : 8, int NX = 0>
 cudaError_t newton_run(const NewtonArgs &a, int grid, cudaStream_t stream, int mode, int *occ)
 {
-    auto *k = newton_kernel<TPW, NTF, PPN, NT, NBK, MIX, PAIR, NW>;
+    auto *k = newton_kernel<TPW, NTF, PPN, NT, NBK, MIX, PAIR, NW, NX>;
     if (mode == 1)
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smemBytes);
     if (mode == 2) {

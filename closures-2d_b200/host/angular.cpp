@@ -246,7 +246,7 @@ void product_columns(int n, unsigned short *pairs)
 }
 
 int build_gaunt_ell(int n, const int *off, const int *idx, const double *val, unsigned short *pair,
-                    unsigned short *eidx, double *eval, int *eoff, int maxRows)
+                    unsigned short *eidx, double *eval, int *eoff, int maxGroups)
 {
     const int np = n * (n + 1) / 2;
     int pi[528], pj[528], pc[528];   // n <= 32
@@ -274,31 +274,33 @@ int build_gaunt_ell(int n, const int *off, const int *idx, const double *val, un
         pc[b + 1] = tc;
     }
     const int chunks = gaunt_ell_chunks(n);
-    int rows = 0;
+    int groups = 0;
     for (int c = 0; c < chunks; c++) {
-        eoff[c] = rows;
-        int rc = 0;
-        for (int l = 0; l < 32; l++) {
-            int p = c * 32 + l;
-            if (p < m && pc[p] > rc)
-                rc = pc[p];
+        eoff[c] = groups;
+        int gc = 0;
+        for (int l = 0; l < 64; l++) {
+            int p = c * 64 + l;
+            if (p < m && (pc[p] + 3) / 4 > gc)
+                gc = (pc[p] + 3) / 4;
         }
-        if (rows + rc > maxRows)
+        if (groups + gc > maxGroups)
             return -1;
-        for (int l = 0; l < 32; l++) {
-            int p = c * 32 + l;
-            pair[c * 32 + l] = (p < m) ? (unsigned short)((pi[p] << 8) | pj[p]) : (unsigned short)0xFFFF;
+        for (int l = 0; l < 64; l++) {
+            int p = c * 64 + l;
+            pair[p] = (p < m) ? (unsigned short)((pi[p] << 8) | pj[p]) : (unsigned short)0xFFFF;
             int r0 = (p < m) ? off[pi[p] * n + pj[p]] : 0;
-            for (int e = 0; e < rc; e++) {
+            const int lane = l & 31, h = l >> 5;
+            for (int e = 0; e < 4 * gc; e++) {
                 bool live = p < m && e < pc[p];
-                eidx[(size_t)(rows + e) * 32 + l] = live ? (unsigned short)idx[r0 + e] : (unsigned short)0;
-                eval[(size_t)(rows + e) * 32 + l] = live ? val[r0 + e] : 0.0;
+                const size_t g = groups + e / 4;
+                eidx[(g * 32 + lane) * 8 + h * 4 + e % 4] = live ? (unsigned short)idx[r0 + e] : (unsigned short)0;
+                eval[((g * 4 + h * 2 + e % 4 / 2) * 32 + lane) * 2 + e % 2] = live ? val[r0 + e] : 0.0;
             }
         }
-        rows += rc;
+        groups += gc;
     }
-    eoff[chunks] = rows;
-    return rows;
+    eoff[chunks] = groups;
+    return groups;
 }
 
 }  // namespace clb

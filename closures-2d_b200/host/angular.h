@@ -22,16 +22,21 @@ int build_angular(int order, int Q, int useGaunt, Angular &A);
 namespace clb {
 
 // Gaunt contraction H_ij = sum_k c_ijk G_k (fobj.cpp:130-144) rearranged for
-// 32 lanes: the upper pairs (i <= j, CSR row i*n+j) are sorted by entry count
-// and grouped 32 to a chunk; chunk c holds rows eoff[c]..eoff[c+1]-1 of
-// [row][lane] entries (eidx, eval), zero padded, each pair's entries in CSR
-// order so the sum is formed in the reference's order.  pair[c*32+lane] is
-// (i << 8) | j, or 0xFFFF for an empty lane.  Fills caller buffers (no
-// allocation); returns the number of rows, or -1 if maxRows is too small.
-// Buffer sizes: pair and eoff for ceil(n(n+1)/2 / 32) chunks (+1 for eoff).
+// 32 lanes of two pairs each: the upper pairs (i <= j, CSR row i*n+j) are
+// sorted by entry count and taken 64 to a chunk, lane l holding pairs l and
+// 32 + l of it.  Chunk c has the entry groups eoff[c]..eoff[c+1]-1 of four
+// entries per pair, zero padded, each pair's entries in CSR order so the sum
+// is formed in the reference's order:
+//   eidx[(group*32 + lane)*8 + h*4 + e]                     (one 16-byte load)
+//   eval[((group*4 + h*2 + e/2)*32 + lane)*2 + e%2]         (16-byte loads)
+// for entry e of pair h.  pair[c*64 + h*32 + lane] is (i << 8) | j, or 0xFFFF
+// for an empty place.  Fills caller buffers (no allocation); returns the
+// number of groups (256 entries each), or -1 if maxGroups is too small.
+// pair holds 64 and eoff one entry per chunk (+1 for eoff).
 int build_gaunt_ell(int n, const int *off, const int *idx, const double *val, unsigned short *pair,
-                    unsigned short *eidx, double *eval, int *eoff, int maxRows);
-inline int gaunt_ell_chunks(int n) { return (n * (n + 1) / 2 + 31) / 32; }
+                    unsigned short *eidx, double *eval, int *eoff, int maxGroups);
+constexpr int kEllGroup = 256;   // entries per group
+inline int gaunt_ell_chunks(int n) { return (n * (n + 1) / 2 + 63) / 64; }
 
 // Column order of the packed Hessian products p_i p_j (j <= i) used without
 // the Gaunt table: the n products with p_0 first (they hold the gradient and

@@ -214,9 +214,9 @@ int cl_set_last_iterations(cl_ctx *ctx, const int *iters);
  * per-cell loop is an OpenMP schedule(dynamic,1) over cells
  * (momopt_update.cpp:208-277, :214).  Candidates, each run on copies of the
  * context's current state (the real state is untouched):
- *   K1 (Newton):  cells per CTA and warps -- 32 cells / 8 warps / one CTA
- *                 per SM, or 16 cells / 4 warps / two CTAs per SM (the
- *                 direction-pair layout) -- and the Hessian tile layout:
+ *   K1 (Newton):  cells per CTA -- 32 and one CTA per SM, or 16 and two
+ *                 CTAs per SM (the direction-pair layout); the FP64 instances
+ *                 run a warp per two cells -- and the Hessian tile layout:
  *                 direction pairs (even/odd degree column tiles) or one
  *                 direction at a time, where both exist (Mn, FP64);
  *   K2+K3 (flux): the same two tile layouts.
@@ -232,7 +232,7 @@ int cl_set_last_iterations(cl_ctx *ctx, const int *iters);
  * the same sums in another order. */
 #define CL_TUNE_MAX 8
 typedef struct {
-    int newton_warps;         /* K1 warps per CTA: 8 (32 cells per CTA) or 4 (16) */
+    int newton_warps;         /* K1 launch shape: 8 (32 cells per CTA) or 4 (16) */
     int newton_ctas;          /* K1 persistent CTAs per launch */
     int newton_contraction;   /* K1 Hessian tile layout: CL_CONTRACT_PAIRS or _SINGLE */
     int flux_contraction;     /* K2+K3 tile layout */
@@ -248,7 +248,7 @@ int cl_tune(cl_ctx *ctx, int use_cache, cl_tuning *out);   /* use_cache 0: alway
 /* The shapes in use (after cl_tune, cl_set_launch_shape or the defaults). */
 int cl_get_tuning(cl_ctx *ctx, cl_tuning *out);
 /* Forces the shapes (CL_ERR_ARG where the configuration has no such
- * instance): newton_warps 8 or 4, contractions CL_CONTRACT_PAIRS/_SINGLE. */
+ * instance): newton_warps 8 (32 cells per CTA) or 4 (16), contractions CL_CONTRACT_PAIRS/_SINGLE. */
 int cl_set_launch_shape(cl_ctx *ctx, int newton_warps, int newton_contraction, int flux_contraction);
 /* The exponent-range test of K1 (on by default; Mn in FP64): an evaluation
  * whose gradient meets the tolerance converges without forming the Hessian
