@@ -560,6 +560,8 @@ struct cl_ctx {
     cl_mlp *warm = nullptr;           // learned warm start (null: previous stage's alpha)
     int warmMinIters = 0;             // > 0: predict only cells whose previous stage took this many iterations
     double *dAlphaPred = nullptr;     // [C][n] predicted starts when warm is set
+    double *dFluxF = nullptr;         // stencil fluxes of a shared-out direction loop (small grids)
+    int *dTileRun = nullptr;          // whether each tile ran its direction loop
     double *dP2M = nullptr, *dAlphaP = nullptr;   // change-of-basis state per cell (opt type 1)
     double *dCbScratch = nullptr;     // working basis per Newton slot (opt type 1)
     NewtonArgs nargs;
@@ -884,6 +886,16 @@ int cl_create(const cl_grid *grid, const cl_options *opts, const cl_angular *ang
         ctx->err = std::string("flux kernel attributes: ") + cudaGetErrorString(ce);
         return ctx_fail(ctx, CL_ERR_CUDA);
     }
+    f.sms = sm_count();
+    if (const size_t fd = flux_split_doubles(f)) {
+        if (cudaMalloc(&ctx->dFluxF, fd * sizeof(double)) != cudaSuccess ||
+            cudaMalloc(&ctx->dTileRun, (size_t)f.tilesX * f.tilesY * sizeof(int)) != cudaSuccess) {
+            ctx->err = "device allocation failed";
+            return ctx_fail(ctx, CL_ERR_CUDA);
+        }
+        f.F = ctx->dFluxF;
+        f.tileRun = ctx->dTileRun;
+    }
     if (cudaDeviceSynchronize() != cudaSuccess) {
         ctx->err = std::string("set-up: ") + cudaGetErrorString(cudaGetLastError());
         return ctx_fail(ctx, CL_ERR_CUDA);
@@ -926,6 +938,8 @@ void cl_destroy(cl_ctx *ctx)
     cudaFreeHost(ctx->hErr);
     cudaFree(ctx->dIters);
     cudaFree(ctx->dAlphaPred);
+    cudaFree(ctx->dFluxF);
+    cudaFree(ctx->dTileRun);
     cudaFree(ctx->dP2M);
     cudaFree(ctx->dAlphaP);
     cudaFree(ctx->dCbScratch);
@@ -1093,10 +1107,7 @@ static cudaError_t enqueue_stage(cl_ctx *ctx, int stage, double dt, double dx, d
     f.dx = dx;
     f.dy = dy;
     f.momentsOld = (stage == 1) ? ctx->dOld : nullptr;
-    if ((e = launch_flux(f, ctx->stream)) != cudaSuccess)
-        return e;
-    *nk += 1;
-    return cudaSuccess;
+    return launch_flux(f, ctx->stream, nk);
 }
 
 // Enqueues one RK2 step on the context's stream (uncaptured form).
@@ -1210,8 +1221,7 @@ int cl_step_timed(cl_ctx *ctx, double dt, double dx, double dy, float *ms)
         f.dy = dy;
         f.momentsOld = (stage == 1) ? ctx->dOld : nullptr;
         if (e == cudaSuccess)
-            e = launch_flux(f, ctx->stream);
-        nk++;
+            e = launch_flux(f, ctx->stream, &nk);
         cudaEventRecord(ev[3 * stage + 2], ctx->stream);
     }
     g_launches += nk;
@@ -1434,8 +1444,7 @@ int cl_step_host(cl_ctx *ctx, double dt, double dx, double dy, double *moments, 
         f.momentsOld = (stage == 1) ? ctx->dOld : nullptr;
         if (stage == 0) {
             if (e == cudaSuccess)
-                run(launch_flux(f, S));
-            nk++;
+                run(launch_flux(f, S, &nk));
             continue;
         }
         // the multipliers are final: read them back under the flux
@@ -1452,16 +1461,14 @@ int cl_step_host(cl_ctx *ctx, double dt, double dx, double dy, double *moments, 
         size_t rowsA = 0;
         if (tA > 0) {
             if (e == cudaSuccess)
-                run(launch_flux_tiles(f, 0, tA, S));
-            nk++;
+                run(launch_flux_tiles(f, 0, tA, S, &nk));
             rowsA = 2 + (size_t)fullRows * flux_tile_rows(f);
             run(cudaEventRecord(ctx->evFlux, S));
             run(cudaStreamWaitEvent(X, ctx->evFlux, 0));
             run(cudaMemcpyAsync(moments, ctx->dMom, rowsA * rowBytes, cudaMemcpyDeviceToHost, X));
         }
         if (e == cudaSuccess)
-            run(launch_flux_tiles(f, tA, tiles - tA, S));
-        nk++;
+            run(launch_flux_tiles(f, tA, tiles - tA, S, &nk));
         run(cudaMemcpyAsync(moments + rowsA * ctx->NY * n, ctx->dMom + rowsA * ctx->NY * n,
                             C * n * 8 - rowsA * rowBytes, cudaMemcpyDeviceToHost, S));
     }
@@ -1672,9 +1679,10 @@ static float time_flux(cl_ctx *ctx, FluxArgs f, TuneScratch &S)
         if (cudaMemcpyAsync(S.u, ctx->dMom, C * n * 8, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
             return -1.0f;
         cudaEventRecord(S.e0, st);
-        if (launch_flux(f, st) != cudaSuccess)
+        int nk = 0;
+        if (launch_flux(f, st, &nk) != cudaSuccess)
             return -1.0f;
-        g_launches++;
+        g_launches += nk;
         cudaEventRecord(S.e1, st);
         if (cudaStreamSynchronize(st) != cudaSuccess)
             return -1.0f;

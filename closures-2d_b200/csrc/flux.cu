@@ -40,6 +40,7 @@ __device__ __forceinline__ int halo_cell(int r)
     r -= TX * HY;
     return (TX + 2 + r / TY) * HY + 2 + r % TY;
 }
+constexpr size_t kSplitBytes = (size_t)512 << 20;   // most memory the stencil fluxes may take
 constexpr int kFluxThreads = 512;          // 16 warps: one interior m-tile each
 constexpr int kFluxWarps = kFluxThreads / 32;
 constexpr int kQ = 16;                     // directions per chunk
@@ -85,6 +86,49 @@ __device__ __forceinline__ void closure_n(double (&v)[K], const double (&kin)[K]
     }
 }
 
+// Euler + collision + source (+ Heun average) of the 16 cells of m-tile mt
+// from their projected fluxes.
+template <int PAIR>
+__device__ __forceinline__ void flux_update(const FluxArgs &f, const double (&acc)[4][4], int i0, int j0, int mt, int g,
+                                            int t4)
+{
+    const int n = f.n, NTf = f.nb / 8;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        if (j >= NTf)
+            continue;
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            int ic = mt * 16 + g + ((h & 2) ? 8 : 0);
+            int k = j * 8 + 2 * t4 + (h & 1);
+            if (PAIR)
+                k = f.binv[k];
+            int i = i0 + ic / TY, jj = j0 + ic % TY;
+            if (k < 0 || k >= n || i >= f.NX - 2 || jj >= f.NY - 2)
+                continue;
+            size_t cell = (size_t)i * f.NY + jj;
+            double st = f.sigmaT[cell], ss = f.sigmaS[cell];
+            double u = f.moments[cell * n + k];
+            double F = acc[j][h];
+            double dt = f.dt;
+            double v;
+            if (k == 0)
+                v = u * (1.0 + dt * ss - dt * st) - dt * F;
+            else
+                v = u * (1.0 - dt * st) - dt * F;
+            if (k == 0 && f.initCond == 1) {
+                double x = f.initX + (i - 2) * f.dx;
+                double y = f.initY + (jj - 2) * f.dy;
+                if (fabs(x) < 0.5 && fabs(y) < 0.5)
+                    v = v + dt * 2.0 * kSqrtPi;
+            }
+            if (f.momentsOld != nullptr)
+                v = 0.5 * (v + f.momentsOld[cell * n + k]);
+            f.moments[cell * n + k] = v;
+        }
+    }
+}
+
 // PAIR = 1: direction pairs.  Directions q and q + Q (phi and phi + pi) have
 // the same weight and p_l(q + Q) = (-1)^l p_l(q), so with the basis columns
 // grouped by degree parity one MMA chain per parity gives both exponents,
@@ -92,7 +136,16 @@ __device__ __forceinline__ void closure_n(double (&v)[K], const double (&kin)[K]
 // takes F(q) + F(q + Q) on the even columns and F(q) - F(q + Q) on the odd
 // ones: half the tensor-core work of one direction at a time.  The stencil
 // is per direction either way.
-template <int PAIR>
+//
+// SPLIT = 1: a grid of few tiles (a 36 x 74 grid has 15) leaves most SMs idle
+// through the whole direction loop.  blockIdx.y then takes one share of the
+// chunks and leaves their stencil fluxes F in global memory, and
+// flux_project_kernel projects them, every cell's sum over the directions in
+// the order it has here.  Per stage: 50 x 50 M2, Q = 20 (16 tiles) 165 us
+// before; a whole RK2 step went from 467 to 274 us, 36 x 74 M3, Q = 30 (15
+// tiles) from 854 to 415 us, PP3 from 1487 to 846 us, 200 x 200 M4 (169 tiles
+// on 148 SMs) from 3726 to 3547 us.
+template <int PAIR, int SPLIT>
 __global__ void __launch_bounds__(kFluxThreads, 1) flux_kernel(const __grid_constant__ FluxArgs f)
 {
     extern __shared__ __align__(16) double sm[];
@@ -207,7 +260,7 @@ __global__ void __launch_bounds__(kFluxThreads, 1) flux_kernel(const __grid_cons
             }
         }
     };
-    auto stencil = [&](const double *Qb) {
+    auto stencil = [&](const double *Qb, int chunk) {
         // 2. limited upwind stencil.  Thread (q = warp, column j = lane % 16)
         //    sweeps interior rows ib..ib+7 (ib = 8 * (lane / 16)) down its
         //    column: each slopefit of a cell is formed once and serves the
@@ -260,7 +313,8 @@ __global__ void __launch_bounds__(kFluxThreads, 1) flux_kernel(const __grid_cons
                 const double *hr = sA + q * ldA + (ib + j + 2) * HY;   // halo row, column c at hr[c + 2]
                 edge = (eta > 0) ? slopefit(hr[0], hr[1], hr[2], th) : slopefit(hr[17], hr[18], hr[19], th);
             }
-            double *out = sF + q * ldF + ib * TY + j;
+            double *out = SPLIT ? f.F + ((size_t)(tile - f.tileBase) * nchunks + chunk) * (kQ * IC) + q * IC + ib * TY + j
+                                : sF + q * ldF + ib * TY + j;
 #pragma unroll
             for (int r = 0; r < 8; r++) {
                 const double *row = col + (ib + r) * HY;
@@ -318,7 +372,9 @@ __global__ void __launch_bounds__(kFluxThreads, 1) flux_kernel(const __grid_cons
             }
         }
     };
-    load_chunk(0, 0);
+    const int cBegin = SPLIT ? (int)((long long)nchunks * blockIdx.y / gridDim.y) : 0;
+    const int cEnd = SPLIT ? (int)((long long)nchunks * (blockIdx.y + 1) / gridDim.y) : nchunks;
+    load_chunk(cBegin, 0);
     cp_async_wait<0>();
     __syncthreads();
     // A uniform neighbourhood: when every staged alpha of the tile and its
@@ -333,60 +389,84 @@ __global__ void __launch_bounds__(kFluxThreads, 1) flux_kernel(const __grid_cons
         const int h = idx / nb, c = idx % nb;
         differs |= __double_as_longlong(sAl[h * ldAl + c]) != __double_as_longlong(sAl[c]);
     }
-    const int nloop = (__syncthreads_or(differs) || !f.skipUniform) ? nchunks : 0;
-    if (tid == 0 && nloop > 0 && f.tilesRun != nullptr)
-        atomicAdd(f.tilesRun, 1ull);
-    if (nloop > 0)
-        ansatz(sP);   // chunk 0, buffer 0
+    const bool run = __syncthreads_or(differs) || !f.skipUniform;
+    if (tid == 0 && (!SPLIT || blockIdx.y == 0)) {
+        if (run && f.tilesRun != nullptr)
+            atomicAdd(f.tilesRun, 1ull);
+        if (SPLIT)
+            f.tileRun[tile - f.tileBase] = run ? 1 : 0;
+    }
+    if (run)
+        ansatz(sP);   // the first chunk, buffer 0
     __syncthreads();
-    for (int c = 0; c < nloop; c++) {
-        const int buf = c & 1;
-        if (c + 1 < nchunks)
+    for (int c = cBegin; run && c < cEnd; c++) {
+        const int buf = (c - cBegin) & 1;
+        if (c + 1 < cEnd)
             load_chunk(c + 1, buf ^ 1);   // the buffer of chunk c - 1, free since the last barrier
-        stencil(sQ + buf * 4 * kq);
+        stencil(sQ + buf * 4 * kq, c);
         cp_async_wait<0>();
         __syncthreads();   // the stencil flux of chunk c complete; chunk c + 1 staged
-        projection(sP + buf * kq * ldPf);
-        if (c + 1 < nchunks)
+        if (!SPLIT)
+            projection(sP + buf * kq * ldPf);
+        if (c + 1 < cEnd)
             ansatz(sP + (buf ^ 1) * kq * ldPf);
         __syncthreads();   // the ansatz of chunk c + 1 complete; chunk c's buffers free
     }
+    if (SPLIT)
+        return;
+    flux_update<PAIR>(f, acc, i0, j0, warp, g, t4);
+}
 
-    // epilogue: Euler + collision + source (+ Heun average)
+// Projection and update of the SPLIT form: a warp per 16 cells of a tile, the
+// chunks in order, F and the basis rows read through L2.
+constexpr int kProjWarps = 4;
+template <int PAIR>
+__global__ void __launch_bounds__(kProjWarps * 32) flux_project_kernel(const __grid_constant__ FluxArgs f)
+{
+    const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    const int local = blockIdx.x / (IC / 16 / kProjWarps);
+    const int mt = (blockIdx.x % (IC / 16 / kProjWarps)) * kProjWarps + (threadIdx.x >> 5);
+    const int tile = local + f.tileBase;
+    const int i0 = 2 + (tile / f.tilesY) * TX, j0 = 2 + (tile % f.tilesY) * TY;
+    constexpr int kr = PAIR ? kQ / 2 : kQ;
+    const int nchunks = f.nqp / kr, ldPf = f.ldPf, NTf = f.nb / 8;
+    double acc[4][4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        if (j >= NTf)
-            continue;
+    for (int j = 0; j < 4; j++)
+        acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0;
+    if (f.tileRun[local]) {
+        const double *F = f.F + (size_t)local * nchunks * (kQ * IC) + t4 * IC + mt * 16 + g;
+        const double *B = f.P + t4 * ldPf + g;
+#pragma unroll 4
+        for (int c = 0; c < nchunks; c++, F += kQ * IC, B += kr * ldPf) {
+            if (PAIR) {
+                const double f0 = F[0], f1 = F[8], f2 = F[4 * IC], f3 = F[4 * IC + 8];
+                const double p0 = F[8 * IC], p1 = F[8 * IC + 8], p2 = F[12 * IC], p3 = F[12 * IC + 8];
+                const double s0 = f0 + p0, s1 = f1 + p1, s2 = f2 + p2, s3 = f3 + p3;
+                const double d0 = f0 - p0, d1 = f1 - p1, d2 = f2 - p2, d3 = f3 - p3;
 #pragma unroll
-        for (int h = 0; h < 4; h++) {
-            int ic = warp * 16 + g + ((h & 2) ? 8 : 0);
-            int k = j * 8 + 2 * t4 + (h & 1);
-            if (PAIR)
-                k = f.binv[k];
-            int i = i0 + ic / TY, jj = j0 + ic % TY;
-            if (k < 0 || k >= n || i >= f.NX - 2 || jj >= f.NY - 2)
-                continue;
-            size_t cell = (size_t)i * f.NY + jj;
-            double st = f.sigmaT[cell], ss = f.sigmaS[cell];
-            double u = f.moments[cell * n + k];
-            double F = acc[j][h];
-            double dt = f.dt;
-            double v;
-            if (k == 0)
-                v = u * (1.0 + dt * ss - dt * st) - dt * F;
-            else
-                v = u * (1.0 - dt * st) - dt * F;
-            if (k == 0 && f.initCond == 1) {
-                double x = f.initX + (i - 2) * f.dx;
-                double y = f.initY + (jj - 2) * f.dy;
-                if (fabs(x) < 0.5 && fabs(y) < 0.5)
-                    v = v + dt * 2.0 * kSqrtPi;
+                for (int j = 0; j < 4; j++) {
+                    if (j < NTf) {
+                        if (j * 8 < f.nbe)
+                            dmma16x8x8(acc[j], s0, s1, s2, s3, B[j * 8], B[4 * ldPf + j * 8]);
+                        else
+                            dmma16x8x8(acc[j], d0, d1, d2, d3, B[j * 8], B[4 * ldPf + j * 8]);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int k0 = 0; k0 < kQ; k0 += 8) {
+                    const double a0 = F[k0 * IC], a1 = F[k0 * IC + 8];
+                    const double a2 = F[(k0 + 4) * IC], a3 = F[(k0 + 4) * IC + 8];
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        if (j < NTf)
+                            dmma16x8x8(acc[j], a0, a1, a2, a3, B[k0 * ldPf + j * 8], B[(k0 + 4) * ldPf + j * 8]);
+                }
             }
-            if (f.momentsOld != nullptr)
-                v = 0.5 * (v + f.momentsOld[cell * n + k]);
-            f.moments[cell * n + k] = v;
         }
     }
+    flux_update<PAIR>(f, acc, i0, j0, mt, g, t4);
 }
 
 __global__ void ghost_periodic_kernel(double *m, int n, int NX, int NY)
@@ -508,27 +588,75 @@ int plan_flux(FluxArgs &f)
 
 cudaError_t prepare_flux(const FluxArgs &f)
 {
-    if (f.paired)
-        return cudaFuncSetAttribute(flux_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, f.smemBytes);
-    return cudaFuncSetAttribute(flux_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, f.smemBytes);
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = f.paired ? cudaFuncSetAttribute(flux_kernel<1, 0>, attr, f.smemBytes)
+                             : cudaFuncSetAttribute(flux_kernel<0, 0>, attr, f.smemBytes);
+    if (e != cudaSuccess)
+        return e;
+    return f.paired ? cudaFuncSetAttribute(flux_kernel<1, 1>, attr, f.smemBytes)
+                    : cudaFuncSetAttribute(flux_kernel<0, 1>, attr, f.smemBytes);
 }
 
-cudaError_t launch_flux_tiles(const FluxArgs &f, int first, int count, cudaStream_t stream)
+// Shares of the direction loop for `tiles` tiles on `sms` SMs (one CTA each):
+// 1, or the number that takes the fewest chunk times, a CTA's start (staging
+// of alpha) counted as one chunk and the pass over F as half a chunk per wave
+// of tiles.
+static int flux_shares(int tiles, int chunks, int sms)
+{
+    auto waves = [&](int s) { return (tiles * s + sms - 1) / sms; };
+    int best = 1;
+    double cost = waves(1) * (chunks + 1.0);
+    for (int s = 2; s <= chunks && s <= 64; s++) {
+        const double c = waves(s) * ((chunks + s - 1) / s + 1.0) + 1.5 + 0.5 * tiles / sms;
+        if (c < 0.95 * cost) {
+            cost = c;
+            best = s;
+        }
+    }
+    return best;
+}
+
+size_t flux_split_doubles(const FluxArgs &f)
+{
+    // Splitting pays while the tiles fill less than about two waves (the
+    // chunk times saved are then a sizeable share), and F has to stay small.
+    const size_t tiles = (size_t)f.tilesX * f.tilesY;
+    const size_t dirs = (size_t)(f.paired ? 2 : 1) * f.nqp;   // whole chunks of either layout
+    const size_t doubles = tiles * dirs * IC;
+    return (tiles <= 2 * (size_t)f.sms && doubles * sizeof(double) <= kSplitBytes) ? doubles : 0;
+}
+
+cudaError_t launch_flux_tiles(const FluxArgs &f, int first, int count, cudaStream_t stream, int *kernels)
 {
     if (first < 0 || count <= 0 || first + count > f.tilesX * f.tilesY)
         return cudaErrorInvalidValue;
     FluxArgs g = f;
     g.tileBase = first;
+    const int shares = (f.F && f.tileRun) ? flux_shares(count, f.nqp / (f.paired ? kQ / 2 : kQ), f.sms) : 1;
+    if (shares > 1) {
+        const dim3 grid((unsigned)count, (unsigned)shares);
+        const int pgrid = count * (IC / 16 / kProjWarps);
+        if (g.paired) {
+            flux_kernel<1, 1><<<grid, kFluxThreads, g.smemBytes, stream>>>(g);
+            flux_project_kernel<1><<<pgrid, kProjWarps * 32, 0, stream>>>(g);
+        } else {
+            flux_kernel<0, 1><<<grid, kFluxThreads, g.smemBytes, stream>>>(g);
+            flux_project_kernel<0><<<pgrid, kProjWarps * 32, 0, stream>>>(g);
+        }
+        *kernels += 2;
+        return cudaGetLastError();
+    }
     if (g.paired)
-        flux_kernel<1><<<count, kFluxThreads, g.smemBytes, stream>>>(g);
+        flux_kernel<1, 0><<<count, kFluxThreads, g.smemBytes, stream>>>(g);
     else
-        flux_kernel<0><<<count, kFluxThreads, g.smemBytes, stream>>>(g);
+        flux_kernel<0, 0><<<count, kFluxThreads, g.smemBytes, stream>>>(g);
+    *kernels += 1;
     return cudaGetLastError();
 }
 
-cudaError_t launch_flux(const FluxArgs &f, cudaStream_t stream)
+cudaError_t launch_flux(const FluxArgs &f, cudaStream_t stream, int *kernels)
 {
-    return launch_flux_tiles(f, 0, f.tilesX * f.tilesY, stream);
+    return launch_flux_tiles(f, 0, f.tilesX * f.tilesY, stream, kernels);
 }
 
 int flux_tile_rows(const FluxArgs &) { return TX; }
