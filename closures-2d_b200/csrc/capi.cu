@@ -789,8 +789,7 @@ int cl_create(const cl_grid *grid, const cl_options *opts, const cl_angular *ang
 
     NewtonArgs &a = ctx->nargs;
     memset(&a, 0, sizeof(a));
-    a.nprob = 1;
-    a.prob[0] = make_problem(ctx->B);
+    a.prob = make_problem(ctx->B);
     fill_newton_options(a, *opts, gauntNewton);
     a.stats = ctx->dStats;
     a.err = ctx->dErr;
@@ -813,8 +812,8 @@ int cl_create(const cl_grid *grid, const cl_options *opts, const cl_angular *ang
             ctx->err = "device allocation failed";
             return ctx_fail(ctx, CL_ERR_CUDA);
         }
-        a.prob[0].P2M = ctx->dP2M;
-        a.prob[0].alphaP = ctx->dAlphaP;
+        a.prob.P2M = ctx->dP2M;
+        a.prob.alphaP = ctx->dAlphaP;
     }
     int pl = plan_newton(a);
     if (ctx->B.paired && (pl != 0 || a.ntf == 0 || a.ntExact == 0)) {
@@ -826,10 +825,10 @@ int cl_create(const cl_grid *grid, const cl_options *opts, const cl_angular *ang
             ctx->err = std::string("basis upload: ") + cudaGetErrorString(ce);
             return ctx_fail(ctx, CL_ERR_CUDA);
         }
-        NewtonProblem keep = a.prob[0];
-        a.prob[0] = make_problem(ctx->B);
-        a.prob[0].P2M = keep.P2M;
-        a.prob[0].alphaP = keep.alphaP;
+        NewtonProblem keep = a.prob;
+        a.prob = make_problem(ctx->B);
+        a.prob.P2M = keep.P2M;
+        a.prob.alphaP = keep.alphaP;
         pl = plan_newton(a);
     }
     if (pl != 0) {
@@ -988,11 +987,11 @@ static void update_screen(cl_ctx *ctx)
     ctx->tuning.screen_ctas = 0;
     const DeviceBasis &B = ctx->newtonB2 ? ctx->B2 : ctx->B;
     const NewtonArgs &k = ctx->nargs;
-    if (!ctx->rangeTest || !ctx->dPend || !B.paired || !B.screenOk || k.nprob != 1 || k.momentType != 0 ||
-        k.mixed || k.optType != 0 || !(k.prob[0].gramLo > 0.0))
+    if (!ctx->rangeTest || !ctx->dPend || !B.paired || !B.screenOk || k.momentType != 0 ||
+        k.mixed || k.optType != 0 || !(k.prob.gramLo > 0.0))
         return;
     NewtonArgs s = k;
-    s.prob[0] = make_screen_problem(B);
+    s.prob = make_screen_problem(B);
     if (plan_screen(s) != 0 || prepare_screen(s) != cudaSuccess)
         return;
     ctx->sargs = s;
@@ -1024,12 +1023,12 @@ constexpr int kOrderWholeMax = 131072;
 static cudaError_t launch_stage_newton(cl_ctx *ctx, NewtonArgs &a, int slot, cudaStream_t st, int *nk)
 {
     cudaError_t e;
-    const NewtonProblem kp = a.prob[0];
+    const NewtonProblem kp = a.prob;
     if (kp.iters && ctx->dPend && (ctx->screen || kp.count <= kOrderWholeMax)) {
         int gateMin = 0;
         if (ctx->screen) {
             NewtonArgs s = ctx->sargs;
-            NewtonProblem &sp = s.prob[0];
+            NewtonProblem &sp = s.prob;
             sp.count = kp.count;
             sp.first = kp.first;
             sp.u = kp.u;
@@ -1061,8 +1060,8 @@ static cudaError_t launch_stage_newton(cl_ctx *ctx, NewtonArgs &a, int slot, cud
                                     kp.iters, ctx->dPend2 + kp.first, ctx->dOrderCount + slot, st)) != cudaSuccess)
             return e;
         *nk += 1;
-        a.prob[0].cellList = ctx->dPend2 + kp.first;
-        a.prob[0].countDev = ctx->dOrderCount + slot;
+        a.prob.cellList = ctx->dPend2 + kp.first;
+        a.prob.countDev = ctx->dOrderCount + slot;
     }
     if ((e = launch_newton(a, ctx->nCtas, st)) != cudaSuccess)
         return e;
@@ -1089,12 +1088,12 @@ static cudaError_t enqueue_stage(cl_ctx *ctx, int stage, double dt, double dx, d
         *nk += k;
     }
     NewtonArgs a = ctx->nargs;
-    a.prob[0].count = (int)ctx->C;
-    a.prob[0].u = ctx->dMom;
-    a.prob[0].alpha = ctx->dAlpha;
-    a.prob[0].queue = ctx->dQueue + stage;
-    a.prob[0].iters = ctx->dIters;
-    a.prob[0].alphaStart = ctx->warm ? ctx->dAlphaPred : nullptr;
+    a.prob.count = (int)ctx->C;
+    a.prob.u = ctx->dMom;
+    a.prob.alpha = ctx->dAlpha;
+    a.prob.queue = ctx->dQueue + stage;
+    a.prob.iters = ctx->dIters;
+    a.prob.alphaStart = ctx->warm ? ctx->dAlphaPred : nullptr;
     a.momentsOld = (stage == 0) ? ctx->dOld : nullptr;
     if (beforeK1 && (e = cudaEventRecord(beforeK1, ctx->stream)) != cudaSuccess)
         return e;
@@ -1205,12 +1204,12 @@ int cl_step_timed(cl_ctx *ctx, double dt, double dx, double dy, float *ms)
             nk += k < 0 ? 0 : k;
         }
         NewtonArgs a = ctx->nargs;
-        a.prob[0].count = (int)ctx->C;
-        a.prob[0].u = ctx->dMom;
-        a.prob[0].alpha = ctx->dAlpha;
-        a.prob[0].queue = ctx->dQueue + stage;
-        a.prob[0].iters = ctx->dIters;
-        a.prob[0].alphaStart = ctx->warm ? ctx->dAlphaPred : nullptr;
+        a.prob.count = (int)ctx->C;
+        a.prob.u = ctx->dMom;
+        a.prob.alpha = ctx->dAlpha;
+        a.prob.queue = ctx->dQueue + stage;
+        a.prob.iters = ctx->dIters;
+        a.prob.alphaStart = ctx->warm ? ctx->dAlphaPred : nullptr;
         a.momentsOld = (stage == 0) ? ctx->dOld : nullptr;
         if (e == cudaSuccess)
             e = launch_stage_newton(ctx, a, stage, ctx->stream, &nk);
@@ -1420,18 +1419,18 @@ int cl_step_host(cl_ctx *ctx, double dt, double dx, double dy, double *moments, 
             nk += k < 0 ? 0 : k;
         }
         NewtonArgs a = ctx->nargs;
-        a.prob[0].u = ctx->dMom;
-        a.prob[0].alpha = ctx->dAlpha;
-        a.prob[0].iters = ctx->dIters;
-        a.prob[0].alphaStart = ctx->warm ? ctx->dAlphaPred : nullptr;
+        a.prob.u = ctx->dMom;
+        a.prob.alpha = ctx->dAlpha;
+        a.prob.iters = ctx->dIters;
+        a.prob.alphaStart = ctx->warm ? ctx->dAlphaPred : nullptr;
         a.momentsOld = (stage == 0) ? ctx->dOld : nullptr;
         const int parts = (stage == 0) ? bands : 1;
         for (int b = 0; b < parts; b++) {
             if (stage == 0 && bands > 1)
                 run(cudaStreamWaitEvent(S, ctx->evBand[b], 0));
-            a.prob[0].first = (stage == 0) ? (int)band0[b] : 0;
-            a.prob[0].count = (stage == 0) ? (int)(band0[b + 1] - band0[b]) : (int)C;
-            a.prob[0].queue = ctx->dQueue + ((stage == 0 && bands > 1) ? 4 + b : stage);
+            a.prob.first = (stage == 0) ? (int)band0[b] : 0;
+            a.prob.count = (stage == 0) ? (int)(band0[b + 1] - band0[b]) : (int)C;
+            a.prob.queue = ctx->dQueue + ((stage == 0 && bands > 1) ? 4 + b : stage);
             if (e == cudaSuccess) {
                 NewtonArgs ab = a;   // the band's own list and counters
                 run(launch_stage_newton(ctx, ab, (stage == 0 && bands > 1) ? 4 + b : stage, S, &nk));
@@ -1532,12 +1531,12 @@ static int ensure_alt_basis(cl_ctx *ctx)
 static bool newton_shape(const cl_ctx *ctx, const DeviceBasis &B, int nw, NewtonArgs &a)
 {
     a = ctx->nargs;
-    NewtonProblem keep = a.prob[0];
-    a.prob[0] = make_problem(B);
-    a.prob[0].P2M = keep.P2M;
-    a.prob[0].alphaP = keep.alphaP;
+    NewtonProblem keep = a.prob;
+    a.prob = make_problem(B);
+    a.prob.P2M = keep.P2M;
+    a.prob.alphaP = keep.alphaP;
     if (!ctx->rangeTest)
-        a.prob[0].gramLo = 0.0;
+        a.prob.gramLo = 0.0;
     a.nw = nw;
     if (plan_newton(a) != 0 || a.ntf == 0 || (B.paired && a.ntExact == 0))
         return false;
@@ -1592,27 +1591,27 @@ struct TuneScratch {
 static float time_newton(cl_ctx *ctx, NewtonArgs a, const DeviceBasis &B, TuneScratch &S)
 {
     const size_t C = (size_t)ctx->C, n = (size_t)ctx->n;
-    a.prob[0].count = (int)C;
-    a.prob[0].u = S.u;
-    a.prob[0].alpha = S.a;
-    a.prob[0].iters = S.it;
-    a.prob[0].regs = nullptr;
-    a.prob[0].status = nullptr;
-    a.prob[0].alphaStart = nullptr;
-    a.prob[0].queue = S.q;
-    a.prob[0].first = 0;
+    a.prob.count = (int)C;
+    a.prob.u = S.u;
+    a.prob.alpha = S.a;
+    a.prob.iters = S.it;
+    a.prob.regs = nullptr;
+    a.prob.status = nullptr;
+    a.prob.alphaStart = nullptr;
+    a.prob.queue = S.q;
+    a.prob.first = 0;
     a.momentsOld = nullptr;
     a.stats = S.st;
     a.err = S.err;
     const int grid = sm_count() * newton_ctas_per_sm(a);
     NewtonArgs sa;
     int sgrid = 0;
-    if (ctx->rangeTest && ctx->dPend && B.paired && B.screenOk && a.nprob == 1 && a.momentType == 0 &&
-        !a.mixed && a.optType == 0 && a.prob[0].gramLo > 0.0) {
+    if (ctx->rangeTest && ctx->dPend && B.paired && B.screenOk && a.momentType == 0 &&
+        !a.mixed && a.optType == 0 && a.prob.gramLo > 0.0) {
         sa = a;
-        sa.prob[0] = make_screen_problem(B);
+        sa.prob = make_screen_problem(B);
         if (plan_screen(sa) == 0 && prepare_screen(sa) == cudaSuccess) {
-            NewtonProblem &sp = sa.prob[0];
+            NewtonProblem &sp = sa.prob;
             sp.count = (int)C;
             sp.u = S.u;
             sp.alpha = S.a;
@@ -1623,8 +1622,8 @@ static float time_newton(cl_ctx *ctx, NewtonArgs a, const DeviceBasis &B, TuneSc
             sp.gateCount = (const int *)(S.q + 3);
             sp.gateMin = (int)std::ceil(kScreenGate * (double)C);
             sgrid = sm_count() * screen_ctas_per_sm(sa);
-            a.prob[0].cellList = ctx->dPend2;
-            a.prob[0].countDev = (const int *)(S.q + 4);
+            a.prob.cellList = ctx->dPend2;
+            a.prob.countDev = (const int *)(S.q + 4);
         }
     }
     float ms[3] = {0, 0, 0};
@@ -1641,7 +1640,7 @@ static float time_newton(cl_ctx *ctx, NewtonArgs a, const DeviceBasis &B, TuneSc
             if (launch_screen_gate(S.it, 0, (int)C, (int *)(S.q + 3), st) != cudaSuccess ||
                 launch_screen(sa, sgrid, st) != cudaSuccess ||
                 launch_order_cells(ctx->dPend, (const int *)(S.q + 2), 0, (int)C, (const int *)(S.q + 3),
-                                   sa.prob[0].gateMin, kOrderWholeMax, S.it, ctx->dPend2, (int *)(S.q + 4),
+                                   sa.prob.gateMin, kOrderWholeMax, S.it, ctx->dPend2, (int *)(S.q + 4),
                                    st) != cudaSuccess)
                 return -1.0f;
             g_launches += 3;
@@ -1804,7 +1803,7 @@ int cl_set_range_test(cl_ctx *ctx, int enable)
         return CL_ERR_ARG;
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     ctx->rangeTest = enable ? 1 : 0;
-    ctx->nargs.prob[0].gramLo = enable ? make_problem(ctx->newtonB2 ? ctx->B2 : ctx->B).gramLo : 0.0;
+    ctx->nargs.prob.gramLo = enable ? make_problem(ctx->newtonB2 ? ctx->B2 : ctx->B).gramLo : 0.0;
     update_screen(ctx);
     invalidate_graph(ctx);
     return CL_OK;
@@ -2024,14 +2023,14 @@ int cl_solve_batch_device_start(cl_ctx *ctx, int count, double *d_u, double *d_a
     if (count == 0)
         return CL_OK;
     NewtonArgs a = ctx->nargs;
-    a.prob[0].count = count;
-    a.prob[0].u = d_u;
-    a.prob[0].alpha = d_alpha;
-    a.prob[0].iters = d_iters;
-    a.prob[0].regs = d_reg;
-    a.prob[0].status = d_status;
-    a.prob[0].alphaStart = d_alpha_start;
-    a.prob[0].queue = ctx->dQueue + 2;
+    a.prob.count = count;
+    a.prob.u = d_u;
+    a.prob.alpha = d_alpha;
+    a.prob.iters = d_iters;
+    a.prob.regs = d_reg;
+    a.prob.status = d_status;
+    a.prob.alphaStart = d_alpha_start;
+    a.prob.queue = ctx->dQueue + 2;
     a.momentsOld = nullptr;
     CUDA_TRY(ctx, cudaMemsetAsync(ctx->dQueue + 2, 0, sizeof(unsigned), ctx->stream));
     CUDA_TRY(ctx, launch_newton(a, ctx->nCtas, ctx->stream));
@@ -2051,16 +2050,16 @@ int cl_solve_batch_cb_device(cl_ctx *ctx, int count, double *d_u, double *d_P2M,
     if (count == 0)
         return CL_OK;
     NewtonArgs a = ctx->nargs;
-    a.prob[0].count = count;
-    a.prob[0].u = d_u;
-    a.prob[0].alpha = d_alpha;
-    a.prob[0].P2M = d_P2M;
-    a.prob[0].alphaP = d_alphaP;
-    a.prob[0].iters = d_iters;
-    a.prob[0].regs = d_reg;
-    a.prob[0].status = d_status;
-    a.prob[0].alphaStart = nullptr;
-    a.prob[0].queue = ctx->dQueue + 2;
+    a.prob.count = count;
+    a.prob.u = d_u;
+    a.prob.alpha = d_alpha;
+    a.prob.P2M = d_P2M;
+    a.prob.alphaP = d_alphaP;
+    a.prob.iters = d_iters;
+    a.prob.regs = d_reg;
+    a.prob.status = d_status;
+    a.prob.alphaStart = nullptr;
+    a.prob.queue = ctx->dQueue + 2;
     a.momentsOld = nullptr;
     CUDA_TRY(ctx, cudaMemsetAsync(ctx->dQueue + 2, 0, sizeof(unsigned), ctx->stream));
     CUDA_TRY(ctx, launch_newton(a, ctx->nCtas, ctx->stream));
@@ -2114,16 +2113,25 @@ int cl_solve_batch(cl_ctx *ctx, int count, double *u, double *alpha, int *iters,
 // ---------------------------------------------------------------- multi-order
 }  // extern "C"
 
+// Several moment orders: one launch of each order's own instance, on up to
+// kMultiStreams streams forked from the solver's, so that the CTAs of one order
+// take the SMs that the last long chains of another leave.  (One launch over
+// all orders ran the fused instance with runtime tile counts, one direction at
+// a time, and its shared-memory plan was that of the largest order.)
+constexpr int kMaxOrders = 8;
+constexpr int kMultiStreams = 4;
+
 struct cl_multi {
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr, side[kMultiStreams - 1] = {};
+    cudaEvent_t evFork = nullptr, evJoin[kMultiStreams - 1] = {};
     cl_options opt;
     int nprob = 0;
-    DeviceBasis B[kMaxProblems];
-    NewtonArgs nargs;
+    DeviceBasis B[kMaxOrders];
+    NewtonArgs nargs[kMaxOrders];
+    int nCtas[kMaxOrders] = {};
     unsigned int *dQueue = nullptr;
     DevStats *dStats = nullptr;
     int *dErr = nullptr;
-    int nCtas = 0;
     std::string err;
 };
 
@@ -2142,6 +2150,14 @@ void cl_multi_destroy(cl_multi *m)
     cudaFree(m->dQueue);
     cudaFree(m->dStats);
     cudaFree(m->dErr);
+    if (m->evFork)
+        cudaEventDestroy(m->evFork);
+    for (int k = 0; k < kMultiStreams - 1; k++) {
+        if (m->evJoin[k])
+            cudaEventDestroy(m->evJoin[k]);
+        if (m->side[k])
+            cudaStreamDestroy(m->side[k]);
+    }
     if (m->stream)
         cudaStreamDestroy(m->stream);
     delete m;
@@ -2150,7 +2166,7 @@ void cl_multi_destroy(cl_multi *m)
 int cl_multi_create(int norders, const int *orders, int quad_order, int use_gaunt, const cl_options *opts,
                     cl_multi **out)
 {
-    if (!out || !orders || norders < 1 || norders > kMaxProblems) {
+    if (!out || !orders || norders < 1 || norders > kMaxOrders) {
         g_global_err = "bad order list";
         return CL_ERR_ARG;
     }
@@ -2165,6 +2181,7 @@ int cl_multi_create(int norders, const int *orders, int quad_order, int use_gaun
         g_global_err = "the change-of-basis solve runs one moment order per context (cl_create)";
         return CL_ERR_ARG;
     }
+    const char *const mixedText = "mixed precision needs a single moment order per launch";
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) {
         g_global_err = "no CUDA device (the B200 path has no CPU fallback)";
@@ -2173,55 +2190,60 @@ int cl_multi_create(int norders, const int *orders, int quad_order, int use_gaun
     cl_multi *m = new cl_multi();
     m->opt = *opts;
     m->nprob = norders;
-    if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess) {
-        g_global_err = "stream creation failed";
+    auto fail = [&](int code, const std::string &text) {
+        g_global_err = text;
         cl_multi_destroy(m);
-        return CL_ERR_CUDA;
-    }
-    NewtonArgs &a = m->nargs;
-    memset(&a, 0, sizeof(a));
-    a.nprob = norders;
-    for (int p = 0; p < norders; p++) {
-        Angular A;
-        if (orders[p] > 6 || build_angular(orders[p], quad_order, use_gaunt, A) != 0) {
-            g_global_err = "unsupported order (1..6)";
-            cl_multi_destroy(m);
-            return CL_ERR_ARG;
-        }
-        cudaError_t ce = build_device_basis(m->B[p], A.n, A.n2, A.nq, A.useGaunt, A.w.data(), A.xi.data(),
-                                            A.eta.data(), A.p.data(), A.goff.data(), A.gidx.data(),
-                                            A.gval.data(), (int)A.gidx.size());
-        if (ce != cudaSuccess) {
-            g_global_err = std::string("basis upload: ") + cudaGetErrorString(ce);
-            cl_multi_destroy(m);
-            return CL_ERR_CUDA;
-        }
-        a.prob[p] = make_problem(m->B[p]);
-    }
-    fill_newton_options(a, *opts, use_gaunt ? 1 : 0);
-    if (cudaMalloc(&m->dQueue, kMaxProblems * sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc(&m->dStats, sizeof(DevStats)) != cudaSuccess || cudaMalloc(&m->dErr, 2 * sizeof(int)) != cudaSuccess) {
-        g_global_err = "device allocation failed";
-        cl_multi_destroy(m);
-        return CL_ERR_CUDA;
-    }
+        return code;
+    };
+    bool streams = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) == cudaSuccess &&
+                   cudaEventCreateWithFlags(&m->evFork, cudaEventDisableTiming) == cudaSuccess;
+    for (int k = 0; k < kMultiStreams - 1 && streams; k++)
+        streams = cudaStreamCreateWithFlags(&m->side[k], cudaStreamNonBlocking) == cudaSuccess &&
+                  cudaEventCreateWithFlags(&m->evJoin[k], cudaEventDisableTiming) == cudaSuccess;
+    if (!streams)
+        return fail(CL_ERR_CUDA, "stream creation failed");
+    if (cudaMalloc(&m->dQueue, kMaxOrders * sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&m->dStats, sizeof(DevStats)) != cudaSuccess || cudaMalloc(&m->dErr, 2 * sizeof(int)) != cudaSuccess)
+        return fail(CL_ERR_CUDA, "device allocation failed");
     cudaMemset(m->dStats, 0, sizeof(DevStats));
     cudaMemset(m->dErr, 0, 2 * sizeof(int));
-    a.stats = m->dStats;
-    a.err = m->dErr;
-    const int pl = plan_newton(a);
-    if (pl != 0) {
-        g_global_err = pl == -2 ? "mixed precision needs a single moment order per launch"
-                                : "Newton kernel layout does not fit in shared memory";
-        cl_multi_destroy(m);
-        return CL_ERR_ARG;
+    for (int p = 0; p < norders; p++) {
+        Angular A;
+        if (orders[p] > 6 || build_angular(orders[p], quad_order, use_gaunt, A) != 0)
+            return fail(CL_ERR_ARG, "unsupported order (1..6)");
+        if (opts->precision == CL_MIXED && norders > 1)
+            return fail(CL_ERR_ARG, mixedText);
+        NewtonArgs &a = m->nargs[p];
+        // direction pairs where a fused instance takes them, else one
+        // direction at a time, as in cl_create
+        int paired = 0, pl = -1;
+        if (opts->moment_type == CL_MN && opts->precision == CL_FP64 && opts->contraction == CL_CONTRACT_PAIRS) {
+            int pnt = 0, pnbk = 0;
+            paired_counts(A.n, A.n2, A.useGaunt, pnt, pnbk);
+            paired = newton_pair_supported(pnt, pnbk, A.n) ? 1 : 0;
+        }
+        for (;; paired = 0) {
+            m->B[p].release();
+            cudaError_t ce = build_device_basis(m->B[p], A.n, A.n2, A.nq, A.useGaunt, A.w.data(), A.xi.data(),
+                                                A.eta.data(), A.p.data(), A.goff.data(), A.gidx.data(),
+                                                A.gval.data(), (int)A.gidx.size(), paired);
+            if (ce != cudaSuccess)
+                return fail(CL_ERR_CUDA, std::string("basis upload: ") + cudaGetErrorString(ce));
+            memset(&a, 0, sizeof(a));
+            a.prob = make_problem(m->B[p]);
+            fill_newton_options(a, *opts, use_gaunt ? 1 : 0);
+            a.stats = m->dStats;
+            a.err = m->dErr;
+            pl = plan_newton(a);
+            if (!m->B[p].paired || (pl == 0 && a.ntf > 0))
+                break;
+        }
+        if (pl != 0)
+            return fail(CL_ERR_ARG, pl == -2 ? mixedText : "Newton kernel layout does not fit in shared memory");
+        if (prepare_newton(a) != cudaSuccess)
+            return fail(CL_ERR_CUDA, "Newton kernel attributes");
+        m->nCtas[p] = sm_count() * newton_ctas_per_sm(a);
     }
-    if (prepare_newton(a) != cudaSuccess) {
-        g_global_err = "Newton kernel attributes";
-        cl_multi_destroy(m);
-        return CL_ERR_CUDA;
-    }
-    m->nCtas = sm_count() * newton_ctas_per_sm(a);
     cudaDeviceSynchronize();
     *out = m;
     return CL_OK;
@@ -2239,23 +2261,54 @@ int cl_multi_solve_device_start(cl_multi *m, const int *counts, double *const *d
 {
     if (!m || !counts || !d_u || !d_alpha)
         return CL_ERR_ARG;
-    NewtonArgs a = m->nargs;
+    // the longest launches first: directions times columns times vectors
+    int order[kMaxOrders];
+    double work[kMaxOrders];
     for (int p = 0; p < m->nprob; p++) {
-        a.prob[p].count = counts[p];
-        a.prob[p].u = d_u[p];
-        a.prob[p].alpha = d_alpha[p];
-        a.prob[p].iters = d_iters ? d_iters[p] : nullptr;
-        a.prob[p].regs = d_reg ? d_reg[p] : nullptr;
-        a.prob[p].status = d_status ? d_status[p] : nullptr;
-        a.prob[p].alphaStart = d_alpha_start ? d_alpha_start[p] : nullptr;
-        a.prob[p].queue = m->dQueue + p;
+        order[p] = p;
+        work[p] = (double)counts[p] * m->nargs[p].prob.nqp * m->nargs[p].prob.ldP;
     }
-    cudaError_t e = cudaMemsetAsync(m->dQueue, 0, kMaxProblems * sizeof(unsigned), m->stream);
-    if (e == cudaSuccess)
-        e = launch_newton(a, m->nCtas, m->stream);
-    if (e == cudaSuccess)
-        e = cudaStreamSynchronize(m->stream);
-    g_launches += 1;
+    std::stable_sort(order, order + m->nprob, [&](int x, int y) { return work[x] > work[y]; });
+    cudaError_t e = cudaMemsetAsync(m->dQueue, 0, kMaxOrders * sizeof(unsigned), m->stream);
+    auto run = [&](cudaError_t r) {
+        if (e == cudaSuccess)
+            e = r;
+    };
+    run(cudaEventRecord(m->evFork, m->stream));
+    bool used[kMultiStreams] = {true};
+    int launched = 0;
+    for (int i = 0; i < m->nprob && e == cudaSuccess; i++) {
+        const int p = order[i];
+        if (counts[p] <= 0)
+            continue;
+        NewtonArgs a = m->nargs[p];
+        a.prob.count = counts[p];
+        a.prob.u = d_u[p];
+        a.prob.alpha = d_alpha[p];
+        a.prob.iters = d_iters ? d_iters[p] : nullptr;
+        a.prob.regs = d_reg ? d_reg[p] : nullptr;
+        a.prob.status = d_status ? d_status[p] : nullptr;
+        a.prob.alphaStart = d_alpha_start ? d_alpha_start[p] : nullptr;
+        a.prob.queue = m->dQueue + p;
+        const int k = launched % kMultiStreams;
+        cudaStream_t st = k == 0 ? m->stream : m->side[k - 1];
+        if (!used[k]) {
+            run(cudaStreamWaitEvent(st, m->evFork, 0));
+            used[k] = true;
+        }
+        // no more CTAs than vectors: the others' SMs go to the next launch
+        if (e == cudaSuccess)
+            run(launch_newton(a, std::min(m->nCtas[p], counts[p]), st));
+        launched++;
+    }
+    for (int k = 1; k < kMultiStreams; k++)
+        if (used[k]) {
+            run(cudaEventRecord(m->evJoin[k - 1], m->side[k - 1]));
+            run(cudaStreamWaitEvent(m->stream, m->evJoin[k - 1], 0));
+        }
+    const cudaError_t es = cudaStreamSynchronize(m->stream);
+    run(es);
+    g_launches += launched;
     if (e != cudaSuccess) {
         m->err = std::string("multi solve: ") + cudaGetErrorString(e);
         return CL_ERR_CUDA;

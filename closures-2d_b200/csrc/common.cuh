@@ -8,7 +8,6 @@ namespace clb {
 constexpr int kThreads = 256;        // 8 warps per CTA
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxN = 32;            // moments per cell handled by one warp (order <= 6)
-constexpr int kMaxProblems = 8;      // moment orders sharing one persistent launch
 constexpr int kNumReg = 5;
 // change-of-basis working state of one Newton slot in global memory: the
 // basis T and the rows of L^-1 ([kMaxN][kMaxN] each), then alphaP, the

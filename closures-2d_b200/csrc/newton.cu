@@ -11,24 +11,17 @@ namespace clb {
 
 int plan_newton(NewtonArgs &a)
 {
-    int nbMax = 8, ldPMax = 0, K2tot = 0, nMax = 1, ellGroups = 0, ellChunks = 0;
-    for (int p = 0; p < a.nprob; p++) {
-        const NewtonProblem &pb = a.prob[p];
-        ellGroups = pb.ellGroups > ellGroups ? pb.ellGroups : ellGroups;
-        ellChunks = pb.ellChunks > ellChunks ? pb.ellChunks : ellChunks;
-        nbMax = pb.nb > nbMax ? pb.nb : nbMax;
-        ldPMax = pb.ldP > ldPMax ? pb.ldP : ldPMax;
-        int kt = pb.K2p + (a.momentType == 1 ? pb.nb : 0);
-        K2tot = kt > K2tot ? kt : K2tot;
-        nMax = pb.n > nMax ? pb.n : nMax;
-    }
+    const NewtonProblem &pb = a.prob;
+    const int nbMax = pb.nb > 8 ? pb.nb : 8, ldPMax = pb.ldP, nMax = pb.n;
+    const int K2tot = pb.K2p + (a.momentType == 1 ? pb.nb : 0);
+    int ellGroups = pb.ellGroups, ellChunks = pb.ellChunks;
     if (a.nw == 0)
         a.nw = kWarps;
     if (a.nw != kWarps && a.nw != 4)
         return -1;
     const int nw = a.nw;
     a.T = 4 * nw;
-    // fused contractions when every problem's G fits in 16 column tiles; in
+    // fused contractions when the problem's G fits in 16 column tiles; in
     // FP64 one warp per 8 slots x 8 quadrature rows of a 32-row chunk, mixed
     // one per 16 slots x 8 rows
     const int nt2 = K2tot / 8;
@@ -70,13 +63,13 @@ int plan_newton(NewtonArgs &a)
     const int unionBase = off;
     const int ntiles2 = (T / 16) * (K2tot / 8);
     a.tpw = (ntiles2 + nw - 1) / nw;
-    a.ntExact = (a.ntf > 0 && a.nprob == 1) ? nt2 : 0;
-    a.nbk = (a.ntf > 0 && a.nprob == 1) ? a.prob[0].nb / 8 : 0;
+    a.ntExact = a.ntf > 0 ? nt2 : 0;
+    a.nbk = a.ntf > 0 ? pb.nb / 8 : 0;
     if (a.mixed && a.ntExact == 0)
         return -2;
-    if (nw != kWarps && (a.ntExact == 0 || a.nprob != 1 || !a.prob[0].paired || a.mixed || a.optType != 0 ||
-                         !newton_pair4_supported(a.ntExact, a.nbk, a.prob[0].n)))
-        return -1;   // the 16-slot shape: single-order direction-pair Newton only
+    if (nw != kWarps && (a.ntExact == 0 || !pb.paired || a.mixed || a.optType != 0 ||
+                         !newton_pair4_supported(a.ntExact, a.nbk, a.prob.n)))
+        return -1;   // the 16-slot shape: direction-pair Newton only
     // phase-B region
     int offG = unionBase;
     a.strideH = nMax * a.ldh;   // ldh is even
@@ -131,10 +124,9 @@ int plan_newton(NewtonArgs &a)
     return -1;
 }
 
-// Instance selection: a single-problem launch on the fused path runs the
-// kernel specialised to its exact column-tile and k-step counts; mixed
-// orders run the fused instance with runtime counts; the rest the general
-// contractions.  mode: 0 launch, 1 shared-memory attribute, 2 occupancy.
+// Instance selection: the kernel specialised to the problem's exact column-tile
+// and k-step counts where there is one, else the fused instance with runtime
+// counts or the general contractions.  mode: 0 launch, 1 shared-memory attribute, 2 occupancy.
 static cudaError_t run(const NewtonArgs &a, int grid, cudaStream_t stream, int mode, int *occ)
 {
     cudaError_t e = cudaErrorInvalidValue;
@@ -143,7 +135,7 @@ static cudaError_t run(const NewtonArgs &a, int grid, cudaStream_t stream, int m
             return e;
         return cudaErrorInvalidValue;
     }
-    if (a.nprob == 1 && a.prob[0].paired) {
+    if (a.prob.paired) {
         // the direction-pair layout runs only its own fused instances
         if (a.nw == 4)
             return (a.ntf > 0 && a.ntExact > 0 && newton_run_exact_pair4(a, grid, stream, mode, occ, &e))

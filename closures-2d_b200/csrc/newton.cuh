@@ -6,7 +6,7 @@
 
 namespace clb {
 
-// One moment order ("problem") of a launch.  Basis rows are padded to
+// The moment order ("problem") of a launch.  Basis rows are padded to
 // nqp = multiple of the q-chunk, columns laid out as
 //   [0, nb)              basis p_k, k < n (zero for n <= k < nb)
 //   [nb, nb + K2p)       Hessian columns: extended basis (Gaunt) or the
@@ -109,8 +109,7 @@ enum { SC_T = 0, SC_FREF, SC_GD, SC_MAXF, SC_RTOL, SC_U0, SC_ASCALE, SC_DELTA, S
 enum { SI_CELL = 0, SI_STATE, SI_ITER, SI_TOTAL, SI_REG, SI_MAXITER, SI_PRED, SI_CB, SI_BFGS, SI_N };
 
 struct NewtonArgs {
-    NewtonProblem prob[kMaxProblems];
-    int nprob;
+    NewtonProblem prob;
     int momentType, maxIter, useGaunt;
     double tolRel, condHMax, deltaPPn, tolGamma;
     // grid mode: copy interior moments to momentsOld before solving them
@@ -128,7 +127,7 @@ struct NewtonArgs {
     int smemBytes;
     int tpw;                    // column tiles per warp (general contractions)
     int ntf;                    // > 0: fused contractions with this many tiles per warp
-    int ntExact, nbk;           // single problem on the fused path: its column tiles and
+    int ntExact, nbk;           // on the fused path: the problem's column tiles and
                                 // GEMM1 k-steps (selects a specialised instance), else 0
     int mixed;                  // Hessian-only tiles by split TF32 (CL_MIXED); needs ntExact
     int optType;                // 0 Newton (opt.cpp), 1 change of basis (optcb.cpp),
@@ -159,7 +158,7 @@ cudaError_t prepare_newton(const NewtonArgs &a);
 bool newton_pair_supported(int nt, int nbk, int n);
 // ... and in the 16-slot launch shape.
 bool newton_pair4_supported(int nt, int nbk, int n);
-// Screening pass (Mn, FP64, direction pairs; a.prob[0] the gradient-column
+// Screening pass (Mn, FP64, direction pairs; a.prob the gradient-column
 // layout of the problem): layout, instance check, shared-memory attribute,
 // launch and resident CTAs per SM.
 int plan_screen(NewtonArgs &a);

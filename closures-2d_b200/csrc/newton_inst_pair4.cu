@@ -24,8 +24,8 @@ bool newton_run_exact_pair4(const NewtonArgs &a, int grid, cudaStream_t s, int m
     if (a.momentType != 0 || a.mixed || a.nw != 4)
         return false;
 #define CLB_PAIR4(NT_, NBK_, N_, NTE_, NBE_)                                                     \
-    if (a.ntExact == NT_ && a.nbk == NBK_ && a.prob[0].n == N_ && a.prob[0].K2e == 8 * NTE_ &&   \
-        a.prob[0].nbe == 8 * NBE_) {                                                            \
+    if (a.ntExact == NT_ && a.nbk == NBK_ && a.prob.n == N_ && a.prob.K2e == 8 * NTE_ &&   \
+        a.prob.nbe == 8 * NBE_) {                                                            \
         *err = newton_run<1, NT_, 0, NT_, NBK_, 0, 16 * NTE_ + NBE_, 8, N_>(a, grid, s, mode, occ); \
         return true;                                                                           \
     }

@@ -7,8 +7,8 @@ namespace clb {
 bool newton_run_exact_pair_b(const NewtonArgs &a, int grid, cudaStream_t s, int mode, int *occ, cudaError_t *err)
 {
 #define CLB_PAIR(NT_, NBK_, N_, NTE_, NBE_)                                                     \
-    if (a.ntExact == NT_ && a.nbk == NBK_ && a.prob[0].n == N_ && a.prob[0].K2e == 8 * NTE_ &&   \
-        a.prob[0].nbe == 8 * NBE_) {                                                            \
+    if (a.ntExact == NT_ && a.nbk == NBK_ && a.prob.n == N_ && a.prob.K2e == 8 * NTE_ &&   \
+        a.prob.nbe == 8 * NBE_) {                                                            \
         *err = newton_run<1, NT_, 0, NT_, NBK_, 0, 16 * NTE_ + NBE_, 16, N_>(a, grid, s, mode, occ); \
         return true;                                                                           \
     }

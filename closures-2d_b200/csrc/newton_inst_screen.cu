@@ -10,8 +10,8 @@ bool screen_supported(int nt, int nbk) { return nt == nbk && nt >= 2 && nt <= 4;
 
 int plan_screen(NewtonArgs &a)
 {
-    const NewtonProblem &pb = a.prob[0];
-    if (a.nprob != 1 || !pb.paired || a.momentType != 0 || a.mixed || a.optType != 0)
+    const NewtonProblem &pb = a.prob;
+    if (!pb.paired || a.momentType != 0 || a.mixed || a.optType != 0)
         return -1;
     a.nw = a.warps = kWarps;
     a.T = 32;

@@ -1,7 +1,7 @@
 // newton_kernel.cuh -- persistent dual-Newton kernel for the Mn / PPn entropy
 // closure (device code; instantiated by the newton_inst_*.cu units).
 //
-// One launch solves, for every vector u of every problem, the dual problem of
+// One launch solves, for every vector u of a problem, the dual problem of
 // opt() (src/momopt/opt/opt.cpp:82-343): minimise <eta*(alpha.m)> - alpha.u by
 // Newton's method with the Armijo backtracking line search of
 // linesearch.cpp:21-99 and the isotropic-restart regularisation ladder
@@ -2250,8 +2250,7 @@ __global__ void __launch_bounds__(NW * 32, (NTF > 0 && !MIX && NW == 8) ? 2 : 1)
     constexpr int kThreads = NW * 32, kWarps = NW;
     constexpr int NM = NX ? NX : (NBK > 0 && 8 * NBK < kMaxN) ? 8 * NBK : kMaxN;   // n <= nb = 8 NBK
     extern __shared__ __align__(16) double sm[];
-    // [0] problem, [1] done, [2] exhausted, [3] next slot of phase B, [4] problems whose first share is taken
-    __shared__ int ctl[5];
+    __shared__ int ctl[3];   // [0] done, [1] work counter exhausted, [2] next slot of phase B
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t4 = lane & 3;
     const int T = a.T, MT = a.T / 16, kq = a.kq, ldv = a.ldv, ldE = a.ldE, ldG = a.ldG;
@@ -2271,81 +2270,82 @@ __global__ void __launch_bounds__(NW * 32, (NTF > 0 && !MIX && NW == 8) ? 2 : 1)
         ctl[0] = 0;
         ctl[1] = 0;
         ctl[2] = 0;
-        ctl[4] = 0;
         for (int b = 0; b < 3; b++) {
             mbar_init(&L.bar[b], 1);
             mbar_init(&L.bar[3 + b], kWarps);
         }
         mbar_init_fence();
     }
+    // the Gaunt contraction table in shared memory, or read from global memory
+    // through L1 where the launch shape leaves no room for it (a compile-time
+    // choice: the 32-slot shape's table pointers stay shared-memory pointers,
+    // which the loads in phase B rely on)
+    const NewtonProblem &pb = a.prob;
+    if constexpr (R8 && NW == 8) {
+        if (a.useGaunt) {
+            L.ellVal = const_cast<double *>(pb.ellVal);
+            L.ellIdx = const_cast<unsigned short *>(pb.ellIdx);
+            L.ellPair = const_cast<unsigned short *>(pb.ellPair);
+            L.ellOff = const_cast<int *>(pb.ellOff);
+        }
+    } else if (a.useGaunt) {
+        for (int i = tid; i < pb.ellGroups * 256; i += kThreads) {
+            L.ellVal[i] = pb.ellVal[i];
+            L.ellIdx[i] = pb.ellIdx[i];
+        }
+        for (int i = tid; i < pb.ellChunks * 64; i += kThreads)
+            L.ellPair[i] = pb.ellPair[i];
+        for (int i = tid; i <= pb.ellChunks; i += kThreads)
+            L.ellOff[i] = pb.ellOff[i];
+    }
     __syncthreads();
-    int loadedProb = -1;
+    bool first = true;      // warp 0: the CTA's first share of the vectors is still to come
     unsigned mbPhase = 0;   // parity of the next phase of each chunk mbarrier (full; empty three bits up)
 
     for (;;) {
-        // ---- refill idle slots from the work counter of the current problem:
-        // warp 0, lane s for slot s.  A launch with fewer vectors than slots
-        // spreads them over the CTAs (quota per CTA): the first quota of each
-        // CTA are the vectors blockIdx.x + k * gridDim.x, so that the longest
-        // chains, listed first, fall to different CTAs; the work counter hands
-        // out the rest.
+        // ---- refill idle slots from the work counter: warp 0, lane s for slot
+        // s.  A launch with fewer vectors than slots spreads them over the
+        // CTAs (quota per CTA): the first quota of each CTA are the vectors
+        // blockIdx.x + k * gridDim.x, so that the longest chains, listed
+        // first, fall to different CTAs; the work counter hands out the rest.
         if (warp == 0) {
             int *si = L.ints + lane * SI_N;
-            const bool mine = lane < T;
-            int p = ctl[0];
-            int st = mine ? si[SI_STATE] : -1;
+            int st = (lane < T) ? si[SI_STATE] : -1;
             if (st == S_HELP) {   // helpers serve one round
                 st = S_IDLE;
                 si[SI_STATE] = S_IDLE;
             }
             unsigned idle = __ballot_sync(0xffffffffu, st == S_IDLE);
             int nActive = T - __popc(idle);
-            bool exhausted = ctl[2] != 0;
-            while (idle) {
-                if (exhausted) {
-                    if (nActive == 0 && p + 1 < a.nprob) {
-                        p++;
-                        exhausted = false;
-                        continue;
-                    }
-                    break;
-                }
-                const NewtonProblem &pb = a.prob[p];
-                const bool list = pb.cellList && *pb.countDev >= 0;
-                const int count = list ? *pb.countDev : pb.count;
-                const int quota = (count + (int)gridDim.x - 1) / (int)gridDim.x;
-                const int cap = min(T, quota);
-                int item = -1;   // this lane's vector
+            bool exhausted = ctl[1] != 0;
+            const bool list = pb.cellList && *pb.countDev >= 0;
+            const int count = list ? *pb.countDev : pb.count;
+            const int quota = (count + (int)gridDim.x - 1) / (int)gridDim.x;
+            const int cap = min(T, quota);
+            while (idle && !exhausted) {
+                long long at;   // this lane's vector
                 const int rank = __popc(idle & ((1u << lane) - 1u));
-                const bool isIdle = (idle >> lane) & 1u;
-                if (nActive == 0 && ctl[4] <= p) {
-                    // the CTA's first vectors of this problem
-                    const int at = (int)blockIdx.x + rank * (int)gridDim.x;
-                    if (isIdle && rank < cap && at < count)
-                        item = at;
-                    __syncwarp();
-                    if (lane == 0)
-                        ctl[4] = p + 1;
-                    __syncwarp();
-                    if (cap == quota)   // quota <= T: the CTAs took everything
-                        exhausted = true;
+                if (first) {
+                    // the CTA's first share (everything, when quota <= T)
+                    at = (rank < cap) ? (long long)blockIdx.x + (long long)rank * gridDim.x : count;
+                    first = false;
+                    exhausted = cap == quota;
                 } else {
                     const int want = __popc(idle);
                     unsigned base = 0;
                     if (lane == 0)
                         base = atomicAdd(pb.queue, (unsigned)want);
                     base = __shfl_sync(0xffffffffu, base, 0);
-                    const long long at = (long long)cap * gridDim.x + base + rank;
-                    if (isIdle && at < count)
-                        item = (int)at;
-                    if ((long long)cap * gridDim.x + base + want > count)
-                        exhausted = true;
+                    const long long next = (long long)cap * gridDim.x + base;
+                    at = next + rank;
+                    exhausted = next + want > count;
                 }
-                if (item >= 0) {
-                    si[SI_CELL] = list ? pb.cellList[item] : pb.first + item;
+                const bool take = ((idle >> lane) & 1u) && at < count;
+                if (take) {
+                    si[SI_CELL] = list ? pb.cellList[at] : pb.first + (int)at;
                     si[SI_STATE] = S_NEW;
                 }
-                const unsigned got = __ballot_sync(0xffffffffu, item >= 0);
+                const unsigned got = __ballot_sync(0xffffffffu, take);
                 nActive += __popc(got);
                 idle &= ~got;
             }
@@ -2362,41 +2362,14 @@ __global__ void __launch_bounds__(NW * 32, (NTF > 0 && !MIX && NW == 8) ? 2 : 1)
                 }
             }
             if (lane == 0) {
-                ctl[0] = p;
-                ctl[2] = exhausted ? 1 : 0;
-                ctl[1] = (nActive == 0) ? 1 : 0;
-                ctl[3] = 0;
+                ctl[0] = (nActive == 0) ? 1 : 0;
+                ctl[1] = exhausted ? 1 : 0;
+                ctl[2] = 0;
             }
         }
         __syncthreads();
-        if (ctl[1])
+        if (ctl[0])
             break;
-        const NewtonProblem &pb = a.prob[ctl[0]];
-        if (ctl[0] != loadedProb) {
-            // stage this order's Gaunt contraction table in shared memory
-            // (or read it from global memory through L1 where the launch
-            // shape leaves no room for it)
-            loadedProb = ctl[0];
-            // (a compile-time choice: the 32-slot shape's table pointers stay
-            // shared-memory pointers, which the loads in phase B rely on)
-            if constexpr (R8 && NW == 8) {
-                if (a.useGaunt) {
-                    L.ellVal = const_cast<double *>(pb.ellVal);
-                    L.ellIdx = const_cast<unsigned short *>(pb.ellIdx);
-                    L.ellPair = const_cast<unsigned short *>(pb.ellPair);
-                    L.ellOff = const_cast<int *>(pb.ellOff);
-                }
-            } else if (a.useGaunt) {
-                for (int i = tid; i < pb.ellGroups * 256; i += kThreads) {
-                    L.ellVal[i] = pb.ellVal[i];
-                    L.ellIdx[i] = pb.ellIdx[i];
-                }
-                for (int i = tid; i < pb.ellChunks * 64; i += kThreads)
-                    L.ellPair[i] = pb.ellPair[i];
-                for (int i = tid; i <= pb.ellChunks; i += kThreads)
-                    L.ellOff[i] = pb.ellOff[i];
-            }
-        }
         for (int s = warp; s < T; s += kWarps) {
             const int st = L.ints[s * SI_N + SI_STATE];
             if (st == S_NEW)
@@ -2580,7 +2553,7 @@ __global__ void __launch_bounds__(NW * 32, (NTF > 0 && !MIX && NW == 8) ? 2 : 1)
         for (;;) {
             int s = 0;
             if (lane == 0)
-                s = atomicAdd(&ctl[3], 1);
+                s = atomicAdd(&ctl[2], 1);
             s = __shfl_sync(0xffffffffu, s, 0);
             if (s >= T)
                 break;
@@ -2660,7 +2633,7 @@ __global__ void __launch_bounds__(256, 2) screen_kernel(const __grid_constant__ 
     __shared__ int repValid, repHits;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int T = a.T, ldv = a.ldv;
-    const NewtonProblem &pb = a.prob[0];
+    const NewtonProblem &pb = a.prob;
     const int n = pb.n;
     Layout L = make_layout(sm, a);
     // The representative: the start (u, alpha) of a cell this CTA settled,

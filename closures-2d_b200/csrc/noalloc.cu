@@ -171,8 +171,7 @@ extern "C" int cl_solve_batch_noalloc(const cl_angular *ang, const cl_options *o
 
     NewtonArgs a;
     std::memset(&a, 0, sizeof(a));
-    a.nprob = 1;
-    NewtonProblem &pb = a.prob[0];
+    NewtonProblem &pb = a.prob;
     pb.P = (const double *)(base + offP);
     pb.w = (const double *)(base + offW);
     pb.pairs = (const unsigned short *)(base + offPairs);

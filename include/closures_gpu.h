@@ -296,7 +296,7 @@ int cl_solve_batch_cb_device(cl_ctx *ctx, int count, double *d_u, double *d_P2M,
                              double *d_alpha, int *d_iters, double *d_reg, int *d_status);
 
 /* Mixed-order batch: a solver context for several moment orders at one
- * quadrature order, so vectors of different N share one persistent launch.
+ * quadrature order; the orders' launches run side by side on the device.
  * Device pointers; vectors of order orders[s] are packed in segment s. */
 typedef struct cl_multi cl_multi;
 int cl_multi_create(int norders, const int *orders, int quad_order, int use_gaunt,
