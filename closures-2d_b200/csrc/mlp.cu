@@ -9,8 +9,9 @@
 // from the previous stage's alpha (momopt_update.cpp:236-238).
 //
 // Network: n -> W -> W -> W -> n with GELU (exact erf form) between layers,
-// BF16 weights and activations feeding tensor-core MMAs (mma.sync m16n8k16,
-// BF16 x BF16 -> FP32), FP32 master weights, FP32 Adam.  Outputs are the
+// BF16 weights and activations feeding tensor-core MMAs (forward: tcgen05;
+// backward: mma.sync m16n8k16, BF16 x BF16 -> FP32), FP32 master weights, FP32
+// Adam.  Outputs are the
 // multipliers standardised per component with the training set's mean and
 // standard deviation.  Training and inference both run on these kernels.
 #include "closures_gpu.h"
@@ -31,11 +32,8 @@
 namespace {
 
 constexpr int kLayers = 4;
-constexpr int BM = 64, BN = 64, BK = 32, KPAD = 8;
 constexpr double kSqrtPi = 1.7724538509055160273;
 constexpr double kPi = 3.14159265358979323846;
-
-enum Epi { EPI_F32 = 0, EPI_BIAS_GELU = 1, EPI_BIAS = 2 };
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_grad(float z)
@@ -54,30 +52,135 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], unsigned a0, unsigned a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// C[M x N] = op(A)[M x K] . op(B)[K x N].  A is [M x K] row-major (TA = 0) or
-// [K x M] (TA = 1); B is [K x N] row-major (TB = 0) or [N x K] (TB = 1).
-// Epilogues: FP32 store; bias + GELU (pre-activation FP32, activation BF16);
-// bias (FP32).  Tiles 64 x 64 x 32, four warps of 32 x 32.
-// Mdev (nullable): the rows come from a device count, M = min(M, *Mdev - moff)
-// (a compacted selection whose size the host does not know); tiles past it
-// return at once.
-template <int TA, int TB, int EPI>
-__global__ void __launch_bounds__(128) gemm_kernel(const __nv_bfloat16 *__restrict__ A,
-                                                   const __nv_bfloat16 *__restrict__ B, int M, int N, int K,
-                                                   float *__restrict__ C, const float *__restrict__ bias,
-                                                   __nv_bfloat16 *__restrict__ Act, const int *Mdev, int moff)
+// Asynchronous 16-byte copy to shared memory, zero-filled when !valid.
+__device__ __forceinline__ void cp16_zfill(void *smem, const void *gmem, bool valid)
 {
-    __shared__ __align__(16) __nv_bfloat16 As[BM][BK + KPAD];
-    __shared__ __align__(16) __nv_bfloat16 Bs[BN][BK + KPAD];
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    const int bytes = valid ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4(unsigned (&r)[4], const void *p)
+{
+    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(s));
+}
+__device__ __forceinline__ void ldmatrix4_t(unsigned (&r)[4], const void *p)
+{
+    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(s));
+}
+
+// One layer of the backward pass in one launch.  Its three products need
+// only the layer's dZ, so their CTAs run side by side:
+//   dW = in^T . dZ           64 x 64 tiles, K = rows
+//   db = column sums of dZ   32 columns per CTA
+//   dA . gelu'(Z) = next dZ  64 x 64 tiles of dZ . W^T, K = N (layers above 0)
+// Every sum runs in the order of a plain loop over K in steps of 16 (mma.sync
+// m16n8k16, the k-steps of one output a single chain; db one addition per
+// row), so the gradients do not depend on the tiling, and training, whose
+// first Adam steps divide gradients by their own size, is reproducible to the
+// bit.  The chains set the time: 256 dependent MMAs for 4096 rows.  So the
+// operands, staged with 16-byte asynchronous copies four stages deep, have to
+// arrive faster than that (through scalar loads the four dW took 1810 us a
+// step at 4096 x 512, the column sums 910, dA 164).
+// Row strides (ldin, ldz, ldw) are multiples of 8.
+struct BackArgs {
+    const __nv_bfloat16 *in;   // [rows][ldin], K columns
+    const __nv_bfloat16 *dZ;   // [rows][ldz], N columns
+    const float *dZf;          // [rows][ldz]
+    const __nv_bfloat16 *W;    // [K][ldw]: row i the weights of input i (ldw >= N, zero padded)
+    const float *Zprev;        // [rows][K] pre-activations of the layer below; null for layer 0
+    float *gW, *gb;            // [K][N], [N]
+    __nv_bfloat16 *dZnext;     // [rows][ldn], K columns
+    float *dZfnext;
+    int rows, K, N, ldin, ldz, ldw, ldn;
+    int tilesW, tilesB;        // dW tiles, db CTAs; the rest are dA tiles
+};
+constexpr int kBackStages = 4, kBackK = 64;
+constexpr int kBackTile = 64 * (kBackK + 8);   // bf16 of one staged operand (rows padded by 16 bytes)
+constexpr int kBackSmem = kBackStages * 2 * kBackTile * 2;
+
+__global__ void __launch_bounds__(128) backward_kernel(const BackArgs a)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    if (Mdev) {
-        const int rem = *Mdev - moff;
-        M = rem < M ? (rem > 0 ? rem : 0) : M;
-        if (m0 >= M)
-            return;
+    int block = blockIdx.x;
+    if (block >= a.tilesW && block < a.tilesW + a.tilesB) {
+        // db: warp 0 adds the rows in order, all threads stage them
+        constexpr int R = 64, S = 6;   // rows per stage, stages: 48 KB
+        float *buf = reinterpret_cast<float *>(smraw);
+        const int j0 = (block - a.tilesW) * 32;
+        const int nst = (a.rows + R - 1) / R;
+        auto load = [&](int st) {
+            float *d = buf + (st % S) * (R * 32);
+            for (int i = tid; i < R * 8; i += 128) {
+                const int r = st * R + i / 8, c = j0 + (i % 8) * 4;
+                const bool ok = r < a.rows && c < a.ldz;
+                cp16_zfill(d + (i / 8) * 32 + (i % 8) * 4, a.dZf + (ok ? (size_t)r * a.ldz + c : 0), ok);
+            }
+        };
+        for (int st = 0; st < S - 1; st++) {
+            if (st < nst)
+                load(st);
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        }
+        float s = 0.0f;
+        for (int st = 0; st < nst; st++) {
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(S - 2) : "memory");
+            __syncthreads();
+            if (st + S - 1 < nst)
+                load(st + S - 1);
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+            if (warp == 0) {
+                const float *d = buf + (st % S) * (R * 32) + lane;
+                const int cnt = min(R, a.rows - st * R);
+                if (cnt == R) {
+#pragma unroll
+                    for (int r = 0; r < R; r++)
+                        s += d[r * 32];
+                } else {
+                    for (int r = 0; r < cnt; r++)
+                        s += d[r * 32];
+                }
+            }
+        }
+        if (warp == 0 && j0 + lane < a.N)
+            a.gb[j0 + lane] = s;
+        return;
     }
+    const bool isW = block < a.tilesW;
+    if (!isW)
+        block -= a.tilesW + a.tilesB;
+    // C [M x N] = A . B over kTot: dW: A = in^T, B = dZ, both staged as [k][64];
+    // dA: A = dZ, B = W^T, staged as [64][k]
+    const int M = isW ? a.K : a.rows, N = isW ? a.N : a.K, kTot = isW ? a.rows : a.ldw;
+    const int tn = (N + 63) / 64;
+    const int m0 = (block / tn) * 64, n0 = (block % tn) * 64;
+    const __nv_bfloat16 *A = isW ? a.in : a.dZ, *B = isW ? a.dZ : a.W;
+    const int lda = isW ? a.ldin : a.ldz, ldb = isW ? a.ldz : a.ldw;
+    __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(smraw), *sB = sA + kBackStages * kBackTile;
+    constexpr int LD = kBackK + 8;   // also 64 + 8 for the [k][64] form
+    const int nst = (kTot + kBackK - 1) / kBackK;
+    auto load = [&](int st) {
+        __nv_bfloat16 *da = sA + (st % kBackStages) * kBackTile, *db = sB + (st % kBackStages) * kBackTile;
+        const int k0 = st * kBackK;
+        for (int i = tid; i < 64 * 8; i += 128) {
+            const int r = i / 8, c = (i % 8) * 8;
+            if (isW) {
+                const bool okA = k0 + r < kTot && m0 + c < lda, okB = k0 + r < kTot && n0 + c < ldb;
+                cp16_zfill(da + r * LD + c, A + (okA ? (size_t)(k0 + r) * lda + m0 + c : 0), okA);
+                cp16_zfill(db + r * LD + c, B + (okB ? (size_t)(k0 + r) * ldb + n0 + c : 0), okB);
+            } else {
+                const bool okA = m0 + r < M && k0 + c < lda, okB = n0 + r < N && k0 + c < ldb;
+                cp16_zfill(da + r * LD + c, A + (okA ? (size_t)(m0 + r) * lda + k0 + c : 0), okA);
+                cp16_zfill(db + r * LD + c, B + (okB ? (size_t)(n0 + r) * ldb + k0 + c : 0), okB);
+            }
+        }
+    };
     const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
     float acc[2][4][4];
 #pragma unroll
@@ -85,84 +188,84 @@ __global__ void __launch_bounds__(128) gemm_kernel(const __nv_bfloat16 *__restri
 #pragma unroll
         for (int j = 0; j < 4; j++)
             acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0f;
-    const __nv_bfloat16 zero = __float2bfloat16(0.0f);
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        for (int idx = tid; idx < BM * BK; idx += 128) {
-            int r = idx / BK, c = idx % BK;
-            int m = m0 + r, k = k0 + c;
-            __nv_bfloat16 v = zero;
-            if (m < M && k < K)
-                v = TA ? A[(size_t)k * M + m] : A[(size_t)m * K + k];
-            As[r][c] = v;
-        }
-        for (int idx = tid; idx < BN * BK; idx += 128) {
-            int r = idx / BK, c = idx % BK;
-            int nn = n0 + r, k = k0 + c;
-            __nv_bfloat16 v = zero;
-            if (nn < N && k < K)
-                v = TB ? B[(size_t)nn * K + k] : B[(size_t)k * N + nn];
-            Bs[r][c] = v;
-        }
+    for (int st = 0; st < kBackStages - 1; st++) {
+        if (st < nst)
+            load(st);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    for (int st = 0; st < nst; st++) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kBackStages - 2) : "memory");
         __syncthreads();
+        if (st + kBackStages - 1 < nst)
+            load(st + kBackStages - 1);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const __nv_bfloat16 *ta = sA + (st % kBackStages) * kBackTile, *tb = sB + (st % kBackStages) * kBackTile;
 #pragma unroll
-        for (int kk = 0; kk < BK; kk += 16) {
-            unsigned a[2][4], b[4][2];
+        for (int kk = 0; kk < kBackK; kk += 16) {
+            unsigned fa[2][4], fb[2][4];
+            if (isW) {
+                // [k][m]: 8x8 blocks (k, m) transposed; block order m, m + 8, then k + 8
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
-                int r = wm + i * 16 + g;
-                a[i][0] = *reinterpret_cast<const unsigned *>(&As[r][kk + 2 * t]);
-                a[i][1] = *reinterpret_cast<const unsigned *>(&As[r + 8][kk + 2 * t]);
-                a[i][2] = *reinterpret_cast<const unsigned *>(&As[r][kk + 2 * t + 8]);
-                a[i][3] = *reinterpret_cast<const unsigned *>(&As[r + 8][kk + 2 * t + 8]);
-            }
+                for (int i = 0; i < 2; i++)
+                    ldmatrix4_t(fa[i], ta + (kk + (lane & 7) + ((lane >> 4) & 1) * 8) * LD + wm + i * 16 +
+                                           ((lane >> 3) & 1) * 8);
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                int c = wn + j * 8 + g;
-                b[j][0] = *reinterpret_cast<const unsigned *>(&Bs[c][kk + 2 * t]);
-                b[j][1] = *reinterpret_cast<const unsigned *>(&Bs[c][kk + 2 * t + 8]);
+                for (int j = 0; j < 2; j++)
+                    ldmatrix4_t(fb[j], tb + (kk + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + wn + j * 16 +
+                                           ((lane >> 4) & 1) * 8);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+                    ldmatrix4(fa[i], ta + (wm + i * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + kk +
+                                         ((lane >> 4) & 1) * 8);
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+                    ldmatrix4(fb[j], tb + (wn + j * 16 + (lane & 7) + ((lane >> 4) & 1) * 8) * LD + kk +
+                                         ((lane >> 3) & 1) * 8);
             }
 #pragma unroll
             for (int i = 0; i < 2; i++)
 #pragma unroll
                 for (int j = 0; j < 4; j++)
-                    mma_bf16(acc[i][j], a[i][0], a[i][1], a[i][2], a[i][3], b[j][0], b[j][1]);
+                    mma_bf16(acc[i][j], fa[i][0], fa[i][1], fa[i][2], fa[i][3], fb[j >> 1][(j & 1) * 2],
+                             fb[j >> 1][(j & 1) * 2 + 1]);
         }
-        __syncthreads();
     }
+    const int g = lane >> 2, t = lane & 3;
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++)
 #pragma unroll
             for (int h = 0; h < 4; h++) {
-                int m = m0 + wm + i * 16 + g + ((h & 2) ? 8 : 0);
-                int nn = n0 + wn + j * 8 + 2 * t + (h & 1);
+                const int m = m0 + wm + i * 16 + g + ((h & 2) ? 8 : 0);
+                const int nn = n0 + wn + j * 8 + 2 * t + (h & 1);
                 if (m >= M || nn >= N)
                     continue;
-                float v = acc[i][j][h];
-                if (EPI == EPI_F32) {
-                    C[(size_t)m * N + nn] = v;
-                } else if (EPI == EPI_BIAS_GELU) {
-                    v += bias[nn];
-                    C[(size_t)m * N + nn] = v;
-                    Act[(size_t)m * N + nn] = __float2bfloat16(gelu(v));
+                if (isW) {
+                    a.gW[(size_t)m * N + nn] = acc[i][j][h];
                 } else {
-                    C[(size_t)m * N + nn] = v + bias[nn];
+                    const float v = acc[i][j][h] * gelu_grad(a.Zprev[(size_t)m * N + nn]);
+                    a.dZnext[(size_t)m * a.ldn + nn] = __float2bfloat16(v);
+                    a.dZfnext[(size_t)m * a.ldn + nn] = v;
                 }
             }
 }
 
-__global__ void cast_bf16_kernel(const float *x, __nv_bfloat16 *y, size_t n)
+// W [K x N] FP32 -> W16 [K x ldw] BF16, zero columns N..ldw-1
+__global__ void cast_bf16_kernel(const float *W, int K, int N, int ldw, __nv_bfloat16 *W16)
 {
     size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (i < n)
-        y[i] = __float2bfloat16(x[i]);
+    if (i >= (size_t)K * ldw)
+        return;
+    const int r = (int)(i / ldw), c = (int)(i % ldw);
+    W16[i] = __float2bfloat16(c < N ? W[(size_t)r * N + c] : 0.0f);
 }
 
-// dY = 2 (Y - T) / (B n) for the mean squared error over B x n entries; returns
-// per-block partial losses.
-__global__ void mse_grad_kernel(const float *Y, const float *T, __nv_bfloat16 *dY, float *dYf, int total, float scale,
-                                float *lossPart)
+// dY = 2 (Y - T) / (B n) for the mean squared error over B x n entries, row
+// stride ld; returns per-block partial losses.
+__global__ void mse_grad_kernel(const float *Y, const float *T, __nv_bfloat16 *dY, float *dYf, int total, int n, int ld,
+                                float scale, float *lossPart)
 {
     __shared__ float red[256];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -171,8 +274,12 @@ __global__ void mse_grad_kernel(const float *Y, const float *T, __nv_bfloat16 *d
         float d = Y[i] - T[i];
         l = d * d;
         float gval = 2.0f * d * scale;
-        dY[i] = __float2bfloat16(gval);
-        dYf[i] = gval;
+        const size_t at = (size_t)(i / n) * ld + i % n;
+        dY[at] = __float2bfloat16(gval);
+        dYf[at] = gval;
+        if (i % n == n - 1)   // the padding columns are operands too
+            for (int k = 1; k <= ld - n; k++)
+                dY[at + k] = __float2bfloat16(0.0f);
     }
     red[threadIdx.x] = l;
     __syncthreads();
@@ -185,53 +292,69 @@ __global__ void mse_grad_kernel(const float *Y, const float *T, __nv_bfloat16 *d
         lossPart[blockIdx.x] = red[0];
 }
 
-// dZ = dA * gelu'(Z)
-__global__ void gelu_back_kernel(const float *dA, const float *Z, __nv_bfloat16 *dZ, float *dZf, size_t n)
+__device__ __forceinline__ float adam(float w, float *m, float *v, float gi, float lr, float b1, float b2, float eps,
+                                      float c1, float c2)
 {
-    size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (i < n) {
-        float v = dA[i] * gelu_grad(Z[i]);
-        dZ[i] = __float2bfloat16(v);
-        dZf[i] = v;
-    }
+    float mi = b1 * *m + (1.0f - b1) * gi;
+    float vi = b2 * *v + (1.0f - b2) * gi * gi;
+    *m = mi;
+    *v = vi;
+    w -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    return w;
 }
 
-// db[j] = sum_rows dZ[r][j]
-__global__ void colsum_kernel(const float *dZ, int rows, int cols, float *db)
-{
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < cols) {
-        float s = 0.0f;
-        for (int r = 0; r < rows; r++)
-            s += dZ[(size_t)r * cols + j];
-        db[j] = s;
-    }
-}
+// Adam on every parameter, and the BF16 copies of the weights the GEMMs read
+// (row-major and transposed), in one launch: 32 x 32 tiles of each weight
+// matrix, transposed through shared memory, then the biases 256 to a block.
+// (Eight launches of Adam and eight of the copies took 50 us a step.)
+struct UpdateArgs {
+    float *W[kLayers], *mW[kLayers], *vW[kLayers], *b[kLayers], *mb[kLayers], *vb[kLayers];
+    const float *gW[kLayers], *gb[kLayers];
+    __nv_bfloat16 *W16[kLayers], *Wt16[kLayers];
+    int dims[kLayers + 1], first[kLayers + 1];   // first tile of each layer; first[kLayers]: of the biases
+    float lr, b1, b2, eps, c1, c2;
+};
 
-// rows perm[0..batch) of (u, alpha) into contiguous minibatch buffers
-__global__ void gather_kernel(const double *u, const double *alpha, const int *perm, int batch, int n, double *bu,
-                              double *ba)
+__global__ void __launch_bounds__(256) update_kernel(const UpdateArgs a)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < batch * n) {
-        int r = i / n, k = i % n;
-        size_t src = (size_t)perm[r] * n + k;
-        bu[i] = u[src];
-        ba[i] = alpha[src];
+    __shared__ __nv_bfloat16 tile[32][34];
+    int block = blockIdx.x;
+    const int tid = threadIdx.x;
+    if (block >= a.first[kLayers]) {
+        int j = (block - a.first[kLayers]) * 256 + tid;
+        for (int l = 0; l < kLayers; l++) {
+            const int N = a.dims[l + 1];
+            if (j < N) {
+                a.b[l][j] = adam(a.b[l][j], a.mb[l] + j, a.vb[l] + j, a.gb[l][j], a.lr, a.b1, a.b2, a.eps, a.c1, a.c2);
+                return;
+            }
+            j -= N;
+        }
+        return;
     }
-}
-
-__global__ void adam_kernel(float *w, float *m, float *v, const float *g, size_t n, float lr, float b1, float b2,
-                            float eps, float c1, float c2)
-{
-    size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (i < n) {
-        float gi = g[i];
-        float mi = b1 * m[i] + (1.0f - b1) * gi;
-        float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    int l = 0;
+    while (block >= a.first[l + 1])
+        l++;
+    block -= a.first[l];
+    const int K = a.dims[l], N = a.dims[l + 1], ldw = (N + 7) / 8 * 8, Kp = (K + 7) / 8 * 8;
+    const int tn = (N + 31) / 32, i0 = (block / tn) * 32, j0 = (block % tn) * 32;
+    const int x = tid & 31, y = tid >> 5;
+    for (int r = y; r < 32; r += 8) {
+        const int i = i0 + r, j = j0 + x;
+        if (i < K && j < N) {
+            const size_t at = (size_t)i * N + j;
+            const float w = adam(a.W[l][at], a.mW[l] + at, a.vW[l] + at, a.gW[l][at], a.lr, a.b1, a.b2, a.eps, a.c1, a.c2);
+            a.W[l][at] = w;
+            const __nv_bfloat16 h = __float2bfloat16(w);
+            a.W16[l][(size_t)i * ldw + j] = h;
+            tile[r][x] = h;
+        }
+    }
+    __syncthreads();
+    for (int r = y; r < 32; r += 8) {
+        const int j = j0 + r, i = i0 + x;
+        if (i < K && j < N)
+            a.Wt16[l][(size_t)j * Kp + i] = tile[x][r];
     }
 }
 
@@ -247,19 +370,21 @@ __device__ __forceinline__ double alpha_linear(int k, double x, int momentType)
     return k == 0 ? 2.0 * kSqrtPi * log(0.5 / kSqrtPi) : 2.0 * kSqrtPi * x;
 }
 
-// Inputs: x = u/u0 (BF16); targets (alpha_scaled - linear - mean)/std (FP32).
-__global__ void prep_kernel(const double *u, const double *alpha, int count, int n, int momentType,
-                            const float *mean, const float *stdv, __nv_bfloat16 *X, float *Tgt)
+// Inputs: x = u/u0 (BF16, row stride np); targets (alpha_scaled - linear -
+// mean)/std (FP32).  With perm (nullable) row c comes from vector perm[c].
+__global__ void prep_kernel(const double *u, const double *alpha, const int *perm, int count, int n, int np,
+                            int momentType, const float *mean, const float *stdv, __nv_bfloat16 *X, float *Tgt)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count * n)
         return;
     int c = i / n, k = i % n;
-    double u0 = u[(size_t)c * n];
-    double x = u[i] / u0;
-    X[i] = __float2bfloat16((float)x);
+    const size_t row = (size_t)(perm ? perm[c] : c) * n;
+    double u0 = u[row];
+    double x = u[row + k] / u0;
+    X[(size_t)c * np + k] = __float2bfloat16((float)x);
     if (Tgt) {
-        double a = alpha[i];
+        double a = alpha[row + k];
         if (momentType == CL_MN) {
             if (k == 0)
                 a -= log(u0) * 2.0 * kSqrtPi;
@@ -322,15 +447,6 @@ __global__ void predict_out_kernel(const float *Y, const double *u, double *alph
     }
 }
 
-template <int TA, int TB, int EPI>
-cudaError_t gemm(const __nv_bfloat16 *A, const __nv_bfloat16 *B, int M, int N, int K, float *C, const float *bias,
-                 __nv_bfloat16 *Act, cudaStream_t s, const int *Mdev = nullptr, int moff = 0)
-{
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    gemm_kernel<TA, TB, EPI><<<grid, 128, 0, s>>>(A, B, M, N, K, C, bias, Act, Mdev, moff);
-    return cudaGetLastError();
-}
-
 // Cells whose last optimisation took at least minIters iterations are listed
 // in idx (count in *cnt, order arbitrary); the others get a NaN start, so the
 // Newton kernel starts them from their own (previous-stage) multipliers.
@@ -346,7 +462,7 @@ __global__ void select_kernel(const int *iters, int count, int minIters, int *id
 }
 
 // Inputs x = u/u0 of the listed cells idx[off + r], r < min(rows, *cnt - off).
-__global__ void prep_idx_kernel(const double *u, const int *idx, const int *cnt, int off, int rows, int n,
+__global__ void prep_idx_kernel(const double *u, const int *idx, const int *cnt, int off, int rows, int n, int np,
                                 __nv_bfloat16 *X)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -354,23 +470,12 @@ __global__ void prep_idx_kernel(const double *u, const int *idx, const int *cnt,
     if (r >= rows || off + r >= *cnt)
         return;
     const size_t c = (size_t)idx[off + r];
-    X[i] = __float2bfloat16((float)(u[c * n + k] / u[c * n]));
+    X[(size_t)r * np + k] = __float2bfloat16((float)(u[c * n + k] / u[c * n]));
 }
 
 int blocks(size_t n, int t = 256) { return (int)((n + t - 1) / t); }
 
 int round8(int x) { return (x + 7) / 8 * 8; }
-
-// x [rows x n] -> xp [rows x np] with zero columns n..np-1 (a row stride of a
-// multiple of 16 bytes, as the tensor-memory GEMM's TMA loads need)
-__global__ void pad_cols_kernel(const __nv_bfloat16 *x, int rows, int n, int np, __nv_bfloat16 *xp)
-{
-    size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (i >= (size_t)rows * np)
-        return;
-    const int r = (int)(i / np), k = (int)(i % np);
-    xp[i] = k < n ? x[(size_t)r * n + k] : __float2bfloat16(0.0f);
-}
 
 // W [K x N] FP32 row-major -> Wt [N x Kp] BF16 (the K-major B operand), zero
 // columns K..Kp-1
@@ -431,7 +536,7 @@ int sm_count_dev()
 // The persistent tensor-memory GEMM: one CTA per SM (or per tile, if fewer).
 template <int BN, int EPI>
 cudaError_t tc_gemm_bn(const CUtensorMap &ma, const CUtensorMap &mb, int M, int N, int K, float *Z, const float *bias,
-                       __nv_bfloat16 *Act, const int *Mdev, int moff, int *err, cudaStream_t s)
+                       __nv_bfloat16 *Act, int ldAct, const int *Mdev, int moff, int *err, cudaStream_t s)
 {
     static bool attr = false;
     auto *k = clb::tc::tc_gemm_persistent_kernel<BN, EPI>;
@@ -444,25 +549,25 @@ cudaError_t tc_gemm_bn(const CUtensorMap &ma, const CUtensorMap &mb, int M, int 
     }
     const int tiles = ((N + BN - 1) / BN) * ((M + clb::tc::BM - 1) / clb::tc::BM);
     const int grid = tiles < sm_count_dev() ? tiles : sm_count_dev();
-    k<<<grid, 192, smem, s>>>(ma, mb, M, N, K, Z, bias, Act, Mdev, moff, err);
+    k<<<grid, 192, smem, s>>>(ma, mb, M, N, K, Z, bias, Act, ldAct, Mdev, moff, err);
     return cudaGetLastError();
 }
 
-// Z (nullable) / Act (nullable) [M x N] = epilogue(A [M x K] . B [N x K]^T):
-// the tensor-memory GEMM (tc_gemm.cuh); K a multiple of 8.
+// Z (nullable) [M x N] / Act (nullable) [M x ldAct] = epilogue(A [M x K] .
+// B [N x K]^T): the tensor-memory GEMM (tc_gemm.cuh); K a multiple of 8.
 template <int EPI>
 cudaError_t tc_gemm(const __nv_bfloat16 *A, const __nv_bfloat16 *B, int M, int N, int K, float *Z, const float *bias,
-                    __nv_bfloat16 *Act, const int *Mdev, int moff, int *err, cudaStream_t s)
+                    __nv_bfloat16 *Act, int ldAct, const int *Mdev, int moff, int *err, cudaStream_t s)
 {
     const int bn = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
     CUtensorMap ma, mb;
     if (!bf16_map(&ma, A, M, K, clb::tc::BM) || !bf16_map(&mb, B, N, K, bn))
         return cudaErrorInvalidValue;
     if (bn == 32)
-        return tc_gemm_bn<32, EPI>(ma, mb, M, N, K, Z, bias, Act, Mdev, moff, err, s);
+        return tc_gemm_bn<32, EPI>(ma, mb, M, N, K, Z, bias, Act, ldAct, Mdev, moff, err, s);
     if (bn == 64)
-        return tc_gemm_bn<64, EPI>(ma, mb, M, N, K, Z, bias, Act, Mdev, moff, err, s);
-    return tc_gemm_bn<128, EPI>(ma, mb, M, N, K, Z, bias, Act, Mdev, moff, err, s);
+        return tc_gemm_bn<64, EPI>(ma, mb, M, N, K, Z, bias, Act, ldAct, Mdev, moff, err, s);
+    return tc_gemm_bn<128, EPI>(ma, mb, M, N, K, Z, bias, Act, ldAct, Mdev, moff, err, s);
 }
 
 }  // namespace
@@ -473,17 +578,25 @@ struct cl_mlp {
     int dims[kLayers + 1];
     float *W[kLayers] = {}, *b[kLayers] = {}, *mW[kLayers] = {}, *vW[kLayers] = {}, *mb[kLayers] = {},
           *vb[kLayers] = {}, *gW[kLayers] = {}, *gb[kLayers] = {};
-    __nv_bfloat16 *W16[kLayers] = {};
+    __nv_bfloat16 *W16[kLayers] = {};    // [in x round8(out)] BF16, zero padded (the backward GEMMs' operand)
     __nv_bfloat16 *Wt16[kLayers] = {};   // [out x round8(in)] BF16, the K-major operand of the forward GEMMs
     float *mean = nullptr, *stdv = nullptr;  // device [n]
     std::vector<float> hmean, hstd;
     int adamStep = 0;
     // work buffers (grow only)
     size_t cap = 0;
-    __nv_bfloat16 *X = nullptr, *Xp = nullptr, *Act[kLayers] = {}, *dZ16 = nullptr;   // Xp: X padded to round8(n)
+    // inputs [rows x round8(n)] and activations [rows x round8(width)], zero
+    // padded; dZ of the layer at hand and of the one below, row stride wp
+    __nv_bfloat16 *X = nullptr, *Act[kLayers] = {}, *dZ16[2] = {};
+    float *dZ[2] = {};
     int *tcErr = nullptr;       // error word of the tensor-memory GEMM's bounded waits
     bool keepZ = true;          // forward keeps the hidden pre-activations (training)
-    float *Z[kLayers] = {}, *T = nullptr, *dA = nullptr, *dZ = nullptr, *loss = nullptr;
+    float *Z[kLayers] = {}, *T = nullptr, *loss = nullptr;
+    // training: the epoch's permutation, the loss partials of kLossSteps steps
+    int *perm = nullptr;
+    size_t permCap = 0;
+    float *lossBuf = nullptr;
+    size_t lossCap = 0;
     int *fallbacks = nullptr;
     int *sel = nullptr;         // selected cells (+ their count) of cl_mlp_predict_selected
     size_t selCap = 0;
@@ -491,35 +604,50 @@ struct cl_mlp {
     std::string err;
 };
 
+constexpr int kLossSteps = 256;   // training steps between readbacks of the loss
+
+static void mlp_free_work(cl_mlp *m)
+{
+    cudaFree(m->X);
+    cudaFree(m->T);
+    cudaFree(m->loss);
+    m->X = nullptr;
+    m->T = m->loss = nullptr;
+    for (int h = 0; h < 2; h++) {
+        cudaFree(m->dZ16[h]);
+        cudaFree(m->dZ[h]);
+        m->dZ16[h] = nullptr;
+        m->dZ[h] = nullptr;
+    }
+    for (int l = 0; l < kLayers; l++) {
+        cudaFree(m->Act[l]);
+        cudaFree(m->Z[l]);
+        m->Act[l] = nullptr;
+        m->Z[l] = nullptr;
+    }
+    m->cap = 0;
+}
+
 static int mlp_reserve(cl_mlp *m, size_t rows)
 {
     if (rows <= m->cap)
         return CL_OK;
-    cudaFree(m->X);
-    cudaFree(m->Xp);
-    cudaFree(m->dZ16);
-    cudaFree(m->T);
-    cudaFree(m->dA);
-    cudaFree(m->dZ);
-    cudaFree(m->loss);
-    for (int l = 0; l < kLayers; l++) {
-        cudaFree(m->Act[l]);
-        cudaFree(m->Z[l]);
-    }
-    size_t w = (size_t)(m->width > m->n ? m->width : m->n);
-    bool ok = cudaMalloc(&m->X, rows * m->n * sizeof(__nv_bfloat16)) == cudaSuccess &&
-              cudaMalloc(&m->Xp, rows * round8(m->n) * sizeof(__nv_bfloat16)) == cudaSuccess &&
-              cudaMalloc(&m->dZ16, rows * w * sizeof(__nv_bfloat16)) == cudaSuccess &&
-              cudaMalloc(&m->T, rows * m->n * sizeof(float)) == cudaSuccess &&
-              cudaMalloc(&m->dA, rows * w * sizeof(float)) == cudaSuccess &&
-              cudaMalloc(&m->dZ, rows * w * sizeof(float)) == cudaSuccess &&
+    mlp_free_work(m);
+    const size_t w = (size_t)(m->width > m->n ? m->width : m->n), wp = (size_t)round8((int)w);
+    // padding columns stay zero: they are operands of the GEMMs
+    auto zeroed = [](auto **p, size_t cnt) {
+        return cudaMalloc(p, cnt * sizeof(**p)) == cudaSuccess && cudaMemset(*p, 0, cnt * sizeof(**p)) == cudaSuccess;
+    };
+    bool ok = zeroed(&m->X, rows * round8(m->n)) && cudaMalloc(&m->T, rows * m->n * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&m->loss, (rows * m->n / 256 + 2) * sizeof(float)) == cudaSuccess;
+    for (int h = 0; h < 2 && ok; h++)
+        ok = zeroed(&m->dZ16[h], rows * wp) && zeroed(&m->dZ[h], rows * wp);
     for (int l = 0; l < kLayers && ok; l++)
-        ok = cudaMalloc(&m->Act[l], rows * w * sizeof(__nv_bfloat16)) == cudaSuccess &&
-             cudaMalloc(&m->Z[l], rows * w * sizeof(float)) == cudaSuccess;
+        ok = zeroed(&m->Act[l], rows * wp) && cudaMalloc(&m->Z[l], rows * w * sizeof(float)) == cudaSuccess;
+    ok = ok && cudaDeviceSynchronize() == cudaSuccess;   // the fills, before work on other streams
     if (!ok) {
+        mlp_free_work(m);
         m->err = "MLP work buffer allocation failed";
-        m->cap = 0;
         return CL_ERR_CUDA;
     }
     m->cap = rows;
@@ -533,17 +661,15 @@ static int mlp_reserve(cl_mlp *m, size_t rows)
 // input padded to round8(n) columns, the weights as K-major BF16 copies.
 static cudaError_t mlp_forward(cl_mlp *m, int rows, const int *Mdev = nullptr, int moff = 0)
 {
-    const int np = round8(m->n);
-    pad_cols_kernel<<<blocks((size_t)rows * np), 256, 0, m->stream>>>(m->X, rows, m->n, np, m->Xp);
-    cudaError_t e = cudaGetLastError();
-    const __nv_bfloat16 *in = m->Xp;
+    cudaError_t e = cudaSuccess;
+    const __nv_bfloat16 *in = m->X;
     for (int l = 0; l < kLayers && e == cudaSuccess; l++) {
         const int K = round8(m->dims[l]), N = m->dims[l + 1];
         if (l < kLayers - 1)
             e = tc_gemm<clb::tc::EPI_BIAS_GELU>(in, m->Wt16[l], rows, N, K, m->keepZ ? m->Z[l] : nullptr, m->b[l],
-                                                 m->Act[l], Mdev, moff, m->tcErr, m->stream);
+                                                 m->Act[l], round8(N), Mdev, moff, m->tcErr, m->stream);
         else
-            e = tc_gemm<clb::tc::EPI_BIAS>(in, m->Wt16[l], rows, N, K, m->Z[l], m->b[l], nullptr, Mdev, moff,
+            e = tc_gemm<clb::tc::EPI_BIAS>(in, m->Wt16[l], rows, N, K, m->Z[l], m->b[l], nullptr, 0, Mdev, moff,
                                             m->tcErr, m->stream);
         in = m->Act[l];
     }
@@ -553,45 +679,61 @@ static cudaError_t mlp_forward(cl_mlp *m, int rows, const int *Mdev = nullptr, i
 static cudaError_t mlp_sync_weights(cl_mlp *m)
 {
     for (int l = 0; l < kLayers; l++) {
-        size_t cnt = (size_t)m->dims[l] * m->dims[l + 1];
-        cast_bf16_kernel<<<blocks(cnt), 256, 0, m->stream>>>(m->W[l], m->W16[l], cnt);
-        const int K = m->dims[l], N = m->dims[l + 1], Kp = round8(K);
+        const int K = m->dims[l], N = m->dims[l + 1], Kp = round8(K), ldw = round8(N);
+        cast_bf16_kernel<<<blocks((size_t)K * ldw), 256, 0, m->stream>>>(m->W[l], K, N, ldw, m->W16[l]);
         transpose_cast_kernel<<<blocks((size_t)N * Kp), 256, 0, m->stream>>>(m->W[l], K, N, Kp, m->Wt16[l]);
     }
     return cudaGetLastError();
 }
 
-// backward of the MSE loss for the batch in X/T; gradients into gW/gb
-static cudaError_t mlp_backward(cl_mlp *m, int rows, float *lossOut)
+static int loss_parts(const cl_mlp *m, int rows) { return blocks((size_t)rows * m->n); }
+
+static float loss_value(const float *part, int parts, int total)
 {
-    const int n = m->n;
-    const int total = rows * n;
-    int nb = blocks(total);
-    mse_grad_kernel<<<nb, 256, 0, m->stream>>>(m->Z[kLayers - 1], m->T, m->dZ16, m->dZ, total, 1.0f / (float)total,
-                                               m->loss);
+    double s = 0;
+    for (int i = 0; i < parts; i++)
+        s += part[i];
+    return (float)(s / total);
+}
+
+// backward of the MSE loss for the batch in X/T; gradients into gW/gb, the
+// loss partials (loss_parts of them) into `loss`
+static cudaError_t mlp_backward(cl_mlp *m, int rows, float *loss)
+{
+    const int n = m->n, total = rows * n;
+    mse_grad_kernel<<<loss_parts(m, rows), 256, 0, m->stream>>>(m->Z[kLayers - 1], m->T, m->dZ16[0], m->dZ[0], total, n,
+                                                                round8(n), 1.0f / (float)total, loss);
     cudaError_t e = cudaGetLastError();
-    for (int l = kLayers - 1; l >= 0 && e == cudaSuccess; l--) {
-        int K = m->dims[l], N = m->dims[l + 1];
-        const __nv_bfloat16 *in = (l == 0) ? m->X : m->Act[l - 1];
-        // dW_l = in^T . dZ_l   ([K x rows] . [rows x N])
-        e = gemm<1, 0, EPI_F32>(in, m->dZ16, K, N, rows, m->gW[l], nullptr, nullptr, m->stream);
-        colsum_kernel<<<blocks(N), 256, 0, m->stream>>>(m->dZ, rows, N, m->gb[l]);
-        if (l > 0 && e == cudaSuccess) {
-            // dA_{l-1} = dZ_l . W_l^T   ([rows x N] . [N x K])
-            e = gemm<0, 1, EPI_F32>(m->dZ16, m->W16[l], rows, K, N, m->dA, nullptr, nullptr, m->stream);
-            size_t cnt = (size_t)rows * K;
-            gelu_back_kernel<<<blocks(cnt), 256, 0, m->stream>>>(m->dA, m->Z[l - 1], m->dZ16, m->dZ, cnt);
+    for (int l = kLayers - 1, h = 0; l >= 0 && e == cudaSuccess; l--, h ^= 1) {
+        BackArgs a;
+        a.rows = rows;
+        a.K = m->dims[l];
+        a.N = m->dims[l + 1];
+        a.in = (l == 0) ? m->X : m->Act[l - 1];
+        a.ldin = round8(a.K);
+        a.dZ = m->dZ16[h];
+        a.dZf = m->dZ[h];
+        a.ldz = a.ldw = round8(a.N);
+        a.W = m->W16[l];
+        a.Zprev = (l > 0) ? m->Z[l - 1] : nullptr;
+        a.gW = m->gW[l];
+        a.gb = m->gb[l];
+        a.dZnext = m->dZ16[h ^ 1];
+        a.dZfnext = m->dZ[h ^ 1];
+        a.ldn = round8(a.K);
+        auto tiles = [](int M, int N) { return ((M + 63) / 64) * ((N + 63) / 64); };
+        a.tilesW = tiles(a.K, a.N);
+        a.tilesB = (a.N + 31) / 32;
+        const int grid = a.tilesW + a.tilesB + (l > 0 ? tiles(rows, a.K) : 0);
+        static bool attr = false;
+        if (!attr) {
+            e = cudaFuncSetAttribute(backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBackSmem);
+            if (e != cudaSuccess)
+                return e;
+            attr = true;
         }
-    }
-    if (lossOut && e == cudaSuccess) {
-        std::vector<float> part(nb);
-        e = cudaMemcpyAsync(part.data(), m->loss, sizeof(float) * nb, cudaMemcpyDeviceToHost, m->stream);
-        if (e == cudaSuccess)
-            e = cudaStreamSynchronize(m->stream);
-        double s = 0;
-        for (float p : part)
-            s += p;
-        *lossOut = (float)(s / total);
+        backward_kernel<<<grid, 128, kBackSmem, m->stream>>>(a);
+        e = cudaGetLastError();
     }
     return e;
 }
@@ -643,7 +785,7 @@ int cl_mlp_create(int n, int width, int moment_type, double delta_ppn, unsigned 
             v = U(rng) * sc;
         ok = cudaMalloc(&m->W[l], cnt * 4) == cudaSuccess && cudaMalloc(&m->mW[l], cnt * 4) == cudaSuccess &&
              cudaMalloc(&m->vW[l], cnt * 4) == cudaSuccess && cudaMalloc(&m->gW[l], cnt * 4) == cudaSuccess &&
-             cudaMalloc(&m->W16[l], cnt * 2) == cudaSuccess &&
+             cudaMalloc(&m->W16[l], (size_t)m->dims[l] * round8(N) * 2) == cudaSuccess &&
              cudaMalloc(&m->Wt16[l], (size_t)N * round8(m->dims[l]) * 2) == cudaSuccess &&
              cudaMalloc(&m->b[l], N * 4) == cudaSuccess &&
              cudaMalloc(&m->mb[l], N * 4) == cudaSuccess && cudaMalloc(&m->vb[l], N * 4) == cudaSuccess &&
@@ -691,17 +833,12 @@ void cl_mlp_destroy(cl_mlp *m)
         cudaFree(m->gb[l]);
         cudaFree(m->W16[l]);
         cudaFree(m->Wt16[l]);
-        cudaFree(m->Act[l]);
-        cudaFree(m->Z[l]);
     }
+    mlp_free_work(m);
+    cudaFree(m->perm);
+    cudaFree(m->lossBuf);
     cudaFree(m->mean);
     cudaFree(m->stdv);
-    cudaFree(m->X);
-    cudaFree(m->dZ16);
-    cudaFree(m->T);
-    cudaFree(m->dA);
-    cudaFree(m->dZ);
-    cudaFree(m->loss);
     cudaFree(m->fallbacks);
     cudaFree(m->tcErr);
     cudaFree(m->sel);
@@ -735,14 +872,19 @@ int cl_mlp_train(cl_mlp *m, const double *d_u, const double *d_alpha, int count,
     int rc = mlp_reserve(m, batch);
     if (rc)
         return rc;
-    const int n = m->n;
-    // gather buffers for the minibatch (FP64 on device)
-    double *bu = nullptr, *ba = nullptr;
-    int *dperm = nullptr;
-    if (cudaMalloc(&bu, (size_t)batch * n * 8) != cudaSuccess || cudaMalloc(&ba, (size_t)batch * n * 8) != cudaSuccess ||
-        cudaMalloc(&dperm, (size_t)count * sizeof(int)) != cudaSuccess) {
-        cudaFree(bu);
-        cudaFree(ba);
+    const int n = m->n, np = round8(n), parts = loss_parts(m, batch);
+    auto grow = [](auto **p, size_t &cap, size_t cnt) {
+        if (cnt <= cap)
+            return true;
+        cudaFree(*p);
+        *p = nullptr;
+        cap = 0;
+        if (cudaMalloc(p, cnt * sizeof(**p)) != cudaSuccess)
+            return false;
+        cap = cnt;
+        return true;
+    };
+    if (!grow(&m->perm, m->permCap, (size_t)count) || !grow(&m->lossBuf, m->lossCap, (size_t)kLossSteps * parts)) {
         m->err = "minibatch allocation failed";
         return CL_ERR_CUDA;
     }
@@ -750,47 +892,70 @@ int cl_mlp_train(cl_mlp *m, const double *d_u, const double *d_alpha, int count,
     std::vector<int> order(count);
     for (int i = 0; i < count; i++)
         order[i] = i;
+    std::vector<float> hloss(losses ? (size_t)kLossSteps * parts : 0);
     int pos = count;
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    UpdateArgs up;
+    int first = 0, biases = 0;
+    for (int l = 0; l < kLayers; l++) {
+        up.W[l] = m->W[l];
+        up.mW[l] = m->mW[l];
+        up.vW[l] = m->vW[l];
+        up.gW[l] = m->gW[l];
+        up.b[l] = m->b[l];
+        up.mb[l] = m->mb[l];
+        up.vb[l] = m->vb[l];
+        up.gb[l] = m->gb[l];
+        up.W16[l] = m->W16[l];
+        up.Wt16[l] = m->Wt16[l];
+        up.dims[l] = m->dims[l];
+        up.first[l] = first;
+        first += ((m->dims[l] + 31) / 32) * ((m->dims[l + 1] + 31) / 32);
+        biases += m->dims[l + 1];
+    }
+    up.dims[kLayers] = m->dims[kLayers];
+    up.first[kLayers] = first;
+    up.b1 = 0.9f;
+    up.b2 = 0.999f;
+    up.eps = 1e-8f;
     cudaError_t e = cudaSuccess;
     for (int s = 0; s < steps && e == cudaSuccess; s++) {
         if (pos + batch > count) {
-            // new epoch: a fresh permutation of the training pairs
+            // new epoch: a fresh permutation of the training pairs, drawn while
+            // the device works on the steps already queued (the copy from
+            // pageable memory returns once the source has been read)
             std::shuffle(order.begin(), order.end(), rng);
-            e = cudaMemcpyAsync(dperm, order.data(), (size_t)count * sizeof(int), cudaMemcpyHostToDevice, m->stream);
-            if (e == cudaSuccess)
-                e = cudaStreamSynchronize(m->stream);
+            e = cudaMemcpyAsync(m->perm, order.data(), (size_t)count * sizeof(int), cudaMemcpyHostToDevice, m->stream);
             pos = 0;
         }
-        gather_kernel<<<blocks((size_t)batch * n), 256, 0, m->stream>>>(d_u, d_alpha, dperm + pos, batch, n, bu, ba);
+        prep_kernel<<<blocks((size_t)batch * n), 256, 0, m->stream>>>(d_u, d_alpha, m->perm + pos, batch, n, np,
+                                                                     m->momentType, m->mean, m->stdv, m->X, m->T);
         pos += batch;
-        prep_kernel<<<blocks((size_t)batch * n), 256, 0, m->stream>>>(bu, ba, batch, n, m->momentType, m->mean,
-                                                                     m->stdv, m->X, m->T);
         if (e == cudaSuccess)
             e = mlp_forward(m, batch);
-        float l = 0;
+        const int slot = s % kLossSteps;
         if (e == cudaSuccess)
-            e = mlp_backward(m, batch, losses ? &l : nullptr);
-        if (losses)
-            losses[s] = l;
+            e = mlp_backward(m, batch, m->lossBuf + (size_t)slot * parts);
         m->adamStep++;
-        float c1 = 1.0f - std::pow(b1, (float)m->adamStep), c2 = 1.0f - std::pow(b2, (float)m->adamStep);
-        for (int L = 0; L < kLayers && e == cudaSuccess; L++) {
-            size_t cnt = (size_t)m->dims[L] * m->dims[L + 1];
-            const float lrs = (s >= steps - steps / 5) ? 0.1f * lr : lr;   // step decay for the last fifth
-            adam_kernel<<<blocks(cnt), 256, 0, m->stream>>>(m->W[L], m->mW[L], m->vW[L], m->gW[L], cnt, lrs, b1, b2,
-                                                           eps, c1, c2);
-            adam_kernel<<<blocks(m->dims[L + 1]), 256, 0, m->stream>>>(m->b[L], m->mb[L], m->vb[L], m->gb[L],
-                                                                      m->dims[L + 1], lrs, b1, b2, eps, c1, c2);
+        up.c1 = 1.0f - std::pow(up.b1, (float)m->adamStep);
+        up.c2 = 1.0f - std::pow(up.b2, (float)m->adamStep);
+        up.lr = (s >= steps - steps / 5) ? 0.1f * lr : lr;   // step decay for the last fifth
+        if (e == cudaSuccess) {
+            update_kernel<<<first + (biases + 255) / 256, 256, 0, m->stream>>>(up);
+            e = cudaGetLastError();
         }
-        if (e == cudaSuccess)
-            e = mlp_sync_weights(m);
+        // the loss comes back every kLossSteps steps, not every step
+        if (losses && e == cudaSuccess && (slot == kLossSteps - 1 || s == steps - 1)) {
+            e = cudaMemcpyAsync(hloss.data(), m->lossBuf, (size_t)(slot + 1) * parts * sizeof(float),
+                                cudaMemcpyDeviceToHost, m->stream);
+            if (e == cudaSuccess)
+                e = cudaStreamSynchronize(m->stream);
+            for (int k = 0; k <= slot && e == cudaSuccess; k++)
+                losses[s - slot + k] = loss_value(&hloss[(size_t)k * parts], parts, batch * n);
+        }
     }
+    const cudaError_t es = cudaStreamSynchronize(m->stream);
     if (e == cudaSuccess)
-        e = cudaStreamSynchronize(m->stream);
-    cudaFree(bu);
-    cudaFree(ba);
-    cudaFree(dperm);
+        e = es;
     if (e != cudaSuccess) {
         m->err = std::string("training: ") + cudaGetErrorString(e);
         return CL_ERR_CUDA;
@@ -819,8 +984,9 @@ int cl_mlp_predict(cl_mlp *m, const double *d_u, double *d_alpha, int count, int
     cudaError_t e = cudaMemsetAsync(m->fallbacks, 0, sizeof(int), st);
     for (int c0 = 0; c0 < count && e == cudaSuccess; c0 += chunk) {
         int rows = count - c0 < chunk ? count - c0 : chunk;
-        prep_kernel<<<blocks((size_t)rows * m->n), 256, 0, st>>>(d_u + (size_t)c0 * m->n, nullptr, rows, m->n,
-                                                                m->momentType, m->mean, m->stdv, m->X, nullptr);
+        prep_kernel<<<blocks((size_t)rows * m->n), 256, 0, st>>>(d_u + (size_t)c0 * m->n, nullptr, nullptr, rows, m->n,
+                                                                round8(m->n), m->momentType, m->mean, m->stdv, m->X,
+                                                                nullptr);
         m->keepZ = false;
         e = mlp_forward(m, rows);
         m->keepZ = true;
@@ -879,7 +1045,8 @@ int cl_mlp_predict_selected(cl_mlp *m, const double *d_u, const int *d_iters, in
     select_kernel<<<blocks(count), 256, 0, st>>>(d_iters, count, min_iters, m->sel, cnt, d_alpha, m->n);
     for (int c0 = 0; c0 < count && e == cudaSuccess; c0 += chunk) {
         const int rows = count - c0 < chunk ? count - c0 : chunk;
-        prep_idx_kernel<<<blocks((size_t)rows * m->n), 256, 0, st>>>(d_u, m->sel, cnt, c0, rows, m->n, m->X);
+        prep_idx_kernel<<<blocks((size_t)rows * m->n), 256, 0, st>>>(d_u, m->sel, cnt, c0, rows, m->n, round8(m->n),
+                                                                    m->X);
         m->keepZ = false;
         e = mlp_forward(m, rows, cnt, c0);
         m->keepZ = true;
@@ -909,7 +1076,7 @@ int cl_tc_gemm_bf16(const void *d_A, const void *d_B, int M, int N, int K, float
         return CL_ERR_CUDA;
     cudaMemset(err, 0, sizeof(int));
     cudaError_t e = tc_gemm<clb::tc::EPI_STORE>((const __nv_bfloat16 *)d_A, (const __nv_bfloat16 *)d_B, M, N, K, d_C,
-                                                 nullptr, nullptr, nullptr, 0, err, nullptr);
+                                                 nullptr, nullptr, 0, nullptr, 0, err, nullptr);
     if (e == cudaSuccess)
         e = cudaDeviceSynchronize();
     int h = 0;
@@ -937,11 +1104,18 @@ int cl_mlp_loss_and_grads(cl_mlp *m, const double *u, const double *alpha, int r
     cudaMalloc(&ba, (size_t)rows * n * 8);
     cudaMemcpy(bu, u, (size_t)rows * n * 8, cudaMemcpyHostToDevice);
     cudaMemcpy(ba, alpha, (size_t)rows * n * 8, cudaMemcpyHostToDevice);
-    prep_kernel<<<blocks((size_t)rows * n), 256, 0, m->stream>>>(bu, ba, rows, n, m->momentType, m->mean, m->stdv,
-                                                                m->X, m->T);
+    prep_kernel<<<blocks((size_t)rows * n), 256, 0, m->stream>>>(bu, ba, nullptr, rows, n, round8(n), m->momentType,
+                                                                m->mean, m->stdv, m->X, m->T);
     cudaError_t e = mlp_forward(m, rows);
     if (e == cudaSuccess)
-        e = mlp_backward(m, rows, loss);
+        e = mlp_backward(m, rows, m->loss);
+    std::vector<float> part(loss_parts(m, rows));
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(part.data(), m->loss, sizeof(float) * part.size(), cudaMemcpyDeviceToHost, m->stream);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(m->stream);
+    if (loss && e == cudaSuccess)
+        *loss = loss_value(part.data(), (int)part.size(), rows * n);
     for (int l = 0; l < kLayers && e == cudaSuccess; l++) {
         size_t cnt = (size_t)m->dims[l] * m->dims[l + 1];
         if (gW && gW[l])

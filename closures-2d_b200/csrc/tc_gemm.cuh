@@ -95,7 +95,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
-// Z (nullable) [M x N] FP32 = A B^T (+ bias); Act (nullable) [M x N] BF16 =
+// Z (nullable) [M x N] FP32 = A B^T (+ bias); Act (nullable) [M x ldAct] BF16 =
 // GELU(Z) (EPI_BIAS_GELU) or Z; with Mdev, M = min(M, *Mdev - moff).
 // Persistent (one CTA per SM, tiles taken in turn), six warps:
 //   warp 0 (one lane)  TMA producer over the tiles' k-blocks, kPStages deep;
@@ -111,7 +111,7 @@ constexpr int smem_bytes_persistent(int bn) { return kPStages * (BM * BK * 2 + b
 
 template <int BN, int EPI>
 __device__ __forceinline__ void epilogue_rows(uint32_t tl, int row, int M, int N, int n0, float *Z,
-                                              const float *bias, __nv_bfloat16 *Act)
+                                              const float *bias, __nv_bfloat16 *Act, int ldAct)
 {
 #pragma unroll 1
     for (int c0 = 0; c0 < BN; c0 += 16) {
@@ -141,7 +141,7 @@ __device__ __forceinline__ void epilogue_rows(uint32_t tl, int row, int M, int N
 #pragma unroll
                 for (int j = 0; j < 16; j++)
                     b[j] = __float2bfloat16(EPI == EPI_BIAS_GELU ? gelu_f(v[j]) : v[j]);
-                uint4 *a = reinterpret_cast<uint4 *>(Act + (size_t)row * N + col0);
+                uint4 *a = reinterpret_cast<uint4 *>(Act + (size_t)row * ldAct + col0);
                 a[0] = reinterpret_cast<const uint4 *>(b)[0];
                 a[1] = reinterpret_cast<const uint4 *>(b)[1];
             }
@@ -153,7 +153,7 @@ __device__ __forceinline__ void epilogue_rows(uint32_t tl, int row, int M, int N
                     if (Z)
                         Z[(size_t)row * N + col] = v[j];
                     if (Act)
-                        Act[(size_t)row * N + col] = __float2bfloat16(EPI == EPI_BIAS_GELU ? gelu_f(v[j]) : v[j]);
+                        Act[(size_t)row * ldAct + col] = __float2bfloat16(EPI == EPI_BIAS_GELU ? gelu_f(v[j]) : v[j]);
                 }
             }
         }
@@ -163,8 +163,8 @@ __device__ __forceinline__ void epilogue_rows(uint32_t tl, int row, int M, int N
 template <int BN, int EPI>
 __global__ void __launch_bounds__(192, 1)
     tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                              int M, int N, int K, float *Z, const float *bias, __nv_bfloat16 *Act, const int *Mdev,
-                              int moff, int *err)
+                              int M, int N, int K, float *Z, const float *bias, __nv_bfloat16 *Act, int ldAct,
+                              const int *Mdev, int moff, int *err)
 {
     static_assert(BN == 32 || BN == 64 || BN == 128, "two accumulators of BN columns (power of two)");
     constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE = A_BYTES + B_BYTES;
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(192, 1)
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const int m0 = (t / tilesN) * BM, n0 = (t % tilesN) * BN;
             const uint32_t tl = tmem + (uint32_t)(b * BN) + ((uint32_t)(quarter * 32) << 16);
-            epilogue_rows<BN, EPI>(tl, m0 + quarter * 32 + lane, M, N, n0, Z, bias, Act);
+            epilogue_rows<BN, EPI>(tl, m0 + quarter * 32 + lane, M, N, n0, Z, bias, Act, ldAct);
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
             if (lane == 0)
