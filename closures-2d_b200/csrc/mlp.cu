@@ -59,19 +59,17 @@ __device__ __forceinline__ void cp16_zfill(void *smem, const void *gmem, bool va
     const int bytes = valid ? 16 : 0;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void ldmatrix4(unsigned (&r)[4], const void *p)
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix4(unsigned (&r)[4], unsigned addr)
 {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(s));
-}
-__device__ __forceinline__ void ldmatrix4_t(unsigned (&r)[4], const void *p)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(s));
+    if (TRANS)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(addr));
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(addr));
 }
 
 // One layer of the backward pass in one launch.  Its three products need
@@ -104,7 +102,120 @@ constexpr int kBackStages = 4, kBackK = 64;
 constexpr int kBackTile = 64 * (kBackK + 8);   // bf16 of one staged operand (rows padded by 16 bytes)
 constexpr int kBackSmem = kBackStages * 2 * kBackTile * 2;
 
-__global__ void __launch_bounds__(128) backward_kernel(const BackArgs a)
+// One 64 x 64 tile, eight warps of 32 x 16.  C [M x N] = A . B over kTot: dW
+// (W): A = in^T, B = dZ, both staged as [k][64]; dA: A = dZ, B = W^T, staged as
+// [64][k].  The chains are latency bound, so what a warp issues per stage
+// counts (addresses are fixed before the loop and advance by one stride), and
+// eight warps hide more than four did (a layer's launch 54 us with addresses
+// formed per piece, 35 us with fixed ones, four warps each).
+template <bool W>
+__device__ __forceinline__ void backward_tile(const BackArgs &a, int block, unsigned char *smraw)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int M = W ? a.K : a.rows, N = W ? a.N : a.K, kTot = W ? a.rows : a.ldw;
+    const int tn = (N + 63) / 64;
+    const int m0 = (block / tn) * 64, n0 = (block % tn) * 64;
+    const __nv_bfloat16 *A = W ? a.in : a.dZ, *B = W ? a.dZ : a.W;
+    const int lda = W ? a.ldin : a.ldz, ldb = W ? a.ldz : a.ldw;
+    constexpr int LD = kBackK + 8;   // also 64 + 8 for the [k][64] form
+    __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(smraw), *sB = sA + kBackStages * kBackTile;
+    const int nst = (kTot + kBackK - 1) / kBackK;
+    // this thread's two 16-byte pieces of each operand: rows lr + 32 q
+    const int lr = tid >> 3, lc = (tid & 7) * 8;
+    const __nv_bfloat16 *pA = W ? A + (size_t)lr * lda + m0 + lc : A + (size_t)(m0 + lr) * lda + lc;
+    const __nv_bfloat16 *pB = W ? B + (size_t)lr * ldb + n0 + lc : B + (size_t)(n0 + lr) * ldb + lc;
+    const size_t stepA = W ? (size_t)kBackK * lda : kBackK, stepB = W ? (size_t)kBackK * ldb : kBackK;
+    const size_t rowA = (size_t)32 * lda, rowB = (size_t)32 * ldb;
+    bool inA[2], inB[2];   // the bounds that do not depend on the stage
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        inA[q] = W ? m0 + lc < lda : m0 + lr + 32 * q < M;
+        inB[q] = W ? n0 + lc < ldb : n0 + lr + 32 * q < N;
+    }
+    int kLeft = kTot - (W ? lr : lc);   // k of this thread's first piece still inside
+    const unsigned dstA = (unsigned)__cvta_generic_to_shared(sA + lr * LD + lc);
+    const unsigned dstB = (unsigned)__cvta_generic_to_shared(sB + lr * LD + lc);
+    auto cp = [](unsigned dst, const void *src, bool ok) {
+        const int bytes = ok ? 16 : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+    };
+    auto load = [&](int buf) {   // the next stage into buffer buf
+        const unsigned off = (unsigned)(buf * kBackTile * 2);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const bool okK = W ? kLeft > 32 * q : kLeft > 0;
+            const bool okA = okK && inA[q], okB = okK && inB[q];
+            cp(dstA + off + q * 32 * LD * 2, okA ? pA + q * rowA : A, okA);
+            cp(dstB + off + q * 32 * LD * 2, okB ? pB + q * rowB : B, okB);
+        }
+        pA += stepA;
+        pB += stepB;
+        kLeft -= kBackK;
+    };
+    const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
+    // fragment addresses: W: blocks (k, m) and (k, n) of [k][64] transposed;
+    // else blocks of [m][k] and [n][k]
+    const int l7 = lane & 7, l8 = (lane >> 3) & 1, l16 = lane >> 4;
+    const unsigned fragA = (unsigned)__cvta_generic_to_shared(
+        W ? sA + (l7 + l16 * 8) * LD + wm + l8 * 8 : sA + (wm + l7 + l8 * 8) * LD + l16 * 8);
+    const unsigned fragB = (unsigned)__cvta_generic_to_shared(
+        W ? sB + (l7 + l8 * 8) * LD + wn + l16 * 8 : sB + (wn + l7 + l16 * 8) * LD + l8 * 8);
+    float acc[2][2][4];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0f;
+    for (int st = 0; st < kBackStages - 1; st++) {
+        if (st < nst)
+            load(st);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    int buf = 0;
+    for (int st = 0; st < nst; st++) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kBackStages - 2) : "memory");
+        __syncthreads();
+        if (st + kBackStages - 1 < nst)
+            load((buf + kBackStages - 1) % kBackStages);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const unsigned ta = fragA + buf * kBackTile * 2, tb = fragB + buf * kBackTile * 2;
+#pragma unroll
+        for (int kk = 0; kk < kBackK; kk += 16) {
+            unsigned fa[2][4], fb[4];
+            ldmatrix4<W>(fb, tb + (W ? kk * LD : kk) * 2);
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                ldmatrix4<W>(fa[i], ta + (W ? kk * LD + i * 16 : i * 16 * LD + kk) * 2);
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+                    mma_bf16(acc[i][j], fa[i][0], fa[i][1], fa[i][2], fa[i][3], fb[2 * j], fb[2 * j + 1]);
+        }
+        buf = (buf + 1) % kBackStages;
+    }
+    const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int h = 0; h < 4; h++) {
+                const int m = m0 + wm + i * 16 + g + ((h & 2) ? 8 : 0);
+                const int nn = n0 + wn + j * 8 + 2 * t + (h & 1);
+                if (m >= M || nn >= N)
+                    continue;
+                if (W) {
+                    a.gW[(size_t)m * N + nn] = acc[i][j][h];
+                } else {
+                    const float v = acc[i][j][h] * gelu_grad(a.Zprev[(size_t)m * N + nn]);
+                    a.dZnext[(size_t)m * a.ldn + nn] = __float2bfloat16(v);
+                    a.dZfnext[(size_t)m * a.ldn + nn] = v;
+                }
+            }
+}
+
+__global__ void __launch_bounds__(256) backward_kernel(const BackArgs a)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -117,7 +228,7 @@ __global__ void __launch_bounds__(128) backward_kernel(const BackArgs a)
         const int nst = (a.rows + R - 1) / R;
         auto load = [&](int st) {
             float *d = buf + (st % S) * (R * 32);
-            for (int i = tid; i < R * 8; i += 128) {
+            for (int i = tid; i < R * 8; i += 256) {
                 const int r = st * R + i / 8, c = j0 + (i % 8) * 4;
                 const bool ok = r < a.rows && c < a.ldz;
                 cp16_zfill(d + (i / 8) * 32 + (i % 8) * 4, a.dZf + (ok ? (size_t)r * a.ldz + c : 0), ok);
@@ -139,9 +250,22 @@ __global__ void __launch_bounds__(128) backward_kernel(const BackArgs a)
                 const float *d = buf + (st % S) * (R * 32) + lane;
                 const int cnt = min(R, a.rows - st * R);
                 if (cnt == R) {
+                    // loads well ahead of the chain of additions
+                    float x[2][16];
 #pragma unroll
-                    for (int r = 0; r < R; r++)
-                        s += d[r * 32];
+                    for (int q = 0; q < 16; q++)
+                        x[0][q] = d[q * 32];
+#pragma unroll
+                    for (int r = 0; r < R; r += 16) {
+                        if (r + 16 < R) {
+#pragma unroll
+                            for (int q = 0; q < 16; q++)
+                                x[(r / 16 + 1) & 1][q] = d[(r + 16 + q) * 32];
+                        }
+#pragma unroll
+                        for (int q = 0; q < 16; q++)
+                            s += x[(r / 16) & 1][q];
+                    }
                 } else {
                     for (int r = 0; r < cnt; r++)
                         s += d[r * 32];
@@ -152,104 +276,10 @@ __global__ void __launch_bounds__(128) backward_kernel(const BackArgs a)
             a.gb[j0 + lane] = s;
         return;
     }
-    const bool isW = block < a.tilesW;
-    if (!isW)
-        block -= a.tilesW + a.tilesB;
-    // C [M x N] = A . B over kTot: dW: A = in^T, B = dZ, both staged as [k][64];
-    // dA: A = dZ, B = W^T, staged as [64][k]
-    const int M = isW ? a.K : a.rows, N = isW ? a.N : a.K, kTot = isW ? a.rows : a.ldw;
-    const int tn = (N + 63) / 64;
-    const int m0 = (block / tn) * 64, n0 = (block % tn) * 64;
-    const __nv_bfloat16 *A = isW ? a.in : a.dZ, *B = isW ? a.dZ : a.W;
-    const int lda = isW ? a.ldin : a.ldz, ldb = isW ? a.ldz : a.ldw;
-    __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(smraw), *sB = sA + kBackStages * kBackTile;
-    constexpr int LD = kBackK + 8;   // also 64 + 8 for the [k][64] form
-    const int nst = (kTot + kBackK - 1) / kBackK;
-    auto load = [&](int st) {
-        __nv_bfloat16 *da = sA + (st % kBackStages) * kBackTile, *db = sB + (st % kBackStages) * kBackTile;
-        const int k0 = st * kBackK;
-        for (int i = tid; i < 64 * 8; i += 128) {
-            const int r = i / 8, c = (i % 8) * 8;
-            if (isW) {
-                const bool okA = k0 + r < kTot && m0 + c < lda, okB = k0 + r < kTot && n0 + c < ldb;
-                cp16_zfill(da + r * LD + c, A + (okA ? (size_t)(k0 + r) * lda + m0 + c : 0), okA);
-                cp16_zfill(db + r * LD + c, B + (okB ? (size_t)(k0 + r) * ldb + n0 + c : 0), okB);
-            } else {
-                const bool okA = m0 + r < M && k0 + c < lda, okB = n0 + r < N && k0 + c < ldb;
-                cp16_zfill(da + r * LD + c, A + (okA ? (size_t)(m0 + r) * lda + k0 + c : 0), okA);
-                cp16_zfill(db + r * LD + c, B + (okB ? (size_t)(n0 + r) * ldb + k0 + c : 0), okB);
-            }
-        }
-    };
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-    float acc[2][4][4];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0f;
-    for (int st = 0; st < kBackStages - 1; st++) {
-        if (st < nst)
-            load(st);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-    for (int st = 0; st < nst; st++) {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(kBackStages - 2) : "memory");
-        __syncthreads();
-        if (st + kBackStages - 1 < nst)
-            load(st + kBackStages - 1);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        const __nv_bfloat16 *ta = sA + (st % kBackStages) * kBackTile, *tb = sB + (st % kBackStages) * kBackTile;
-#pragma unroll
-        for (int kk = 0; kk < kBackK; kk += 16) {
-            unsigned fa[2][4], fb[2][4];
-            if (isW) {
-                // [k][m]: 8x8 blocks (k, m) transposed; block order m, m + 8, then k + 8
-#pragma unroll
-                for (int i = 0; i < 2; i++)
-                    ldmatrix4_t(fa[i], ta + (kk + (lane & 7) + ((lane >> 4) & 1) * 8) * LD + wm + i * 16 +
-                                           ((lane >> 3) & 1) * 8);
-#pragma unroll
-                for (int j = 0; j < 2; j++)
-                    ldmatrix4_t(fb[j], tb + (kk + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + wn + j * 16 +
-                                           ((lane >> 4) & 1) * 8);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 2; i++)
-                    ldmatrix4(fa[i], ta + (wm + i * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + kk +
-                                         ((lane >> 4) & 1) * 8);
-#pragma unroll
-                for (int j = 0; j < 2; j++)
-                    ldmatrix4(fb[j], tb + (wn + j * 16 + (lane & 7) + ((lane >> 4) & 1) * 8) * LD + kk +
-                                         ((lane >> 3) & 1) * 8);
-            }
-#pragma unroll
-            for (int i = 0; i < 2; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    mma_bf16(acc[i][j], fa[i][0], fa[i][1], fa[i][2], fa[i][3], fb[j >> 1][(j & 1) * 2],
-                             fb[j >> 1][(j & 1) * 2 + 1]);
-        }
-    }
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const int m = m0 + wm + i * 16 + g + ((h & 2) ? 8 : 0);
-                const int nn = n0 + wn + j * 8 + 2 * t + (h & 1);
-                if (m >= M || nn >= N)
-                    continue;
-                if (isW) {
-                    a.gW[(size_t)m * N + nn] = acc[i][j][h];
-                } else {
-                    const float v = acc[i][j][h] * gelu_grad(a.Zprev[(size_t)m * N + nn]);
-                    a.dZnext[(size_t)m * a.ldn + nn] = __float2bfloat16(v);
-                    a.dZfnext[(size_t)m * a.ldn + nn] = v;
-                }
-            }
+    if (block < a.tilesW)
+        backward_tile<true>(a, block, smraw);
+    else
+        backward_tile<false>(a, block - a.tilesW - a.tilesB, smraw);
 }
 
 // W [K x N] FP32 -> W16 [K x ldw] BF16, zero columns N..ldw-1
@@ -732,7 +762,7 @@ static cudaError_t mlp_backward(cl_mlp *m, int rows, float *loss)
                 return e;
             attr = true;
         }
-        backward_kernel<<<grid, 128, kBackSmem, m->stream>>>(a);
+        backward_kernel<<<grid, 256, kBackSmem, m->stream>>>(a);
         e = cudaGetLastError();
     }
     return e;
