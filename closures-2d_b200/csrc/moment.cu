@@ -2,8 +2,9 @@
 // the device: the state of one grid, the RK2 step of MomentSolver::update
 // (moment_update.cpp:169-247) and the halo of a partitioned grid.
 //
-// One kernel per RK stage (pn_tile_kernel on the FP64 tensor cores up to
-// order 6, pn_stage_kernel above): for each interior cell it applies the moment
+// One kernel per RK stage (pn_parity_kernel; for operators without the
+// harmonics' parity structure pn_tile_kernel on the FP64 tensor cores up to 32
+// moments, pn_stage_kernel above): for each interior cell it applies the moment
 // filter to the stencil values as it loads them (moment_update.cpp:23-40
 // scales the interior in place before the ghost copy, so ghost strips that
 // hold interior copies are filtered too and the physical boundary's are not),
@@ -48,6 +49,8 @@ struct PnArgs {
     int filteredGhosts;     // bit s: ghost strip of side s holds (filtered) interior values
     double dt, rdx, rdy, dx, dy, initX, initY;
     int rowBegin, rowEnd;   // interior rows (x) of this launch; band starts are multiples of kTI
+    int wrap;               // pn_parity_kernel: 1 reads ghost cells from the interior cells they
+                            // copy (periodic grid), 2 also writes the copies to `in`
 };
 
 __device__ __forceinline__ bool filtered_cell(const PnArgs &a, int i, int j)
@@ -303,6 +306,302 @@ __global__ void __launch_bounds__(kTI * 32, 2) pn_tile_kernel(PnArgs a)
     }
 }
 
+// The operators' structure.  For each direction E = Op+ t+ + Op- t- =
+// D (t+ - t-) + S (t+ + t-) with D = (Op+ - Op-) / 2, S = (Op+ + Op-) / 2.  On
+// the quadrature's basis of z-even real harmonics D = <|xi| m m^T> / 2 joins
+// only moments of equal parity under both reflections x -> -x and y -> -y, and
+// S = <xi m m^T> / 2 only those that the recursion of xi times a harmonic
+// reaches (degree and |m| each one apart, the parity of xi flipped; likewise
+// eta): at order 6 560 of the 3136 products remain.  What is left out is the
+// rounding of the set-up's sums (1.6e-15 of the largest entry at most for
+// orders 1-9).
+template <int N>
+struct PnShape {
+    static constexpr int n = (N + 1) * (N + 2) / 2;
+    int deg[n] = {}, m[n] = {}, cls[n] = {};       // class: 2 (odd in x) + (odd in y)
+    int size[4] = {}, member[4][n] = {}, offA[4] = {};
+    int countA = 0, countB[2] = {}, offD[2] = {}, offS[2] = {}, coefs = 0;   // entries and where they start
+    short b[2][n][n] = {};                         // index of S entry (k, i) per direction, -1: none
+    constexpr PnShape()
+    {
+        int k = 0;
+        for (int l = 0; l <= N; l++)
+            for (int mm = -l; mm <= l; mm += 2) {
+                const int am = mm < 0 ? -mm : mm;
+                deg[k] = l;
+                m[k] = am;
+                cls[k] = 2 * (mm >= 0 ? am % 2 : 1 - am % 2) + (mm < 0 ? 1 : 0);
+                k++;
+            }
+        for (int i = 0; i < n; i++)
+            member[cls[i]][size[cls[i]]++] = i;
+        for (int c = 0; c < 4; c++) {
+            offA[c] = countA;
+            countA += size[c] * size[c];
+        }
+        for (int d = 0; d < 2; d++)
+            for (int i = 0; i < n; i++)
+                for (int kk = 0; kk < n; kk++) {
+                    const int dl = deg[kk] - deg[i], dm = m[kk] - m[i];
+                    const bool on = cls[kk] == (cls[i] ^ (d == 0 ? 2 : 1)) && (dl == 1 || dl == -1) && (dm == 1 || dm == -1);
+                    b[d][kk][i] = on ? (short)countB[d]++ : (short)-1;
+                }
+        offD[1] = countA;
+        offS[0] = 2 * countA;
+        offS[1] = 2 * countA + countB[0];
+        coefs = offS[1] + countB[1];
+    }
+};
+template <int N>
+struct PnTable {
+    static constexpr PnShape<N> s{};   // (device code uses it in constant expressions only)
+};
+
+// Nonzero entries of D and S over dx or dy, in the shape's order.
+template <int N>
+struct PnCoef {
+    double c[PnTable<N>::s.coefs];
+};
+
+template <int V>
+struct Int {
+    static constexpr int value = V;
+};
+// f(Int<B>()), ..., f(Int<E - 1>()): a loop whose index is a constant.
+template <int B, int E, class F>
+__device__ __forceinline__ void static_for(F &&f)
+{
+    if constexpr (B < E) {
+        f(Int<B>());
+        static_for<B + 1, E>(f);
+    }
+}
+
+// The stage on that structure.  A CTA stages a tile of kTI x kTJ cells with its
+// halo (no corners) in shared memory, filtered on load; a thread owns a cell,
+// forms t+ - t- and t+ + t- of one parity class at a time and adds their
+// products, coefficients from the constant bank, into the cell's flux in
+// registers.  The new moments go through the tile so that the state, read once
+// and written once, moves in whole lines.  Cells are padded to an odd
+// stride: conflict-free for a thread per cell.
+constexpr int kParThreads = kTI * kTJ;
+template <int N>
+__global__ void __launch_bounds__(kParThreads) pn_parity_kernel(const PnArgs a, const __grid_constant__ PnCoef<N> q)
+{
+    using T = PnTable<N>;
+    constexpr int n = PnShape<N>::n, CS = n | 1, RW = kTJ + 4;
+    extern __shared__ double sm[];
+    double *tile = sm;                           // [kTI+4][RW][CS]
+    double *sFilter = sm + (kTI + 4) * RW * CS;  // [n]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ny = a.NY - 4, tilesJ = (ny + kTJ - 1) / kTJ;
+    const int i0 = 2 + a.rowBegin + (blockIdx.x / tilesJ) * kTI, j0 = 2 + (blockIdx.x % tilesJ) * kTJ;
+    if (a.filter)
+        for (int k = tid; k < n; k += kParThreads)
+            sFilter[k] = a.filter[k];
+    // every cell of the tile and its halo interior: one rule for all of them
+    const bool inner = i0 >= 4 && j0 >= 4 && i0 + kTI + 2 <= a.NX - 2 && j0 + kTJ + 2 <= a.NY - 2;
+    constexpr int V = (n % 2 == 0) ? 2 : 1;      // doubles per load (rows of even n start 16-byte aligned)
+    if (a.filter)
+        __syncthreads();
+    for (int r = warp; r < kTI + 4; r += kParThreads / 32) {
+        const bool full = r >= 2 && r < kTI + 2;
+        const int c0 = full ? 0 : 2, cells = full ? RW : kTJ, gi = i0 - 2 + r;
+        constexpr int kBatch = 8;
+        for (int e0 = lane * V; e0 < cells * n; e0 += kBatch * 32 * V) {
+            double v[kBatch][V];
+#pragma unroll
+            for (int b = 0; b < kBatch; b++) {
+                const int e = e0 + b * 32 * V, gj = j0 - 2 + c0 + e / n;
+                int si = gi, sj = gj;
+                if (!inner && a.wrap) {
+                    // the interior cell a ghost copies (momopt_boundaries.cpp:190-223)
+                    const bool inI = gi >= 2 && gi < a.NX - 2, inJ = gj >= 2 && gj < a.NY - 2;
+                    if (inJ && !inI)
+                        si = gi < 2 ? gi + a.NX - 4 : gi - (a.NX - 4);
+                    if (inI && !inJ)
+                        sj = gj < 2 ? gj + a.NY - 4 : gj - (a.NY - 4);
+                }
+                const bool ok = e < cells * n && (inner || (gi < a.NX && gj < a.NY));
+                const double *src = a.in + ((size_t)si * a.NY + sj) * n + e % n;
+                if constexpr (V == 2) {
+                    const double2 x = ok ? *reinterpret_cast<const double2 *>(src) : make_double2(0.0, 0.0);
+                    v[b][0] = x.x;
+                    v[b][1] = x.y;
+                } else {
+                    v[b][0] = ok ? *src : 0.0;
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < kBatch; b++) {
+                const int e = e0 + b * 32 * V;
+                if (e >= cells * n)
+                    continue;
+                const int c = c0 + e / n, k = e % n, gj = j0 - 2 + c;
+                const bool inI = gi >= 2 && gi < a.NX - 2, inJ = gj >= 2 && gj < a.NY - 2;
+                if (a.wrap == 2 && inI != inJ && gi < a.NX && gj < a.NY) {
+                    double *dst = const_cast<double *>(a.in) + ((size_t)gi * a.NY + gj) * n + k;
+#pragma unroll
+                    for (int h = 0; h < V; h++)
+                        dst[h] = v[b][h];
+                }
+                const bool filt = a.filter && (inner || filtered_cell(a, gi, gj));
+                double *t = tile + (r * RW + c) * CS + k;
+#pragma unroll
+                for (int h = 0; h < V; h++)
+                    t[h] = filt ? __dmul_rn(v[b][h], sFilter[k + h]) : v[b][h];
+            }
+        }
+    }
+    __syncthreads();
+    const int ii = tid / kTJ, jj = tid % kTJ, i = i0 + ii, j = j0 + jj;
+    double *self = tile + ((ii + 2) * RW + jj + 2) * CS;
+    double F[n];
+#pragma unroll
+    for (int k = 0; k < n; k++)
+        F[k] = 0.0;
+    static_for<0, 2>([&](auto dc) {
+        constexpr int d = decltype(dc)::value;
+        constexpr int step = (d == 0) ? RW * CS : CS;
+        static_for<0, 4>([&](auto cc) {
+            constexpr int c = decltype(cc)::value, c2 = c ^ (d == 0 ? 2 : 1);
+            constexpr int sz = T::s.size[c], sz2 = T::s.size[c2];
+            double df[sz > 0 ? sz : 1], su[sz > 0 ? sz : 1];
+            static_for<0, sz>([&](auto pc) {
+                constexpr int p = decltype(pc)::value, k = T::s.member[c][p];
+                // t+ = (x1 + 3 x0 - 5 x-1 + x-2) / 4, t- = (-x2 + 5 x1 - 3 x0 - x-1) / 4
+                // (moment_update.cpp:95-143)
+                const double m2 = self[k - 2 * step], m1 = self[k - step], p1 = self[k + step], p2 = self[k + 2 * step];
+                df[p] = fma(1.5, self[k], fma(0.25, m2 + p2, -(m1 + p1)));
+                su[p] = fma(1.5, p1 - m1, 0.25 * (m2 - p2));
+            });
+            static_for<0, sz>([&](auto rc) {
+                constexpr int r = decltype(rc)::value, k = T::s.member[c][r];
+                static_for<0, sz>([&](auto pc) {
+                    constexpr int p = decltype(pc)::value;
+                    constexpr int e = T::s.offD[d] + T::s.offA[c] + r * sz + p;
+                    F[k] = fma(q.c[e], df[p], F[k]);
+                });
+            });
+            static_for<0, sz>([&](auto pc) {
+                constexpr int p = decltype(pc)::value, from = T::s.member[c][p];
+                static_for<0, sz2>([&](auto rc) {
+                    constexpr int k = T::s.member[c2][decltype(rc)::value];
+                    constexpr int e = T::s.b[d][k][from], off = T::s.offS[d];
+                    if constexpr (e >= 0)
+                        F[k] = fma(q.c[off + e], su[p], F[k]);
+                });
+            });
+        });
+    });
+    const bool mine = i < 2 + a.rowEnd && j < a.NY - 2;
+    if (mine) {
+        const size_t cell = (size_t)i * a.NY + j;
+        const double sT = a.sigT[cell], sS = a.sigS[cell], dt = a.dt;
+        const double gk = __dsub_rn(1.0, __dmul_rn(dt, sT));
+        const double g0 = __dsub_rn(__dadd_rn(1.0, __dmul_rn(dt, sS)), __dmul_rn(dt, sT));
+#pragma unroll
+        for (int k = 0; k < n; k++)   // moment_update.cpp:186-187 / :214-215
+            F[k] = __dsub_rn(__dmul_rn(self[k], k == 0 ? g0 : gk), __dmul_rn(dt, F[k]));
+        if (a.initCond == 1) {
+            const double x = __dadd_rn(a.initX, __dmul_rn((double)(i - 2), a.dx));
+            const double y = __dadd_rn(a.initY, __dmul_rn((double)(j - 2), a.dy));
+            if (fabs(x) < 0.5 && fabs(y) < 0.5)
+                F[0] = __dadd_rn(F[0], __dmul_rn(__dmul_rn(dt, 2.0), kSqrtPiPn));
+        }
+    }
+    __syncthreads();   // every stencil has read the tile
+#pragma unroll
+    for (int k = 0; k < n; k++)
+        self[k] = F[k];
+    __syncthreads();
+    const int cols = min(kTJ, a.NY - 2 - j0);
+    for (int r = warp; r < kTI; r += kParThreads / 32) {
+        if (i0 + r >= 2 + a.rowEnd)
+            break;
+        const size_t base = ((size_t)(i0 + r) * a.NY + j0) * n;
+        const double *row = tile + ((r + 2) * RW + 2) * CS;
+        for (int e = lane * V; e < cols * n; e += 32 * V) {
+            const double *t = row + (e / n) * CS + e % n;
+            if constexpr (V == 2) {
+                double2 u = make_double2(t[0], t[1]);
+                if (a.old) {   // moment_update.cpp:237-246
+                    const double2 o = *reinterpret_cast<const double2 *>(a.old + base + e);
+                    u.x = __dmul_rn(0.5, __dadd_rn(u.x, o.x));
+                    u.y = __dmul_rn(0.5, __dadd_rn(u.y, o.y));
+                }
+                *reinterpret_cast<double2 *>(a.out + base + e) = u;
+            } else {
+                double u = t[0];
+                if (a.old)
+                    u = __dmul_rn(0.5, __dadd_rn(u, a.old[base + e]));
+                a.out[base + e] = u;
+            }
+        }
+    }
+}
+
+template <int N>
+constexpr size_t pn_parity_smem()
+{
+    constexpr int n = PnShape<N>::n;
+    return (size_t)((kTI + 4) * (kTJ + 4) * (n | 1) + n) * sizeof(double);
+}
+
+// The coefficients of ops [4][n][n] (row i column j of c_pnFluxOperator*, xi
+// plus, xi minus, eta plus, eta minus) in the shape's order; false when an
+// entry outside the structure is more than rounding.
+template <int N>
+bool pn_parity_coefs(const double *ops, std::vector<double> &out)
+{
+    constexpr auto &S = PnTable<N>::s;
+    constexpr int n = PnShape<N>::n;
+    double top = 0.0;
+    for (int e = 0; e < 4 * n * n; e++) {
+        if (!std::isfinite(ops[e]))
+            return false;
+        top = std::max(top, std::fabs(ops[e]));
+    }
+    out.assign(S.coefs, 0.0);
+    for (int d = 0; d < 2; d++)
+        for (int k = 0; k < n; k++)
+            for (int i = 0; i < n; i++) {
+                const double p = ops[(2 * d * n + k) * n + i], m = ops[((2 * d + 1) * n + k) * n + i];
+                const double D = 0.5 * (p - m), T = 0.5 * (p + m);
+                const int c = S.cls[i];
+                int rowOf = 0, colOf = 0;
+                for (int x = 0; x < S.size[c]; x++) {
+                    rowOf = S.member[c][x] == k ? x : rowOf;
+                    colOf = S.member[c][x] == i ? x : colOf;
+                }
+                if (S.cls[k] == c)
+                    out[S.offD[d] + S.offA[c] + rowOf * S.size[c] + colOf] = D;
+                else if (!(std::fabs(D) <= 1e-14 * top))
+                    return false;
+                if (S.b[d][k][i] >= 0)
+                    out[S.offS[d] + S.b[d][k][i]] = T;
+                else if (!(std::fabs(T) <= 1e-14 * top))
+                    return false;
+            }
+    return true;
+}
+
+template <int N>
+cudaError_t pn_parity_launch(const PnArgs &a, const std::vector<double> &coef, int tiles, cudaStream_t stream)
+{
+    constexpr auto &S = PnTable<N>::s;
+    PnCoef<N> q;
+    for (int d = 0; d < 2; d++) {
+        const double r = d ? a.rdy : a.rdx;
+        for (int e = 0; e < S.countA; e++)
+            q.c[S.offD[d] + e] = coef[S.offD[d] + e] * r;
+        for (int e = 0; e < S.countB[d]; e++)
+            q.c[S.offS[d] + e] = coef[S.offS[d] + e] * r;
+    }
+    pn_parity_kernel<N><<<tiles, kParThreads, pn_parity_smem<N>(), stream>>>(a, q);
+    return cudaGetLastError();
+}
+
 template <int NP>
 size_t pn_tile_smem() { return (size_t)(4 * NP * (NP + 4) + (kTI + 4) * (kTJ + 4) * (NP + 4)) * sizeof(double); }
 
@@ -317,6 +616,8 @@ struct cl_pn {
     double *opsT = nullptr, *filter = nullptr, *sigT = nullptr, *sigS = nullptr;
     int exchanged = -1;    // sides whose ghosts hold neighbour values (-1: periodic or none)
     int nCtas = 0;
+    int parityOrder = 0;           // > 0: the operators have the structure of this order (pn_parity_kernel)
+    std::vector<double> coef;      // and these nonzero entries
     std::string err;
     // cl_pn_step_host: upload and readback streams and their events (created on first use)
     cudaStream_t up = nullptr, down = nullptr;
@@ -339,10 +640,27 @@ static int pn_fail(cl_pn *p, int rc)
         }                                                                                      \
     } while (0)
 
+// Calls f with the order as a compile-time constant (1..9).
+template <class F>
+static auto pn_with_order(int order, F &&f)
+{
+    switch (order) {
+    case 1: return f(Int<1>());
+    case 2: return f(Int<2>());
+    case 3: return f(Int<3>());
+    case 4: return f(Int<4>());
+    case 5: return f(Int<5>());
+    case 6: return f(Int<6>());
+    case 7: return f(Int<7>());
+    case 8: return f(Int<8>());
+    default: return f(Int<9>());
+    }
+}
+
 // One stage over interior rows [rowBegin, rowEnd) (rowEnd < 0: all rows) on
-// `stream` (null: the solver's); reads p->cur.
+// `stream` (null: the solver's); reads p->cur.  wrap: see PnArgs.
 static cudaError_t pn_launch(cl_pn *p, int stage, double dt, double dx, double dy, int rowBegin = 0,
-                             int rowEnd = -1, cudaStream_t stream = nullptr)
+                             int rowEnd = -1, cudaStream_t stream = nullptr, int wrap = 0)
 {
     if (rowEnd < 0)
         rowEnd = p->NX - 4;
@@ -374,6 +692,14 @@ static cudaError_t pn_launch(cl_pn *p, int stage, double dt, double dx, double d
     const long long rows = rowEnd - rowBegin, ny = p->NY - 4;
     if (rows <= 0)
         return cudaSuccess;
+    a.wrap = wrap;
+    if (p->parityOrder > 0) {
+        const long long tiles = ((rows + kTI - 1) / kTI) * ((ny + kTJ - 1) / kTJ);
+        clb_count_launches(1);
+        return pn_with_order(p->parityOrder, [&](auto N) {
+            return pn_parity_launch<decltype(N)::value>(a, p->coef, (int)tiles, stream);
+        });
+    }
     const long long units = (np <= 32) ? ((rows + kTI - 1) / kTI) * ((ny + kTJ - 1) / kTJ)
                                        : (rows * ny + kPnWarps - 1) / kPnWarps;
     const int ctas = (int)std::max<long long>(1, std::min<long long>(units, p->nCtas));
@@ -447,6 +773,15 @@ int cl_pn_create(const cl_grid *grid, const cl_pn_setup *setup, const double *si
     cudaMemcpy(p->U, moments, C * n * 8, cudaMemcpyHostToDevice);
     cudaMemcpy(p->V, moments, C * n * 8, cudaMemcpyHostToDevice);
     p->cur = p->U;
+    // operators with the harmonics' parity structure: pn_parity_kernel
+    for (int N = 1; N <= 9; N++)
+        if ((N + 1) * (N + 2) / 2 == p->n && pn_with_order(N, [&](auto O) {
+                constexpr int order = decltype(O)::value;
+                return pn_parity_coefs<order>(setup->ops, p->coef) &&
+                       cudaFuncSetAttribute(pn_parity_kernel<order>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)pn_parity_smem<order>()) == cudaSuccess;
+            }))
+            p->parityOrder = N;
     // the kernel for this n, its shared memory, and the units it loops over
     const int np = (int)(n + 7) / 8 * 8;
     const void *fn = nullptr;
@@ -511,7 +846,7 @@ void cl_pn_destroy(cl_pn *p)
 
 const char *cl_pn_last_error(const cl_pn *p) { return p ? p->err.c_str() : cl_global_error(); }
 
-int cl_pn_stage(cl_pn *p, int stage, double dt, double dx, double dy)
+static int pn_stage(cl_pn *p, int stage, double dt, double dx, double dy, int wrap)
 {
     if (!p || (stage != 1 && stage != 2))
         return CL_ERR_ARG;
@@ -519,10 +854,12 @@ int cl_pn_stage(cl_pn *p, int stage, double dt, double dx, double dy)
         p->err = "stages must alternate 1, 2";
         return CL_ERR_STATE;
     }
-    PN_TRY(p, pn_launch(p, stage, dt, dx, dy));
+    PN_TRY(p, pn_launch(p, stage, dt, dx, dy, 0, -1, nullptr, wrap));
     p->cur = (stage == 1) ? p->V : p->U;
     return CL_OK;
 }
+
+int cl_pn_stage(cl_pn *p, int stage, double dt, double dx, double dy) { return pn_stage(p, stage, dt, dx, dy, 0); }
 
 int cl_pn_sync(cl_pn *p)
 {
@@ -537,11 +874,18 @@ int cl_pn_step(cl_pn *p, double dt, double dx, double dy)
     if (!p)
         return CL_ERR_ARG;
     for (int stage = 1; stage <= 2; stage++) {
+        // periodic ghosts: pn_parity_kernel reads the cells they copy (a
+        // step leaves the state's ghosts as of its first stage)
+        int wrap = 0;
         if (p->grid.init_cond == 2) {
-            PN_TRY(p, launch_ghost_periodic(p->cur, p->n, p->NX, p->NY, p->stream));
-            clb_count_launches(2);
+            if (p->parityOrder > 0) {
+                wrap = stage == 1 ? 2 : 1;
+            } else {
+                PN_TRY(p, launch_ghost_periodic(p->cur, p->n, p->NX, p->NY, p->stream));
+                clb_count_launches(2);
+            }
         }
-        int rc = cl_pn_stage(p, stage, dt, dx, dy);
+        int rc = pn_stage(p, stage, dt, dx, dy, wrap);
         if (rc)
             return rc;
     }
