@@ -386,7 +386,7 @@ __device__ __forceinline__ void static_for(F &&f)
 // stride: conflict-free for a thread per cell.
 constexpr int kParThreads = kTI * kTJ;
 template <int N>
-__global__ void __launch_bounds__(kParThreads) pn_parity_kernel(const PnArgs a, const __grid_constant__ PnCoef<N> q)
+__global__ void __launch_bounds__(kParThreads, N <= 6 ? 4 : 2) pn_parity_kernel(const PnArgs a, const __grid_constant__ PnCoef<N> q)
 {
     using T = PnTable<N>;
     constexpr int n = PnShape<N>::n, CS = n | 1, RW = kTJ + 4;
@@ -521,21 +521,37 @@ __global__ void __launch_bounds__(kParThreads) pn_parity_kernel(const PnArgs a, 
             break;
         const size_t base = ((size_t)(i0 + r) * a.NY + j0) * n;
         const double *row = tile + ((r + 2) * RW + 2) * CS;
-        for (int e = lane * V; e < cols * n; e += 32 * V) {
-            const double *t = row + (e / n) * CS + e % n;
-            if constexpr (V == 2) {
-                double2 u = make_double2(t[0], t[1]);
-                if (a.old) {   // moment_update.cpp:237-246
-                    const double2 o = *reinterpret_cast<const double2 *>(a.old + base + e);
-                    u.x = __dmul_rn(0.5, __dadd_rn(u.x, o.x));
-                    u.y = __dmul_rn(0.5, __dadd_rn(u.y, o.y));
+        // the old state's loads of a row all in flight before the first is used
+        constexpr int kIter = (kTJ * n + 32 * V - 1) / (32 * V), kB = kIter < 8 ? kIter : 8;
+#pragma unroll
+        for (int it0 = 0; it0 < kIter; it0 += kB) {
+            double o[kB][V];
+#pragma unroll
+            for (int b = 0; b < kB; b++) {
+                const int e = ((it0 + b) * 32 + lane) * V;
+                const bool ok = a.old && e < cols * n;
+                if constexpr (V == 2) {
+                    const double2 x = ok ? *reinterpret_cast<const double2 *>(a.old + base + e) : make_double2(0.0, 0.0);
+                    o[b][0] = x.x;
+                    o[b][1] = x.y;
+                } else {
+                    o[b][0] = ok ? a.old[base + e] : 0.0;
                 }
-                *reinterpret_cast<double2 *>(a.out + base + e) = u;
-            } else {
-                double u = t[0];
-                if (a.old)
-                    u = __dmul_rn(0.5, __dadd_rn(u, a.old[base + e]));
-                a.out[base + e] = u;
+            }
+#pragma unroll
+            for (int b = 0; b < kB; b++) {
+                const int e = ((it0 + b) * 32 + lane) * V;
+                if (e >= cols * n)
+                    continue;
+                const double *t = row + (e / n) * CS + e % n;
+                double u[V];
+#pragma unroll
+                for (int h = 0; h < V; h++)   // moment_update.cpp:237-246
+                    u[h] = a.old ? __dmul_rn(0.5, __dadd_rn(t[h], o[b][h])) : t[h];
+                if constexpr (V == 2)
+                    *reinterpret_cast<double2 *>(a.out + base + e) = make_double2(u[0], u[1]);
+                else
+                    a.out[base + e] = u[0];
             }
         }
     }
