@@ -588,7 +588,7 @@ struct cl_ctx {
     // band, the list length and the screening work counter
     NewtonArgs sargs;
     int screen = 0, nCtasScreen = 0;
-    int *dPend = nullptr, *dPend2 = nullptr, *dPendCount = nullptr, *dGate = nullptr, *dOrderCount = nullptr;
+    int *dPend = nullptr, *dPend2 = nullptr, *dPendCount = nullptr, *dGate = nullptr, *dOrderCount = nullptr, *dOrderWork = nullptr;
     unsigned int *dScreenQ = nullptr;
     int angN = 0, angN2 = 0, angNq = 0, angGaunt = 0, angNnz = 0;
     std::vector<double> aw, axi, aeta, ap, agval;
@@ -773,7 +773,8 @@ int cl_create(const cl_grid *grid, const cl_options *opts, const cl_angular *ang
         cudaMalloc(&ctx->dPendCount, (4 + kHostBands) * sizeof(int)) != cudaSuccess ||
         cudaMalloc(&ctx->dScreenQ, (4 + kHostBands) * sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc(&ctx->dGate, (4 + kHostBands) * sizeof(int)) != cudaSuccess ||
-        cudaMalloc(&ctx->dOrderCount, (4 + kHostBands) * sizeof(int)) != cudaSuccess) {
+        cudaMalloc(&ctx->dOrderCount, (4 + kHostBands) * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&ctx->dOrderWork, (4 + kHostBands) * kOrderWork * sizeof(int)) != cudaSuccess) {
         ctx->err = "device allocation failed";
         return ctx_fail(ctx, CL_ERR_CUDA);
     }
@@ -929,6 +930,7 @@ void cl_destroy(cl_ctx *ctx)
     cudaFree(ctx->dScreenQ);
     cudaFree(ctx->dGate);
     cudaFree(ctx->dOrderCount);
+    cudaFree(ctx->dOrderWork);
     cudaFree(ctx->dSigT);
     cudaFree(ctx->dSigS);
     cudaFree(ctx->dQueue);
@@ -1008,11 +1010,10 @@ static void update_screen(cl_ctx *ctx)
 // (and its window at t = 0.9, 56 % one-iteration cells, 6 % faster screened).
 constexpr double kScreenGate = 0.45;
 
-// Whole stages of at most this many cells are ordered for K1 too (gate
-// shut, or no screening): one CTA sorts them in a small fraction of the
-// stage.  Larger stages keep cell order: sorting 646,416 cells in one CTA
-// took about a millisecond per stage and measured 4-6 % slower at t = 0.9 of
-// the M6 pulse.
+// Whole stages of at most this many cells (gate shut, or no screening) are
+// ordered for K1 too.  Larger stages keep cell order: at t = 0.9 of the M6
+// pulse (646,416 cells) grouping the hard cells into the same rounds measured
+// 4-6 % slower.
 constexpr int kOrderWholeMax = 131072;
 
 // K1 of a grid stage or band (`a` complete; `slot` selects the counters).
@@ -1057,9 +1058,9 @@ static cudaError_t launch_stage_newton(cl_ctx *ctx, NewtonArgs &a, int slot, cud
         }
         if ((e = launch_order_cells(ctx->screen ? ctx->dPend + kp.first : nullptr, ctx->dPendCount + slot, kp.first,
                                     kp.count, ctx->screen ? ctx->dGate + slot : nullptr, gateMin, kOrderWholeMax,
-                                    kp.iters, ctx->dPend2 + kp.first, ctx->dOrderCount + slot, st)) != cudaSuccess)
+                                    kp.iters, ctx->dOrderWork + slot * kOrderWork, ctx->dPend2 + kp.first,
+                                    ctx->dOrderCount + slot, st, nk)) != cudaSuccess)
             return e;
-        *nk += 1;
         a.prob.cellList = ctx->dPend2 + kp.first;
         a.prob.countDev = ctx->dOrderCount + slot;
     }
@@ -1637,13 +1638,14 @@ static float time_newton(cl_ctx *ctx, NewtonArgs a, const DeviceBasis &B, TuneSc
             return -1.0f;
         cudaEventRecord(S.e0, st);
         if (sgrid > 0) {
+            int nk = 2;
             if (launch_screen_gate(S.it, 0, (int)C, (int *)(S.q + 3), st) != cudaSuccess ||
                 launch_screen(sa, sgrid, st) != cudaSuccess ||
                 launch_order_cells(ctx->dPend, (const int *)(S.q + 2), 0, (int)C, (const int *)(S.q + 3),
-                                   sa.prob.gateMin, kOrderWholeMax, S.it, ctx->dPend2, (int *)(S.q + 4),
-                                   st) != cudaSuccess)
+                                   sa.prob.gateMin, kOrderWholeMax, S.it, ctx->dOrderWork, ctx->dPend2,
+                                   (int *)(S.q + 4), st, &nk) != cudaSuccess)
                 return -1.0f;
-            g_launches += 3;
+            g_launches += nk;
         }
         if (launch_newton(a, grid, st) != cudaSuccess)
             return -1.0f;

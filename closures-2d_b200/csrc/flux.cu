@@ -418,36 +418,64 @@ __global__ void __launch_bounds__(kFluxThreads, 1) flux_kernel(const __grid_cons
 }
 
 // Projection and update of the SPLIT form: a warp per 16 cells of a tile, the
-// chunks in order, F and the basis rows read through L2.
-constexpr int kProjWarps = 4;
+// chunks in order.  The chain over the chunks is short (a few MMAs each), so
+// the loads decide: F of the CTA's 64 cells and the basis rows come through a
+// ring of kProjStages chunks of asynchronous copies (read straight from L2 they
+// took 80 us for 57 chunks).
+constexpr int kProjWarps = 4, kProjCells = 16 * kProjWarps, kProjStages = 6;
+constexpr int kProjLd = kProjCells + 4;   // % 16 == 4: conflict-free fragment loads
 template <int PAIR>
 __global__ void __launch_bounds__(kProjWarps * 32) flux_project_kernel(const __grid_constant__ FluxArgs f)
 {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-    const int local = blockIdx.x / (IC / 16 / kProjWarps);
-    const int mt = (blockIdx.x % (IC / 16 / kProjWarps)) * kProjWarps + (threadIdx.x >> 5);
+    extern __shared__ __align__(16) double sm[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+    constexpr int kGroups = IC / kProjCells;
+    const int local = blockIdx.x / kGroups, cell0 = (blockIdx.x % kGroups) * kProjCells;
     const int tile = local + f.tileBase;
     const int i0 = 2 + (tile / f.tilesY) * TX, j0 = 2 + (tile % f.tilesY) * TY;
     constexpr int kr = PAIR ? kQ / 2 : kQ;
-    const int nchunks = f.nqp / kr, ldPf = f.ldPf, NTf = f.nb / 8;
+    const int nchunks = f.nqp / kr, ldPf = f.ldPf, NTf = f.nb / 8, nbe = f.nbe;
+    const int stage = kQ * kProjLd + kr * ldPf;
     double acc[4][4];
 #pragma unroll
     for (int j = 0; j < 4; j++)
         acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0;
     if (f.tileRun[local]) {
-        const double *F = f.F + (size_t)local * nchunks * (kQ * IC) + t4 * IC + mt * 16 + g;
-        const double *B = f.P + t4 * ldPf + g;
-#pragma unroll 4
-        for (int c = 0; c < nchunks; c++, F += kQ * IC, B += kr * ldPf) {
+        auto load = [&](int c) {
+            double *d = sm + (c % kProjStages) * stage;
+            const double *F = f.F + ((size_t)local * nchunks + c) * (kQ * IC) + cell0;
+            for (int i = tid; i < kQ * kProjCells / 2; i += kProjWarps * 32) {
+                const int q = i / (kProjCells / 2), x = 2 * (i % (kProjCells / 2));
+                cp_async16(d + q * kProjLd + x, F + q * IC + x);
+            }
+            const double *P = f.P + (size_t)c * kr * ldPf;
+            for (int i = tid; i < kr * ldPf / 2; i += kProjWarps * 32)
+                cp_async16(d + kQ * kProjLd + 2 * i, P + 2 * i);
+        };
+        for (int c = 0; c < kProjStages - 1; c++) {
+            if (c < nchunks)
+                load(c);
+            cp_async_commit();
+        }
+        for (int c = 0; c < nchunks; c++) {
+            cp_async_wait<kProjStages - 2>();
+            __syncthreads();   // chunk c is there; everybody is done with chunk c - 1
+            if (c + kProjStages - 1 < nchunks)
+                load(c + kProjStages - 1);
+            cp_async_commit();
+            const double *d = sm + (c % kProjStages) * stage;
+            const double *F = d + t4 * kProjLd + warp * 16 + g;
+            const double *B = d + kQ * kProjLd + t4 * ldPf + g;
             if (PAIR) {
-                const double f0 = F[0], f1 = F[8], f2 = F[4 * IC], f3 = F[4 * IC + 8];
-                const double p0 = F[8 * IC], p1 = F[8 * IC + 8], p2 = F[12 * IC], p3 = F[12 * IC + 8];
+                const double f0 = F[0], f1 = F[8], f2 = F[4 * kProjLd], f3 = F[4 * kProjLd + 8];
+                const double p0 = F[8 * kProjLd], p1 = F[8 * kProjLd + 8];
+                const double p2 = F[12 * kProjLd], p3 = F[12 * kProjLd + 8];
                 const double s0 = f0 + p0, s1 = f1 + p1, s2 = f2 + p2, s3 = f3 + p3;
                 const double d0 = f0 - p0, d1 = f1 - p1, d2 = f2 - p2, d3 = f3 - p3;
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     if (j < NTf) {
-                        if (j * 8 < f.nbe)
+                        if (j * 8 < nbe)
                             dmma16x8x8(acc[j], s0, s1, s2, s3, B[j * 8], B[4 * ldPf + j * 8]);
                         else
                             dmma16x8x8(acc[j], d0, d1, d2, d3, B[j * 8], B[4 * ldPf + j * 8]);
@@ -456,8 +484,8 @@ __global__ void __launch_bounds__(kProjWarps * 32) flux_project_kernel(const __g
             } else {
 #pragma unroll
                 for (int k0 = 0; k0 < kQ; k0 += 8) {
-                    const double a0 = F[k0 * IC], a1 = F[k0 * IC + 8];
-                    const double a2 = F[(k0 + 4) * IC], a3 = F[(k0 + 4) * IC + 8];
+                    const double a0 = F[k0 * kProjLd], a1 = F[k0 * kProjLd + 8];
+                    const double a2 = F[(k0 + 4) * kProjLd], a3 = F[(k0 + 4) * kProjLd + 8];
 #pragma unroll
                     for (int j = 0; j < 4; j++)
                         if (j < NTf)
@@ -466,7 +494,12 @@ __global__ void __launch_bounds__(kProjWarps * 32) flux_project_kernel(const __g
             }
         }
     }
-    flux_update<PAIR>(f, acc, i0, j0, mt, g, t4);
+    flux_update<PAIR>(f, acc, i0, j0, cell0 / 16 + warp, g, t4);
+}
+
+static int project_smem(const FluxArgs &f)
+{
+    return kProjStages * (kQ * kProjLd + (f.paired ? kQ / 2 : kQ) * f.ldPf) * (int)sizeof(double);
 }
 
 __global__ void ghost_periodic_kernel(double *m, int n, int NX, int NY)
@@ -593,8 +626,12 @@ cudaError_t prepare_flux(const FluxArgs &f)
                              : cudaFuncSetAttribute(flux_kernel<0, 0>, attr, f.smemBytes);
     if (e != cudaSuccess)
         return e;
-    return f.paired ? cudaFuncSetAttribute(flux_kernel<1, 1>, attr, f.smemBytes)
-                    : cudaFuncSetAttribute(flux_kernel<0, 1>, attr, f.smemBytes);
+    e = f.paired ? cudaFuncSetAttribute(flux_kernel<1, 1>, attr, f.smemBytes)
+                 : cudaFuncSetAttribute(flux_kernel<0, 1>, attr, f.smemBytes);
+    if (e != cudaSuccess)
+        return e;
+    return f.paired ? cudaFuncSetAttribute(flux_project_kernel<1>, attr, project_smem(f))
+                    : cudaFuncSetAttribute(flux_project_kernel<0>, attr, project_smem(f));
 }
 
 // Shares of the direction loop for `tiles` tiles on `sms` SMs (one CTA each):
@@ -635,13 +672,13 @@ cudaError_t launch_flux_tiles(const FluxArgs &f, int first, int count, cudaStrea
     const int shares = (f.F && f.tileRun) ? flux_shares(count, f.nqp / (f.paired ? kQ / 2 : kQ), f.sms) : 1;
     if (shares > 1) {
         const dim3 grid((unsigned)count, (unsigned)shares);
-        const int pgrid = count * (IC / 16 / kProjWarps);
+        const int pgrid = count * (IC / kProjCells), psmem = project_smem(g);
         if (g.paired) {
             flux_kernel<1, 1><<<grid, kFluxThreads, g.smemBytes, stream>>>(g);
-            flux_project_kernel<1><<<pgrid, kProjWarps * 32, 0, stream>>>(g);
+            flux_project_kernel<1><<<pgrid, kProjWarps * 32, psmem, stream>>>(g);
         } else {
             flux_kernel<0, 1><<<grid, kFluxThreads, g.smemBytes, stream>>>(g);
-            flux_project_kernel<0><<<pgrid, kProjWarps * 32, 0, stream>>>(g);
+            flux_project_kernel<0><<<pgrid, kProjWarps * 32, psmem, stream>>>(g);
         }
         *kernels += 2;
         return cudaGetLastError();

@@ -88,15 +88,17 @@ struct NewtonProblem {
 // Cells of [first, first + count) whose previous solve took at most one
 // iteration (iters[c] <= 1), added to *out (zero before the launch).
 cudaError_t launch_screen_gate(const int *iters, int first, int count, int *out, cudaStream_t stream);
-// K1's list, most previous iterations first (iters[c], a counting sort in
-// one CTA), so that K1 starts the longest Newton chains first and the short
+// K1's list, most previous iterations first (iters[c], a counting sort), so
+// that K1 starts the longest Newton chains first and the short
 // ones fill in behind them: the *listCount cells of `list` when the
 // screening gate is open (list non-null and *gateCount >= gateMin); else the
 // cells first .. first + count - 1 when count <= wholeMax, or *outCount = -1
-// (K1 takes the range in cell order); written to out[0 .. *outCount).
+// (K1 takes the range in cell order); written to out[0 .. *outCount).  work:
+// kOrderWork ints of this launch.  *kernels += the kernels launched.
+constexpr int kOrderWork = 64;
 cudaError_t launch_order_cells(const int *list, const int *listCount, int first, int count, const int *gateCount,
-                               int gateMin, int wholeMax, const int *iters, int *out, int *outCount,
-                               cudaStream_t stream);
+                               int gateMin, int wholeMax, const int *iters, int *work, int *out, int *outCount,
+                               cudaStream_t stream, int *kernels);
 
 // Per-slot state in shared memory: slot states, doubles (SC_*) and ints (SI_*).
 // S_HELP: an idle slot lent, for one round, to a slot whose line search is
