@@ -55,6 +55,7 @@ struct DeviceBasis {
     // direction pairs (Newton layout): basis and Hessian columns grouped by
     // degree parity, even group first (nbe, K2e columns, multiples of 8)
     int paired = 0, nbe = 0, K2e = 0;
+    int quad = 0;                                  // fourfold: four column groups, one row per four directions
     short *binv = nullptr;                         // [nb] moment of each basis column, -1 padding
     int *pcol = nullptr;                           // [n(n+1)/2] G column of each product (no Gaunt)
     double p0 = 0;
@@ -135,28 +136,85 @@ static void harmonic_degrees(int count, std::vector<int> &deg)
             deg[k++] = l;
 }
 
+// Columns of a grouped layout: the entries of class 0 first, then class 1, ...,
+// each group padded to a multiple of `pad`; col[i] = position of entry i,
+// start[c] = first column of class c (start[classes] = the total).
+static void group_columns(const std::vector<int> &cls, int classes, int pad, std::vector<int> &col,
+                          std::vector<int> &start)
+{
+    std::vector<int> count(classes, 0);
+    col.resize(cls.size());
+    for (size_t i = 0; i < cls.size(); i++)
+        col[i] = count[cls[i]]++;
+    start.assign(classes + 1, 0);
+    for (int c = 0; c < classes; c++)
+        start[c + 1] = start[c] + round_up(count[c], pad);
+    for (size_t i = 0; i < cls.size(); i++)
+        col[i] += start[cls[i]];
+}
+
 // Columns of one group layout: even-parity entries first, then odd, each
 // group padded to a multiple of 8; col[i] = position of entry i.
 static void parity_columns(const std::vector<int> &deg, int paired, std::vector<int> &col, int &evenCols,
                            int &total)
 {
-    const int cnt = (int)deg.size();
-    col.resize(cnt);
-    if (!paired) {
-        for (int i = 0; i < cnt; i++)
-            col[i] = i;
-        evenCols = 0;
-        total = round_up(cnt, 8);
-        return;
+    std::vector<int> cls(deg.size(), 0), start;
+    if (paired)
+        for (size_t i = 0; i < deg.size(); i++)
+            cls[i] = deg[i] % 2;
+    group_columns(cls, paired ? 2 : 1, 8, col, start);
+    evenCols = paired ? start[1] : 0;
+    total = start.back();
+}
+
+// Class of each z-even harmonic of `count` in the basis order under
+// phi -> phi + pi and phi -> -phi: 2 (odd degree) + (sine).
+static std::vector<int> harmonic_classes(int count)
+{
+    std::vector<int> cls(count);
+    int k = 0;
+    for (int l = 0; k < count; l++)
+        for (int m = -l; m <= l && k < count; m += 2)
+            cls[k++] = 2 * (l % 2) + (m < 0 ? 1 : 0);
+    return cls;
+}
+
+// The direction of row r of a fourfold layout (phi in the first quadrant of
+// its Gauss-Legendre level) and its images phi + pi, -phi, pi - phi, with
+// phi_k = (k + 1/2) pi / Q.
+static void quad_directions(int r, int Q, int (&q)[4])
+{
+    const int level = r / (Q / 2) * 2 * Q, k = r % (Q / 2);
+    q[0] = level + k;
+    q[1] = level + k + Q;
+    q[2] = level + 2 * Q - 1 - k;
+    q[3] = level + Q - 1 - k;
+}
+
+// Whether the weights and all `cols` basis columns have the fourfold symmetry
+// (to 1e-12; the library's own quadrature does to 1.4e-14).
+static bool quad_symmetric(int nq, int cols, int ld, const double *w, const double *p)
+{
+    const int Q = (int)std::lround(std::sqrt((double)nq));
+    if (Q * Q != nq || Q % 2 != 0)
+        return false;
+    const std::vector<int> cls = harmonic_classes(cols);
+    for (int r = 0; r < nq / 4; r++) {
+        int q[4];
+        quad_directions(r, Q, q);
+        for (int h = 1; h < 4; h++) {
+            if (!(std::fabs(w[q[h]] - w[q[0]]) <= 1e-12 * std::fabs(w[q[0]])))
+                return false;
+            for (int k = 0; k < cols; k++) {
+                // signs under phi + pi (odd degree) and -phi (sine)
+                const bool flip = ((h == 1 || h == 3) && cls[k] >= 2) != ((h == 2 || h == 3) && cls[k] % 2);
+                const double a = p[(size_t)q[0] * ld + k], b = p[(size_t)q[h] * ld + k];
+                if (!(std::fabs(b - (flip ? -a : a)) <= 1e-12))
+                    return false;
+            }
+        }
     }
-    int ne = 0;
-    for (int i = 0; i < cnt; i++)
-        ne += (deg[i] % 2 == 0);
-    evenCols = round_up(ne, 8);
-    int ie = 0, io = 0;
-    for (int i = 0; i < cnt; i++)
-        col[i] = (deg[i] % 2 == 0) ? ie++ : evenCols + io++;
-    total = evenCols + round_up(cnt - ne, 8);
+    return true;
 }
 
 // n, n2, nq, w, xi, eta, p[nq*n2], Gaunt CSR -> device layouts.
@@ -180,7 +238,13 @@ cudaError_t build_device_basis(DeviceBasis &B, int n, int n2, int nq, int useGau
     const int Q = (int)std::lround(std::sqrt((double)nq));
     if (Q * Q != nq || Q % 2 != 0)
         paired = fluxPaired = 0;
+    // the Gaunt orders 3-6 fold four directions into one (phi -> -phi as
+    // well); tables without that symmetry keep one direction per row
+    const int quad = (paired && useGaunt && newton_quad_supported(n)) ? 1 : 0;
+    if (quad && !quad_symmetric(nq, n2, n2, w, p))
+        paired = 0;
     B.paired = paired;
+    B.quad = quad && paired;
     const int K2 = useGaunt ? n2 : n * (n + 1) / 2;
     std::vector<unsigned short> prod(n * (n + 1) / 2);
     product_columns(n, prod.data());
@@ -195,7 +259,23 @@ cudaError_t build_device_basis(DeviceBasis &B, int n, int n2, int nq, int useGau
     }
     parity_columns(degB, paired, colB, B.nbe, B.nb);
     parity_columns(degH, paired, colH, B.K2e, B.K2p);
-    const int rows = paired ? nq / 2 : nq;
+    std::vector<int> startH;
+    if (B.quad) {
+        // basis groups in k-steps of 4, column groups in tiles of 8
+        std::vector<int> startB;
+        group_columns(harmonic_classes(n), 4, 4, colB, startB);
+        group_columns(harmonic_classes(n2), 4, 8, colH, startH);
+        B.nb = startB[4];
+        B.K2p = startH[4];
+    }
+    const int rows = B.quad ? nq / 4 : paired ? nq / 2 : nq;
+    auto direction = [&](int r) {   // of row r
+        if (!B.quad)
+            return paired ? (r / Q) * 2 * Q + r % Q : r;
+        int q[4];
+        quad_directions(r, Q, q);
+        return q[0];
+    };
     B.nqp = round_up(rows, 32);
     int ldP = B.nb + B.K2p;
     while (ldP % 16 != 4)
@@ -204,7 +284,7 @@ cudaError_t build_device_basis(DeviceBasis &B, int n, int n2, int nq, int useGau
     B.p0 = p[0];
     std::vector<double> P((size_t)B.nqp * ldP + B.nqp, 0.0), W(B.nqp, 0.0);
     for (int r = 0; r < rows; r++) {
-        const int q = paired ? (r / Q) * 2 * Q + r % Q : r;
+        const int q = direction(r);
         const double *pq = p + (size_t)q * n2;
         double *row = &P[(size_t)basis_row(r, ldP)];
         for (int k = 0; k < n; k++)
@@ -369,8 +449,17 @@ cudaError_t build_device_basis(DeviceBasis &B, int n, int n2, int nq, int useGau
         B.K2ps = B.K2es + round_up(n - ne, 8);
         std::vector<int> colS(n);
         bool ok = true;
+        if (B.quad) {
+            const std::vector<int> cls = harmonic_classes(n);
+            std::vector<int> startS;
+            group_columns(cls, 4, 8, colS, startS);
+            B.K2ps = startS[4];
+            for (int k = 0; k < n; k++)   // the same place in its group as in the full layout
+                ok = ok && colS[k] - startS[cls[k]] == colH[k] - startH[cls[k]];
+        }
         for (int k = 0; k < n; k++) {
-            colS[k] = (degB[k] % 2 == 0) ? colH[k] : colH[k] - B.K2e + B.K2es;
+            if (!B.quad)
+                colS[k] = (degB[k] % 2 == 0) ? colH[k] : colH[k] - B.K2e + B.K2es;
             ok = ok && (degH[k] == degB[k]) && colS[k] >= 0 && colS[k] < B.K2ps;
         }
         int ldPs = B.nb + B.K2ps;
@@ -379,7 +468,7 @@ cudaError_t build_device_basis(DeviceBasis &B, int n, int n2, int nq, int useGau
         B.ldPs = ldPs;
         std::vector<double> Ps((size_t)B.nqp * ldPs + B.nqp, 0.0);
         for (int r = 0; r < rows; r++) {
-            const int q = (r / Q) * 2 * Q + r % Q;
+            const int q = direction(r);
             const double *pq = p + (size_t)q * n2;
             double *row = &Ps[(size_t)basis_row(r, ldPs)];
             for (int k = 0; k < n; k++)
@@ -456,6 +545,7 @@ NewtonProblem make_problem(const DeviceBasis &B)
     pb.nqp = B.nqp;
     pb.ldP = B.ldP;
     pb.paired = B.paired;
+    pb.quad = B.quad;
     pb.nbe = B.nbe;
     pb.K2e = B.K2e;
     pb.binv = B.binv;

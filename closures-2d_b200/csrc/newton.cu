@@ -68,7 +68,7 @@ int plan_newton(NewtonArgs &a)
     if (a.mixed && a.ntExact == 0)
         return -2;
     if (nw != kWarps && (a.ntExact == 0 || !pb.paired || a.mixed || a.optType != 0 ||
-                         !newton_pair4_supported(a.ntExact, a.nbk, a.prob.n)))
+                         !(pb.quad ? newton_quad_supported(pb.n) : newton_pair4_supported(a.ntExact, a.nbk, pb.n))))
         return -1;   // the 16-slot shape: direction-pair Newton only
     // phase-B region
     int offG = unionBase;

@@ -55,6 +55,7 @@ struct NewtonProblem {
     // K2e even Hessian columns, each group padded to 8); binv[j] is the moment
     // of basis column j (-1 padding), pcol[c] the G column of product c
     int paired, nbe, K2e;
+    int quad;                   // fourfold directions (paired too): four column groups, see quad_groups()
     const short *binv;
     const int *pcol;
     int count;                  // vectors to solve
@@ -160,6 +161,8 @@ cudaError_t prepare_newton(const NewtonArgs &a);
 bool newton_pair_supported(int nt, int nbk, int n);
 // ... and in the 16-slot launch shape.
 bool newton_pair4_supported(int nt, int nbk, int n);
+// Fourfold instances (both shapes, and the screening pass) exist for n moments.
+bool newton_quad_supported(int n);
 // Screening pass (Mn, FP64, direction pairs; a.prob the gradient-column
 // layout of the problem): layout, instance check, shared-memory attribute,
 // launch and resident CTAs per SM.

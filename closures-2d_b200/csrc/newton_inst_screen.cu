@@ -1,14 +1,14 @@
 // newton_inst_screen.cu -- the screening pass of K1 (screen_kernel in
 // newton_kernel.cuh): layout planning and its instances, one per (gradient
-// column tiles, k-steps) of the direction-pair layouts of orders 1-6:
-// N = 1..3 -> (2, 2), N = 4 -> (3, 3), N = 5, 6 -> (4, 4).
+// column tiles, k-steps) of the direction-pair layouts: orders 1, 2 and direct
+// 3 -> (2, 2), direct 4 -> (3, 3); and one per Gaunt order 3-6 (fourfold).
 #include "newton_kernel.cuh"
 
 #include <algorithm>
 
 namespace clb {
 
-bool screen_supported(int nt, int nbk) { return nt == nbk && nt >= 2 && nt <= 4; }
+bool screen_supported(int nt, int nbk) { return nt == nbk && nt >= 2 && nt <= 3; }
 
 int plan_screen(NewtonArgs &a)
 {
@@ -16,7 +16,7 @@ int plan_screen(NewtonArgs &a)
     if (!pb.paired || a.momentType != 0 || a.mixed || a.optType != 0)
         return -1;
     a.nw = a.warps = kWarps;
-    a.T = 32;
+    a.T = pb.quad ? 16 : 32;
     a.kq = 32;
     a.ntq = a.kq / 8;
     a.ldv = pb.nb + 4;
@@ -47,7 +47,7 @@ int plan_screen(NewtonArgs &a)
     exp_consts_init(a.ex);
     const int unionBase = off;
     const int endG = unionBase + ((T * a.ldG + 1) & ~1);
-    const int endA = unionBase + 3 * (a.kq * pb.ldP + a.kq);   // three staged chunks
+    const int endA = unionBase + (pb.quad ? 2 : 3) * (a.kq * pb.ldP + a.kq);   // staged chunks
     a.offP = unionBase;
     a.offG = unionBase;
     a.offH = a.offVec = endG;
@@ -57,20 +57,32 @@ int plan_screen(NewtonArgs &a)
     a.nbk = pb.nb / 8;
     a.tpw = 0;
     a.smemBytes = (endA > endG ? endA : endG) * 8;
-    if (!screen_supported(a.ntExact, a.nbk) || a.smemBytes > 232448 - 1024)
+    if ((pb.quad ? !newton_quad_supported(pb.n) : !screen_supported(a.ntExact, a.nbk)) || a.smemBytes > 232448 - 1024)
         return -1;
     return 0;
 }
 
 static cudaError_t screen_dispatch(const NewtonArgs &a, int grid, cudaStream_t s, int mode, int *occ)
 {
+    if (a.prob.quad) {
+        switch (a.prob.n) {
+        case 10:
+            return screen_run<quad_groups(10, true).tile[4], 1, 10>(a, grid, s, mode, occ);
+        case 15:
+            return screen_run<quad_groups(15, true).tile[4], 1, 15>(a, grid, s, mode, occ);
+        case 21:
+            return screen_run<quad_groups(21, true).tile[4], 1, 21>(a, grid, s, mode, occ);
+        case 28:
+            return screen_run<quad_groups(28, true).tile[4], 1, 28>(a, grid, s, mode, occ);
+        default:
+            return cudaErrorInvalidValue;
+        }
+    }
     switch (a.ntExact) {
     case 2:
-        return screen_run<2, 2>(a, grid, s, mode, occ);
+        return screen_run<2, 2, 0>(a, grid, s, mode, occ);
     case 3:
-        return screen_run<3, 3>(a, grid, s, mode, occ);
-    case 4:
-        return screen_run<4, 4>(a, grid, s, mode, occ);
+        return screen_run<3, 3, 0>(a, grid, s, mode, occ);
     default:
         return cudaErrorInvalidValue;
     }

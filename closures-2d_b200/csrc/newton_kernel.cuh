@@ -1974,6 +1974,41 @@ __device__ __forceinline__ bool phase_a_fused(const NewtonArgs &a, const NewtonP
     return true;
 }
 
+// Fourfold directions (Mn, FP64, the Gaunt orders 3-6): the basis is even or
+// odd under phi -> phi + pi (degree) and under phi -> -phi (cos or sin), so one
+// direction of {phi, phi + pi, -phi, pi - phi} stands for the four.  Columns go
+// in four groups: even cos, even sin, odd cos, odd sin.  For n moments: the
+// k-steps of 4 of each basis group and the 8-column tiles of each group of
+// Hessian (degree 2N) or, in the screening pass, gradient columns (degree N).
+struct QuadGroups {
+    int k4[5], tile[5];   // first of each group, and the total
+};
+__host__ __device__ constexpr QuadGroups quad_groups(int n, bool screen)
+{
+    QuadGroups q = {};
+    int N = 0;
+    while ((N + 1) * (N + 2) / 2 < n)
+        N++;
+    int basis[4] = {}, cols[4] = {};
+    for (int l = 0; l <= 2 * N; l++) {
+        const int g = (l % 2) * 2, cosines = l % 2 ? (l + 1) / 2 : l / 2 + 1, sines = l + 1 - cosines;
+        if (l <= N) {
+            basis[g] += cosines;
+            basis[g + 1] += sines;
+        }
+        if (!screen || l <= N) {
+            cols[g] += cosines;
+            cols[g + 1] += sines;
+        }
+    }
+    for (int g = 0; g < 4; g++) {
+        q.k4[g + 1] = q.k4[g] + (basis[g] + 3) / 4;
+        q.tile[g + 1] = q.tile[g] + (cols[g] + 7) / 8;
+    }
+    return q;
+}
+constexpr int kQuad = -1, kQuadScreen = -2;   // values of PAIR for the fourfold layout
+
 // What phase_a_rows8 needs of the launch and the problem.
 struct PhaseA {
     int offAlpha, offScal, offFpart, offP, offG, offExp, offBar;   // doubles into shared memory
@@ -1983,6 +2018,41 @@ struct PhaseA {
     double invL, L1, L2;
     int *err;
 };
+
+__device__ __forceinline__ PhaseA make_phase_a(const NewtonArgs &a, const NewtonProblem &pb)
+{
+    PhaseA x;
+    x.offAlpha = a.offAlpha;
+    x.offScal = a.offScal;
+    x.offFpart = a.offFpart;
+    x.offP = a.offP;
+    x.offG = a.offG;
+    x.offExp = a.offExp;
+    x.offBar = a.offBar;
+    x.ldv = a.ldv;
+    x.ldG = a.ldG;
+    x.ntq = a.ntq;
+    x.nb = pb.nb;
+    x.ldP = pb.ldP;
+    x.K2p = pb.K2p;
+    x.nchunks = pb.nqp / 32;
+    x.P = pb.P;
+    x.binv = pb.binv;
+    x.invL = a.ex.invL;
+    x.L1 = a.ex.L1;
+    x.L2 = a.ex.L2;
+    x.err = a.err;
+    return x;
+}
+// The barrier parities after a round: each buffer's barriers went through a
+// phase per chunk it held.
+template <int DEPTH>
+__device__ __forceinline__ void advance_phases(unsigned &phases, int nchunks)
+{
+    for (int b = 0; b < DEPTH; b++)
+        if (((nchunks - b + DEPTH - 1) / DEPTH) & 1)
+            phases ^= 9u << b;
+}
 
 // The FP64 contractions in 8-slot row tiles (DMMA m8n8k4): warp w owns the 8
 // slots mt = w / 4 and the q-group qg = w % 4, so T slots take T / 2 warps.
@@ -1995,7 +2065,13 @@ struct PhaseA {
 // has the same terms in the same order as with 16-slot tiles.
 //
 // PAIR (Mn): 0, or 16 * (even column tiles) + even k-steps of the
-// direction-pair layout, whose parity split the unrolled loops then know.
+// direction-pair layout, or kQuad / kQuadScreen: the fourfold layout of NQ
+// moments (quad_groups).  The unrolled loops so know the split.  Fourfold rows
+// halve both the MMAs (M6: 9 + 26 per 8 rows as 8 + 26 with pairs, for four
+// directions instead of two) and the basis bytes a round stages, which set the
+// time when few tiles are in use (2.4k cycles per 35 KB chunk).  Against pairs:
+// 32,000 M6 vectors 4.82 -> 4.06 ms, a step of M6 800 x 800 50.0 -> 43.3 ms,
+// M4 200 x 200 3.42 -> 3.13, M3 36 x 74 0.380 -> 0.370.
 //
 // Chunks arrive by one bulk copy each and are handed back per warp (an
 // "empty" mbarrier per buffer, one arrival per warp), so warps drift up to a
@@ -2006,7 +2082,7 @@ struct PhaseA {
 //
 // A function of its own, so that its registers are not allocated under the
 // pressure of phase B (inlined, the chunk loop reloaded spilled operands).
-template <int NTF, int PPN, int NT, int NBK, int PAIR, int NW>
+template <int NTF, int PPN, int NT, int NBK, int PAIR, int NW, int NQ>
 __device__ __noinline__ bool phase_a_rows8(const PhaseA x, bool active, unsigned phases)
 {
     static_assert(!PAIR || PPN == 0, "direction pairs: Mn");
@@ -2018,10 +2094,13 @@ __device__ __noinline__ bool phase_a_rows8(const PhaseA x, bool active, unsigned
     const int g = lane >> 2, t4 = lane & 3;
     const int mt = warp >> 2, qg = warp & 3;     // a tile's four warps on four schedulers
     const int r0 = mt * 8 + g;
-    const int ldG = x.ldG, nb = (NBK > 0) ? 8 * NBK : x.nb, ldP = x.ldP;
+    constexpr bool QUAD = PAIR < 0;
+    constexpr QuadGroups QG = quad_groups(QUAD ? NQ : 3, PAIR == kQuadScreen);
+    const int ldG = x.ldG, nb = QUAD ? 4 * QG.k4[4] : (NBK > 0) ? 8 * NBK : x.nb, ldP = x.ldP;
     constexpr int NTL = (NT > 0) ? NT : NTF;
-    constexpr int KSL = (NBK > 0) ? NBK : 4;
-    constexpr int NTE = PAIR / 16, NBE = PAIR % 16;
+    constexpr int K4 = QUAD ? QG.k4[4] : (NBK > 0) ? 2 * NBK : 8;   // GEMM1 k-steps of 4
+    constexpr int NTE = QUAD ? 0 : PAIR / 16, NBE = QUAD ? 0 : PAIR % 16;
+    static_assert(!QUAD || NT == QG.tile[4], "column tiles of the fourfold layout");
     const int NTH = (NT > 0) ? NT - (PPN ? NBK : 0) : x.K2p / 8;
     const int NT2 = (NT > 0) ? NT : NTH + (PPN ? nb / 8 : 0);
     const int nchunks = x.nchunks;
@@ -2059,9 +2138,9 @@ __device__ __noinline__ bool phase_a_rows8(const PhaseA x, bool active, unsigned
     const int offB = basis_row(qb, ldP) + g;
     // this slot's multipliers, columns 8 ks + t4 and 8 ks + t4 + 4
     const double *const al = sm + x.offAlpha + r0 * x.ldv;
-    double aA[2 * KSL];
+    double aA[K4];
 #pragma unroll
-    for (int k2 = 0; k2 < 2 * KSL; k2++) {
+    for (int k2 = 0; k2 < K4; k2++) {
         const int c = k2 * 4 + t4;
         if constexpr (PAIR != 0) {
             const int k = x.binv[c];
@@ -2070,24 +2149,49 @@ __device__ __noinline__ bool phase_a_rows8(const PhaseA x, bool active, unsigned
             aA[k2] = (NBK > 0 || k2 * 4 < nb) ? al[c] : 0.0;
         }
     }
-    double e[2], eg[2];
-    // S of the chunk at Pc: cs (PAIR: even half sums), co (odd ones)
-    auto gemm1 = [&](const double *Pc, double (&cs)[2], double (&co)[2]) {
-        cs[0] = cs[1] = co[0] = co[1] = 0.0;
+    // A operands of GEMM2: e (Hessian weights; PAIR: pair sums) and eg (PPn
+    // gradient weights; PAIR: pair differences); fourfold: E of each group
+    double e[2], eg[2], E[QUAD ? 4 : 1][2];
+    // S of the chunk at Pc: cs[0] (PAIR: even half sums), cs[1] (odd ones);
+    // fourfold: the part of each group
+    auto gemm1 = [&](const double *Pc, double (&cs)[QUAD ? 4 : 2][2]) {
+#pragma unroll
+        for (int q = 0; q < (QUAD ? 4 : 2); q++)
+            cs[q][0] = cs[q][1] = 0.0;
         const double *B1 = Pc + offA;
 #pragma unroll
-        for (int k2 = 0; k2 < 2 * KSL; k2++) {
-            if (PAIR && k2 >= 2 * NBE)
-                dmma8x8x4(co, aA[k2], B1[k2 * 4]);
+        for (int k2 = 0; k2 < K4; k2++) {
+            if constexpr (QUAD)
+                dmma8x8x4(cs[(k2 >= QG.k4[1]) + (k2 >= QG.k4[2]) + (k2 >= QG.k4[3])], aA[k2], B1[k2 * 4]);
+            else if (PAIR && k2 >= 2 * NBE)
+                dmma8x8x4(cs[1], aA[k2], B1[k2 * 4]);
             else if (NBK > 0 || k2 * 4 < nb)
-                dmma8x8x4(cs, aA[k2], B1[k2 * 4]);
+                dmma8x8x4(cs[0], aA[k2], B1[k2 * 4]);
         }
     };
-    // its weights: e (Hessian weights; PAIR: pair sums) and eg (PPn gradient
-    // weights; PAIR: pair differences)
-    auto weights = [&](const double *Pc, const double (&cs)[2], const double (&co)[2]) {
+    auto weights = [&](const double *Pc, const double (&cg)[QUAD ? 4 : 2][2]) {
         const double w0 = Pc[wOff], w1 = Pc[wOff + 1];
-        if constexpr (PAIR != 0) {
+        const double(&cs)[2] = cg[0];
+        const double(&co)[2] = cg[1];
+        if constexpr (QUAD) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                // the exponents of phi, phi + pi, -phi, pi - phi
+                const double a = __dadd_rn(cg[0][h], cg[1][h]), b = __dadd_rn(cg[2][h], cg[3][h]);
+                const double c = __dsub_rn(cg[0][h], cg[1][h]), d = __dsub_rn(cg[2][h], cg[3][h]);
+                const double sv[4] = {__dadd_rn(a, b), __dsub_rn(a, b), __dadd_rn(c, d), __dsub_rn(c, d)};
+                double y[4];
+                fast_exp_n<4>(y, sv, exptab, invL, L1, L2);
+                const double w = h ? w1 : w0;
+                const double p = __dadd_rn(y[0], y[1]), q = __dadd_rn(y[2], y[3]);
+                const double r = __dsub_rn(y[0], y[1]), t = __dsub_rn(y[2], y[3]);
+                E[0][h] = __dmul_rn(w, __dadd_rn(p, q));
+                E[1][h] = __dmul_rn(w, __dsub_rn(p, q));
+                E[2][h] = __dmul_rn(w, __dadd_rn(r, t));
+                E[3][h] = __dmul_rn(w, __dsub_rn(r, t));
+            }
+            facc = __dadd_rn(facc, __dadd_rn(E[0][0], E[0][1]));
+        } else if constexpr (PAIR != 0) {
             double sv[4], y[4];
 #pragma unroll
             for (int h = 0; h < 2; h++) {
@@ -2134,7 +2238,11 @@ __device__ __noinline__ bool phase_a_rows8(const PhaseA x, bool active, unsigned
                     const bool hess = (PPN == 0) || nt < NTH;
                     const int col = hess ? nb + nt * 8 : (nt - NTH) * 8;
                     const bool useE = PAIR ? (nt < NTE) : hess;
-                    dmma8x8x4(acc[nt], useE ? e[h] : eg[h], B2[col + h * ldP]);
+                    if constexpr (QUAD)
+                        dmma8x8x4(acc[nt], E[(nt >= QG.tile[1]) + (nt >= QG.tile[2]) + (nt >= QG.tile[3])][h],
+                                  B2[col + h * ldP]);
+                    else
+                        dmma8x8x4(acc[nt], useE ? e[h] : eg[h], B2[col + h * ldP]);
                 }
             }
         }
@@ -2143,10 +2251,10 @@ __device__ __noinline__ bool phase_a_rows8(const PhaseA x, bool active, unsigned
         for (int c = 0; c < DEPTH && c < nchunks; c++)
             load_chunk(c, c);
     bool ok = wait_full(0);
-    double cs[2], co[2];
+    double cs[QUAD ? 4 : 2][2];
     if (active && ok) {
-        gemm1(sP, cs, co);
-        weights(sP, cs, co);
+        gemm1(sP, cs);
+        weights(sP, cs);
     }
     int bc = 0;   // buffer of chunk c
     for (int c = 0; c < nchunks; c++) {
@@ -2171,9 +2279,9 @@ __device__ __noinline__ bool phase_a_rows8(const PhaseA x, bool active, unsigned
                 if (!__all_sync(0xffffffffu, ok))
                     break;
                 if (active) {
-                    gemm1(Pn, cs, co);
+                    gemm1(Pn, cs);
                     gemm2(Pc);
-                    weights(Pn, cs, co);
+                    weights(Pn, cs);
                 }
             } else if (active) {
                 gemm2(Pc);
@@ -2189,8 +2297,8 @@ __device__ __noinline__ bool phase_a_rows8(const PhaseA x, bool active, unsigned
                 if (!__all_sync(0xffffffffu, ok))
                     break;
                 if (active) {
-                    gemm1(Pn, cs, co);
-                    weights(Pn, cs, co);
+                    gemm1(Pn, cs);
+                    weights(Pn, cs);
                 }
             }
         }
@@ -2383,34 +2491,10 @@ __global__ void __launch_bounds__(NW * 32, (NTF > 0 && !MIX && NW == 8) ? 2 : 1)
         if constexpr (R8) {
             const int s8 = (warp >> 2) * 8 + (lane & 7);
             const bool active = __any_sync(0xffffffffu, L.ints[s8 * SI_N + SI_STATE] != S_IDLE);
-            PhaseA x;
-            x.offAlpha = a.offAlpha;
-            x.offScal = a.offScal;
-            x.offFpart = a.offFpart;
-            x.offP = a.offP;
-            x.offG = a.offG;
-            x.offExp = a.offExp;
-            x.offBar = a.offBar;
-            x.ldv = ldv;
-            x.ldG = ldG;
-            x.ntq = a.ntq;
-            x.nb = pb.nb;
-            x.ldP = pb.ldP;
-            x.K2p = pb.K2p;
-            x.nchunks = pb.nqp / 32;
-            x.P = pb.P;
-            x.binv = pb.binv;
-            x.invL = a.ex.invL;
-            x.L1 = a.ex.L1;
-            x.L2 = a.ex.L2;
-            x.err = a.err;
-            if (!phase_a_rows8<NTF, PPN, NT, NBK, PAIR, NW>(x, active, mbPhase))
+            const PhaseA x = make_phase_a(a, pb);
+            if (!phase_a_rows8<NTF, PPN, NT, NBK, PAIR, NW, NX>(x, active, mbPhase))
                 return;   // a staged chunk never arrived (error recorded)
-            // each buffer's barriers went through a phase per chunk it held
-            constexpr int DEPTH = (NW == 16) ? 3 : 2;
-            for (int b = 0; b < DEPTH; b++)
-                if (((x.nchunks - b + DEPTH - 1) / DEPTH) & 1)
-                    mbPhase ^= 9u << b;
+            advance_phases<NW == 16 ? 3 : 2>(mbPhase, x.nchunks);
         } else if constexpr (NTF > 0) {
             if (!phase_a_fused<NTF, PPN, NT, NBK, MIX, PAIR>(a, pb, L, tid, lane, warp, mbPhase))
                 return;   // a staged chunk never arrived (error recorded)
@@ -2624,7 +2708,9 @@ __device__ void screen_logic(const NewtonArgs &a, const NewtonProblem &pb, Layou
     }
 }
 
-template <int NT, int NBK>
+// NQ > 0: the fourfold layout of NQ moments (NBK unused; 16 slots per CTA), else
+// direction pairs (32 slots).
+template <int NT, int NBK, int NQ>
 __global__ void __launch_bounds__(256, 2) screen_kernel(const __grid_constant__ NewtonArgs a)
 {
     constexpr int kThreads = 256, kWarps = 8;
@@ -2656,8 +2742,10 @@ __global__ void __launch_bounds__(256, 2) screen_kernel(const __grid_constant__ 
     for (int i = tid; i < T * SC_N; i += kThreads)
         L.scal[i] = 0.0;
     if (tid == 0) {
-        for (int b = 0; b < 3; b++)
+        for (int b = 0; b < 3; b++) {
             mbar_init(&L.bar[b], 1);
+            mbar_init(&L.bar[3 + b], kWarps);
+        }
         mbar_init_fence();
         repValid = 0;
     }
@@ -2775,8 +2863,16 @@ __global__ void __launch_bounds__(256, 2) screen_kernel(const __grid_constant__ 
             if (L.ints[s * SI_N + SI_STATE] == S_NEW)
                 init_slot(a, pb, L, s, lane, ldv);
         __syncthreads();
-        if (!phase_a_fused<8, 0, NT, NBK, 0, 1>(a, pb, L, tid, lane, warp, mbPhase))
-            return;   // a staged chunk never arrived (error recorded)
+        if constexpr (NQ > 0) {
+            const bool active = (warp >> 2) * 8 < filled;
+            const PhaseA x = make_phase_a(a, pb);
+            if (!phase_a_rows8<8, 0, NT, 1, kQuadScreen, 8, NQ>(x, active, mbPhase))
+                return;   // a staged chunk never arrived (error recorded)
+            advance_phases<2>(mbPhase, x.nchunks);
+        } else {
+            if (!phase_a_fused<8, 0, NT, NBK, 0, 1>(a, pb, L, tid, lane, warp, mbPhase))
+                return;
+        }
         for (;;) {
             int s = 0;
             if (lane == 0)
@@ -2828,10 +2924,10 @@ __global__ void screen_gate_kernel(const int *iters, int first, int count, int *
         atomicAdd(out, v);
 }
 
-template <int NT, int NBK>
+template <int NT, int NBK, int NQ>
 cudaError_t screen_run(const NewtonArgs &a, int grid, cudaStream_t stream, int mode, int *occ)
 {
-    auto *k = screen_kernel<NT, NBK>;
+    auto *k = screen_kernel<NT, NBK, NQ>;
     if (mode == 1)
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smemBytes);
     if (mode == 2) {
