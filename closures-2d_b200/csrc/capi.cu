@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "flux.cuh"
 #include "newton.cuh"
+#include "readback.h"
 
 using namespace clb;
 
@@ -646,6 +647,7 @@ struct cl_ctx {
     DevStats *dStats = nullptr;
     int *dErr = nullptr;
     int *hErr = nullptr;              // pinned [2]
+    clb::ReadBack readback;           // cl_get_state
     int *dIters = nullptr;            // [C] iterations of each cell in the last stage
     cl_mlp *warm = nullptr;           // learned warm start (null: previous stage's alpha)
     int warmMinIters = 0;             // > 0: predict only cells whose previous stage took this many iterations
@@ -1432,9 +1434,9 @@ int cl_get_state(cl_ctx *ctx, double *moments, double *alpha)
     size_t bytes = (size_t)ctx->C * ctx->n * 8;
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     if (moments)
-        CUDA_TRY(ctx, cudaMemcpy(moments, ctx->dMom, bytes, cudaMemcpyDeviceToHost));
+        CUDA_TRY(ctx, ctx->readback.copy(moments, ctx->dMom, bytes));
     if (alpha)
-        CUDA_TRY(ctx, cudaMemcpy(alpha, ctx->dAlpha, bytes, cudaMemcpyDeviceToHost));
+        CUDA_TRY(ctx, ctx->readback.copy(alpha, ctx->dAlpha, bytes));
     return CL_OK;
 }
 

@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "flux.cuh"
+#include "readback.h"
 
 using namespace clb;
 
@@ -638,6 +639,7 @@ struct cl_pn {
     // cl_pn_step_host: upload and readback streams and their events (created on first use)
     cudaStream_t up = nullptr, down = nullptr;
     cudaEvent_t evStart = nullptr, evUp[kPnMaxBands] = {}, evDone[kPnMaxBands] = {};
+    clb::ReadBack readback;   // cl_pn_get_state
 };
 
 static int pn_fail(cl_pn *p, int rc)
@@ -950,7 +952,7 @@ int cl_pn_get_state(cl_pn *p, double *moments)
     if (!p || !moments)
         return CL_ERR_ARG;
     PN_TRY(p, cudaStreamSynchronize(p->stream));
-    PN_TRY(p, cudaMemcpy(moments, p->cur, (size_t)p->C * p->n * 8, cudaMemcpyDeviceToHost));
+    PN_TRY(p, p->readback.copy(moments, p->cur, (size_t)p->C * p->n * 8));
     return CL_OK;
 }
 
