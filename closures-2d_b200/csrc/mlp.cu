@@ -613,8 +613,8 @@ struct cl_mlp {
     float *mean = nullptr, *stdv = nullptr;  // device [n]
     std::vector<float> hmean, hstd;
     int adamStep = 0;
-    // work buffers (grow only)
-    size_t cap = 0;
+    // work buffers (grow only): rows of the forward pass, and of the backward
+    size_t cap = 0, capBack = 0;
     // inputs [rows x round8(n)] and activations [rows x round8(width)], zero
     // padded; dZ of the layer at hand and of the one below, row stride wp
     __nv_bfloat16 *X = nullptr, *Act[kLayers] = {}, *dZ16[2] = {};
@@ -636,12 +636,10 @@ struct cl_mlp {
 
 constexpr int kLossSteps = 256;   // training steps between readbacks of the loss
 
-static void mlp_free_work(cl_mlp *m)
+static void mlp_free_back(cl_mlp *m)
 {
-    cudaFree(m->X);
     cudaFree(m->T);
     cudaFree(m->loss);
-    m->X = nullptr;
     m->T = m->loss = nullptr;
     for (int h = 0; h < 2; h++) {
         cudaFree(m->dZ16[h]);
@@ -649,6 +647,14 @@ static void mlp_free_work(cl_mlp *m)
         m->dZ16[h] = nullptr;
         m->dZ[h] = nullptr;
     }
+    m->capBack = 0;
+}
+
+static void mlp_free_work(cl_mlp *m)
+{
+    mlp_free_back(m);
+    cudaFree(m->X);
+    m->X = nullptr;
     for (int l = 0; l < kLayers; l++) {
         cudaFree(m->Act[l]);
         cudaFree(m->Z[l]);
@@ -658,29 +664,45 @@ static void mlp_free_work(cl_mlp *m)
     m->cap = 0;
 }
 
-static int mlp_reserve(cl_mlp *m, size_t rows)
+// padding columns stay zero: they are operands of the GEMMs
+template <class T>
+static bool mlp_zeroed(T **p, size_t cnt)
 {
-    if (rows <= m->cap)
-        return CL_OK;
-    mlp_free_work(m);
+    return cudaMalloc(p, cnt * sizeof(T)) == cudaSuccess && cudaMemset(*p, 0, cnt * sizeof(T)) == cudaSuccess;
+}
+
+// Work buffers for `rows` rows; those of the backward pass (a third of the
+// whole, 0.8 GB at 131072 x 512) only where it runs.
+static int mlp_reserve(cl_mlp *m, size_t rows, bool back)
+{
     const size_t w = (size_t)(m->width > m->n ? m->width : m->n), wp = (size_t)round8((int)w);
-    // padding columns stay zero: they are operands of the GEMMs
-    auto zeroed = [](auto **p, size_t cnt) {
-        return cudaMalloc(p, cnt * sizeof(**p)) == cudaSuccess && cudaMemset(*p, 0, cnt * sizeof(**p)) == cudaSuccess;
-    };
-    bool ok = zeroed(&m->X, rows * round8(m->n)) && cudaMalloc(&m->T, rows * m->n * sizeof(float)) == cudaSuccess &&
-              cudaMalloc(&m->loss, (rows * m->n / 256 + 2) * sizeof(float)) == cudaSuccess;
-    for (int h = 0; h < 2 && ok; h++)
-        ok = zeroed(&m->dZ16[h], rows * wp) && zeroed(&m->dZ[h], rows * wp);
-    for (int l = 0; l < kLayers && ok; l++)
-        ok = zeroed(&m->Act[l], rows * wp) && cudaMalloc(&m->Z[l], rows * w * sizeof(float)) == cudaSuccess;
+    const bool grow = rows > m->cap, growBack = back && rows > m->capBack;
+    bool ok = true;
+    if (grow) {
+        mlp_free_work(m);
+        ok = mlp_zeroed(&m->X, rows * round8(m->n));
+        for (int l = 0; l < kLayers && ok; l++)
+            ok = mlp_zeroed(&m->Act[l], rows * wp) && cudaMalloc(&m->Z[l], rows * w * sizeof(float)) == cudaSuccess;
+    }
+    if (growBack && ok) {
+        mlp_free_back(m);
+        ok = cudaMalloc(&m->T, rows * m->n * sizeof(float)) == cudaSuccess &&
+             cudaMalloc(&m->loss, (rows * m->n / 256 + 2) * sizeof(float)) == cudaSuccess;
+        for (int h = 0; h < 2 && ok; h++)
+            ok = mlp_zeroed(&m->dZ16[h], rows * wp) && mlp_zeroed(&m->dZ[h], rows * wp);
+    }
+    if (!grow && !growBack)
+        return CL_OK;
     ok = ok && cudaDeviceSynchronize() == cudaSuccess;   // the fills, before work on other streams
     if (!ok) {
         mlp_free_work(m);
         m->err = "MLP work buffer allocation failed";
         return CL_ERR_CUDA;
     }
-    m->cap = rows;
+    if (grow)
+        m->cap = rows;
+    if (growBack)
+        m->capBack = rows;
     return CL_OK;
 }
 
@@ -731,9 +753,13 @@ static float loss_value(const float *part, int parts, int total)
 static cudaError_t mlp_backward(cl_mlp *m, int rows, float *loss)
 {
     const int n = m->n, total = rows * n;
+    // on the current device, whichever it is
+    cudaError_t e = cudaFuncSetAttribute(backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBackSmem);
+    if (e != cudaSuccess)
+        return e;
     mse_grad_kernel<<<loss_parts(m, rows), 256, 0, m->stream>>>(m->Z[kLayers - 1], m->T, m->dZ16[0], m->dZ[0], total, n,
                                                                 round8(n), 1.0f / (float)total, loss);
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     for (int l = kLayers - 1, h = 0; l >= 0 && e == cudaSuccess; l--, h ^= 1) {
         BackArgs a;
         a.rows = rows;
@@ -755,13 +781,6 @@ static cudaError_t mlp_backward(cl_mlp *m, int rows, float *loss)
         a.tilesW = tiles(a.K, a.N);
         a.tilesB = (a.N + 31) / 32;
         const int grid = a.tilesW + a.tilesB + (l > 0 ? tiles(rows, a.K) : 0);
-        static bool attr = false;
-        if (!attr) {
-            e = cudaFuncSetAttribute(backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBackSmem);
-            if (e != cudaSuccess)
-                return e;
-            attr = true;
-        }
         backward_kernel<<<grid, 256, kBackSmem, m->stream>>>(a);
         e = cudaGetLastError();
     }
@@ -899,7 +918,7 @@ int cl_mlp_train(cl_mlp *m, const double *d_u, const double *d_alpha, int count,
 {
     if (!m || !d_u || !d_alpha || count < batch || batch < 1 || steps < 0)
         return CL_ERR_ARG;
-    int rc = mlp_reserve(m, batch);
+    int rc = mlp_reserve(m, batch, true);
     if (rc)
         return rc;
     const int n = m->n, np = round8(n), parts = loss_parts(m, batch);
@@ -1006,7 +1025,7 @@ int cl_mlp_predict(cl_mlp *m, const double *d_u, double *d_alpha, int count, int
         return CL_OK;
     cudaStream_t st = stream ? (cudaStream_t)stream : m->stream;
     const int chunk = 1 << 18;
-    int rc = mlp_reserve(m, count < chunk ? count : chunk);
+    int rc = mlp_reserve(m, count < chunk ? count : chunk, false);
     if (rc)
         return rc;
     cudaStream_t keep = m->stream;
@@ -1054,7 +1073,7 @@ int cl_mlp_predict_selected(cl_mlp *m, const double *d_u, const int *d_iters, in
         return CL_OK;
     cudaStream_t st = stream ? (cudaStream_t)stream : m->stream;
     const int chunk = 1 << 18;
-    int rc = mlp_reserve(m, count < chunk ? count : chunk);
+    int rc = mlp_reserve(m, count < chunk ? count : chunk, false);
     if (rc)
         return rc;
     if (!m->sel || m->selCap < (size_t)count) {
@@ -1125,7 +1144,7 @@ int cl_mlp_loss_and_grads(cl_mlp *m, const double *u, const double *alpha, int r
 {
     if (!m || !u || !alpha || rows < 1)
         return CL_ERR_ARG;
-    int rc = mlp_reserve(m, rows);
+    int rc = mlp_reserve(m, rows, true);
     if (rc)
         return rc;
     const int n = m->n;
@@ -1198,5 +1217,5 @@ int cl_mlp_set_params(cl_mlp *m, float *const *W, float *const *b)
 int clb_mlp_reserve_for(cl_mlp *m, size_t rows)
 {
     const size_t chunk = 1 << 18;
-    return mlp_reserve(m, rows < chunk ? rows : chunk);
+    return mlp_reserve(m, rows < chunk ? rows : chunk, false);
 }
