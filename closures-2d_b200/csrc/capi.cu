@@ -982,8 +982,11 @@ int cl_create(const cl_grid *grid, const cl_options *opts, const cl_angular *ang
     if (const size_t fd = flux_split_doubles(f)) {
         if (cudaMalloc(&ctx->dFluxF, fd * sizeof(double)) != cudaSuccess ||
             cudaMalloc(&ctx->dTileRun, (size_t)f.tilesX * f.tilesY * sizeof(int)) != cudaSuccess) {
-            ctx->err = "device allocation failed";
-            return ctx_fail(ctx, CL_ERR_CUDA);
+            // no room: the direction loops stay whole
+            cudaGetLastError();
+            cudaFree(ctx->dFluxF);
+            ctx->dFluxF = nullptr;
+            ctx->dTileRun = nullptr;
         }
         f.F = ctx->dFluxF;
         f.tileRun = ctx->dTileRun;
