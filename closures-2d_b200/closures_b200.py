@@ -472,7 +472,7 @@ class Context:
 
 
 class MultiSolver:
-    """Several moment orders at one quadrature order, one persistent launch."""
+    """Several moment orders at one quadrature order, a launch per order on forked streams."""
 
     def __init__(self, orders, quad_order, use_gaunt, options):
         self._m = C.c_void_p()

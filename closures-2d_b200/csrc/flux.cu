@@ -420,8 +420,8 @@ __global__ void __launch_bounds__(kFluxThreads, 1) flux_kernel(const __grid_cons
 // Projection and update of the SPLIT form: a warp per 16 cells of a tile, the
 // chunks in order.  The chain over the chunks is short (a few MMAs each), so
 // the loads decide: F of the CTA's 64 cells and the basis rows come through a
-// ring of kProjStages chunks of asynchronous copies (read straight from L2 they
-// took 80 us for 57 chunks).
+// ring of kProjStages chunks of asynchronous copies: 36 us for 57 chunks, 80 us
+// with the loads read straight from L2.
 constexpr int kProjWarps = 4, kProjCells = 16 * kProjWarps, kProjStages = 6;
 constexpr int kProjLd = kProjCells + 4;   // % 16 == 4: conflict-free fragment loads
 template <int PAIR>

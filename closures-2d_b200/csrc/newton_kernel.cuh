@@ -10,11 +10,11 @@
 // B200 mapping.  A CTA owns T "slots" (cells in flight).  Each round every
 // slot needs one evaluation of f, g and H at its current alpha; the rounds are
 // batched contractions over the quadrature on the FP64 tensor cores (DMMA
-// m16n8k8):
+// m8n8k4; m16n8k8 with mixed precision):
 //   S[T x kq]  = alpha[T x nb] . P[kq x nb]^T            (alpha.m per q)
 //   E          = w * exp(S)          (Mn)   or the PPn weights
 //   G[T x K]  += E[T x kq] . Phess[kq x K]               (Hessian columns)
-// with the basis streamed through shared memory in q-chunks by cp.async.
+// with the basis streamed through shared memory in q-chunks by bulk async copies.
 // Then one warp per slot finishes the Newton logic in FP64: H from G (the
 // Gaunt contraction of fobj.cpp:130-144 or the packed products), Cholesky,
 // Hager/Higham 1-norm condition estimate (the quantity dpocon returns),
