@@ -32,7 +32,12 @@ int plan_newton(NewtonArgs &a)
     a.ldv = nbMax + 4;
     a.ldE = a.kq + 4;
     a.ldG = K2tot + 4;
-    a.ldh = (nMax | 1) + 1;   // even: 16-byte row pairs for the broadcast loads
+    // even: 16-byte row pairs for the broadcast loads; half of it odd: a column's
+    // entries, or eight rows' pairs, spread over the banks (with 16 all 15 rows
+    // of M4 fell in one: a step of 200 x 200 cells 3.13 ms, with 18 2.97)
+    a.ldh = (nMax | 1) + 1;
+    if (a.ldh % 4 == 0)
+        a.ldh += 2;
     const int T = a.T;
     int off = 0;
     auto take = [&](int ndoubles) {
