@@ -9,6 +9,13 @@ constexpr int kThreads = 256;        // 8 warps per CTA
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxN = 32;            // moments per cell handled by one warp (order <= 6)
 constexpr int kNumReg = 5;
+
+// Sets a kernel's dynamic shared-memory limit on the current device to `bytes`
+// if it is lower.  Never lowers it: solvers of different orders and tables
+// share kernel instances, each with a plan of its own size, and a launch above
+// the limit in force is refused.
+cudaError_t raise_smem_limit(const void *kernel, int bytes);
+
 // change-of-basis working state of one Newton slot in global memory: the
 // basis T and the rows of L^-1 ([kMaxN][kMaxN] each), then alphaP, the
 // line-search alphaM and step, and 1/T_ii ([kMaxN] each)

@@ -621,17 +621,15 @@ int plan_flux(FluxArgs &f)
 
 cudaError_t prepare_flux(const FluxArgs &f)
 {
-    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = f.paired ? cudaFuncSetAttribute(flux_kernel<1, 0>, attr, f.smemBytes)
-                             : cudaFuncSetAttribute(flux_kernel<0, 0>, attr, f.smemBytes);
+    cudaError_t e = raise_smem_limit(f.paired ? (const void *)flux_kernel<1, 0> : (const void *)flux_kernel<0, 0>,
+                                     f.smemBytes);
     if (e != cudaSuccess)
         return e;
-    e = f.paired ? cudaFuncSetAttribute(flux_kernel<1, 1>, attr, f.smemBytes)
-                 : cudaFuncSetAttribute(flux_kernel<0, 1>, attr, f.smemBytes);
+    e = raise_smem_limit(f.paired ? (const void *)flux_kernel<1, 1> : (const void *)flux_kernel<0, 1>, f.smemBytes);
     if (e != cudaSuccess)
         return e;
-    return f.paired ? cudaFuncSetAttribute(flux_project_kernel<1>, attr, project_smem(f))
-                    : cudaFuncSetAttribute(flux_project_kernel<0>, attr, project_smem(f));
+    return raise_smem_limit(f.paired ? (const void *)flux_project_kernel<1> : (const void *)flux_project_kernel<0>,
+                            project_smem(f));
 }
 
 // Shares of the direction loop for `tiles` tiles on `sms` SMs (one CTA each):

@@ -821,7 +821,7 @@ int cl_pn_create(const cl_grid *grid, const cl_pn_setup *setup, const double *si
         units = (long long)((grid->nx + kTI - 1) / kTI) * ((grid->ny + kTJ - 1) / kTJ);
     else
         units = ((long long)grid->nx * grid->ny + kPnWarps - 1) / kPnWarps;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = raise_smem_limit(fn, (int)smem);
     int occ = 0;
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem);

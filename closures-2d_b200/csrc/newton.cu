@@ -6,8 +6,20 @@
 
 #include <cfloat>
 #include <cmath>
+#include <mutex>
 
 namespace clb {
+
+cudaError_t raise_smem_limit(const void *kernel, int bytes)
+{
+    static std::mutex m;   // two threads' reads and writes in turn
+    std::lock_guard<std::mutex> lock(m);
+    cudaFuncAttributes at;
+    const cudaError_t e = cudaFuncGetAttributes(&at, kernel);
+    if (e != cudaSuccess || at.maxDynamicSharedSizeBytes >= bytes)
+        return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
 
 int plan_newton(NewtonArgs &a)
 {

@@ -2929,7 +2929,7 @@ cudaError_t screen_run(const NewtonArgs &a, int grid, cudaStream_t stream, int m
 {
     auto *k = screen_kernel<NT, NBK, NQ>;
     if (mode == 1)
-        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smemBytes);
+        return raise_smem_limit((const void *)k, a.smemBytes);
     if (mode == 2) {
         int b = 0;
         cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, 256, a.smemBytes);
@@ -2947,7 +2947,7 @@ cudaError_t newton_run(const NewtonArgs &a, int grid, cudaStream_t stream, int m
 {
     auto *k = newton_kernel<TPW, NTF, PPN, NT, NBK, MIX, PAIR, NW, NX>;
     if (mode == 1)
-        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smemBytes);
+        return raise_smem_limit((const void *)k, a.smemBytes);
     if (mode == 2) {
         int b = 0;
         cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, NW * 32, a.smemBytes);
