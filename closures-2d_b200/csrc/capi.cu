@@ -1173,7 +1173,7 @@ static cudaError_t enqueue_stage(cl_ctx *ctx, int stage, double dt, double dx, d
 {
     cudaError_t e;
     if (ghostCopy) {
-        if ((e = launch_ghost_periodic(ctx->dMom, ctx->n, ctx->NX, ctx->NY, ctx->stream)) != cudaSuccess)
+        if ((e = launch_ghost_periodic(ctx->dMom, ctx->dMom, ctx->n, ctx->NX, ctx->NY, ctx->stream)) != cudaSuccess)
             return e;
         *nk += 2;
     }
@@ -1290,7 +1290,7 @@ int cl_step_timed(cl_ctx *ctx, double dt, double dx, double dy, float *ms)
     for (int stage = 0; stage < 2 && e == cudaSuccess; stage++) {
         cudaEventRecord(ev[3 * stage], ctx->stream);
         if (periodic) {
-            e = launch_ghost_periodic(ctx->dMom, ctx->n, ctx->NX, ctx->NY, ctx->stream);
+            e = launch_ghost_periodic(ctx->dMom, ctx->dMom, ctx->n, ctx->NX, ctx->NY, ctx->stream);
             nk += 2;
         }
         if (ctx->warm && e == cudaSuccess) {
@@ -1505,7 +1505,7 @@ int cl_step_host(cl_ctx *ctx, double dt, double dx, double dy, double *moments, 
         if (stage == 0 && bands == 1)
             run(cudaStreamWaitEvent(S, ctx->evBand[0], 0));
         if (periodic) {
-            run(launch_ghost_periodic(ctx->dMom, ctx->n, ctx->NX, ctx->NY, S));
+            run(launch_ghost_periodic(ctx->dMom, ctx->dMom, ctx->n, ctx->NX, ctx->NY, S));
             nk += 2;
         }
         if (ctx->warm && e == cudaSuccess) {

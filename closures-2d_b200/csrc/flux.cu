@@ -502,32 +502,31 @@ static int project_smem(const FluxArgs &f)
     return kProjStages * (kQ * kProjLd + (f.paired ? kQ / 2 : kQ) * f.ldPf) * (int)sizeof(double);
 }
 
-__global__ void ghost_periodic_kernel(double *m, int n, int NX, int NY)
+// momopt_boundaries.cpp:190-223: x strips over interior j, then y strips over
+// interior i (corners untouched).  One thread copies all four cells of a line,
+// in the reference's order: on an axis of one cell the outer ghosts copy inner
+// ones, the first of them (cell 0 <- cell 1) as it was filled by the copy
+// before this one, held by `prev`.
+__device__ __forceinline__ void wrap_line(double *m, const double *prev, size_t at, size_t step, int N)
 {
-    // momopt_boundaries.cpp:190-223: x strips over interior j, then y strips
-    // over interior i (corners untouched).
-    const int ny = NY - 4, nx = NX - 4;
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    int totalX = 2 * ny * n, totalY = 2 * nx * n;
-    if (idx < totalX) {
-        int k = idx % n, r = idx / n;
-        int j = 2 + r % ny, i = r / ny;   // i in {0,1}
-        m[((size_t)(0 + i) * NY + j) * n + k] = m[((size_t)(NX - 4 + i) * NY + j) * n + k];
-        m[((size_t)(NX - 2 + i) * NY + j) * n + k] = m[((size_t)(2 + i) * NY + j) * n + k];
-    }
+    m[at] = (N - 4 < 2 ? prev : m)[at + (N - 4) * step];
+    m[at + (N - 2) * step] = m[at + 2 * step];
+    m[at + step] = m[at + (N - 3) * step];
+    m[at + (N - 1) * step] = m[at + 3 * step];
 }
 
-__global__ void ghost_periodic_y_kernel(double *m, int n, int NX, int NY)
+__global__ void ghost_periodic_kernel(double *m, const double *prev, int n, int NX, int NY)
 {
-    const int nx = NX - 4;
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    int total = 2 * nx * n;
-    if (idx < total) {
-        int k = idx % n, r = idx / n;
-        int j = r % 2, i = 2 + r / 2;
-        m[((size_t)i * NY + 0 + j) * n + k] = m[((size_t)i * NY + NY - 4 + j) * n + k];
-        m[((size_t)i * NY + NY - 2 + j) * n + k] = m[((size_t)i * NY + 2 + j) * n + k];
-    }
+    const size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x, line = (size_t)NY * n;
+    if (idx < (size_t)(NY - 4) * n)
+        wrap_line(m, prev, 2 * (size_t)n + idx, line, NX);
+}
+
+__global__ void ghost_periodic_y_kernel(double *m, const double *prev, int n, int NX, int NY)
+{
+    const size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (idx < (size_t)(NX - 4) * n)
+        wrap_line(m, prev, (2 + idx / n) * NY * n + idx % n, n, NY);
 }
 
 // Node halo (momopt_boundaries.cpp:30-188) for all four sides in one launch:
@@ -696,12 +695,10 @@ cudaError_t launch_flux(const FluxArgs &f, cudaStream_t stream, int *kernels)
 
 int flux_tile_rows(const FluxArgs &) { return TX; }
 
-cudaError_t launch_ghost_periodic(double *moments, int n, int NX, int NY, cudaStream_t stream)
+cudaError_t launch_ghost_periodic(double *moments, const double *prev, int n, int NX, int NY, cudaStream_t stream)
 {
-    int totalX = 2 * (NY - 4) * n;
-    ghost_periodic_kernel<<<(totalX + 255) / 256, 256, 0, stream>>>(moments, n, NX, NY);
-    int totalY = 2 * (NX - 4) * n;
-    ghost_periodic_y_kernel<<<(totalY + 255) / 256, 256, 0, stream>>>(moments, n, NX, NY);
+    ghost_periodic_kernel<<<((NY - 4) * n + 255) / 256, 256, 0, stream>>>(moments, prev, n, NX, NY);
+    ghost_periodic_y_kernel<<<((NX - 4) * n + 255) / 256, 256, 0, stream>>>(moments, prev, n, NX, NY);
     return cudaGetLastError();
 }
 

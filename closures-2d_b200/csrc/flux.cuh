@@ -51,8 +51,10 @@ cudaError_t launch_flux_tiles(const FluxArgs &f, int first, int count, cudaStrea
 // is never shared out); f.tileRun holds one int per tile.
 size_t flux_split_doubles(const FluxArgs &f);
 int flux_tile_rows(const FluxArgs &f);   // interior cells per tile along x
-// duplicateBoundaries (momopt_boundaries.cpp:190-223) on device moments.
-cudaError_t launch_ghost_periodic(double *moments, int n, int NX, int NY, cudaStream_t stream);
+// duplicateBoundaries (momopt_boundaries.cpp:190-223) on device moments; `prev`:
+// the state whose ghosts the last such copy filled (the same one, or the other
+// of two buffers).
+cudaError_t launch_ghost_periodic(double *moments, const double *prev, int n, int NX, int NY, cudaStream_t stream);
 // Halo strips of a node's block: pack (1) the inner strips into p[side] or
 // unpack (0) p[side] into the ghost strips; null sides are skipped.
 struct HaloBuffers {

@@ -50,8 +50,8 @@ struct PnArgs {
     int filteredGhosts;     // bit s: ghost strip of side s holds (filtered) interior values
     double dt, rdx, rdy, dx, dy, initX, initY;
     int rowBegin, rowEnd;   // interior rows (x) of this launch; band starts are multiples of kTI
-    int wrap;               // pn_parity_kernel: 1 reads ghost cells from the interior cells they
-                            // copy (periodic grid), 2 also writes the copies to `in`
+    int wrap;               // pn_parity_kernel: reads ghost cells from the interior cells they copy
+                            // (periodic grid, two cells or more a side) and writes the copies to `in`
 };
 
 __device__ __forceinline__ bool filtered_cell(const PnArgs &a, int i, int j)
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(kParThreads, N <= 6 ? 4 : 2) pn_parity_kernel(
                     continue;
                 const int c = c0 + e / n, k = e % n, gj = j0 - 2 + c;
                 const bool inI = gi >= 2 && gi < a.NX - 2, inJ = gj >= 2 && gj < a.NY - 2;
-                if (a.wrap == 2 && inI != inJ && gi < a.NX && gj < a.NY) {
+                if (a.wrap && inI != inJ && gi < a.NX && gj < a.NY) {
                     double *dst = const_cast<double *>(a.in) + ((size_t)gi * a.NY + gj) * n + k;
 #pragma unroll
                     for (int h = 0; h < V; h++)
@@ -896,14 +896,15 @@ int cl_pn_step(cl_pn *p, double dt, double dx, double dy)
     if (!p)
         return CL_ERR_ARG;
     for (int stage = 1; stage <= 2; stage++) {
-        // periodic ghosts: pn_parity_kernel reads the cells they copy (a
-        // step leaves the state's ghosts as of its first stage)
+        // periodic ghosts: pn_parity_kernel reads the cells they copy, where
+        // those are interior cells (an axis of one cell wraps onto ghosts)
         int wrap = 0;
         if (p->grid.init_cond == 2) {
-            if (p->parityOrder > 0) {
-                wrap = stage == 1 ? 2 : 1;
+            if (p->parityOrder > 0 && p->grid.nx >= 2 && p->grid.ny >= 2) {
+                wrap = 1;
             } else {
-                PN_TRY(p, launch_ghost_periodic(p->cur, p->n, p->NX, p->NY, p->stream));
+                double *other = (p->cur == p->U) ? p->V : p->U;   // filled by the stage before
+                PN_TRY(p, launch_ghost_periodic(p->cur, other, p->n, p->NX, p->NY, p->stream));
                 clb_count_launches(2);
             }
         }
