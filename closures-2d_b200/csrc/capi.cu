@@ -652,8 +652,10 @@ struct cl_ctx {
     cl_mlp *warm = nullptr;           // learned warm start (null: previous stage's alpha)
     int warmMinIters = 0;             // > 0: predict only cells whose previous stage took this many iterations
     double *dAlphaPred = nullptr;     // [C][n] predicted starts when warm is set
-    double *dFluxF = nullptr;         // stencil fluxes of a shared-out direction loop (small grids)
-    int *dTileRun = nullptr;          // whether each tile ran its direction loop
+    // stencil fluxes of a shared-out direction loop (small grids), then whether
+    // each tile ran it
+    double *dFluxF = nullptr;
+    bool fluxRoomTried = false;
     double *dP2M = nullptr, *dAlphaP = nullptr;   // change-of-basis state per cell (opt type 1)
     double *dCbScratch = nullptr;     // working basis per Newton slot (opt type 1)
     NewtonArgs nargs;
@@ -692,6 +694,35 @@ struct cl_ctx {
 extern "C" {
 
 static void update_screen(cl_ctx *ctx);
+
+// The buffer of a shared-out direction loop, where a launch of this grid uses
+// one.  Made with the context, except on grids of one tile: those of batch
+// contexts never step, and a block of device memory takes 0.35 ms, a third of
+// such a context's creation.  Without room, or when the stream is being
+// captured, the loops stay whole.
+static void flux_room(cl_ctx *ctx)
+{
+    FluxArgs &f = ctx->fargs;
+    const size_t tiles = (size_t)f.tilesX * f.tilesY, doubles = flux_split_doubles(f);
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (ctx->fluxRoomTried || doubles == 0 || cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess ||
+        capturing != cudaStreamCaptureStatusNone)
+        return;
+    ctx->fluxRoomTried = true;
+    FluxArgs g = f;
+    if (cudaMalloc(&ctx->dFluxF, doubles * sizeof(double) + tiles * sizeof(int)) == cudaSuccess) {
+        g.F = ctx->dFluxF;
+        g.doublesF = doubles;
+        g.tileRun = (int *)(ctx->dFluxF + doubles);
+        if (prepare_flux(g) == cudaSuccess) {
+            f = g;
+            return;
+        }
+        cudaFree(ctx->dFluxF);
+    }
+    ctx->dFluxF = nullptr;
+    cudaGetLastError();
+}
 
 const char *cl_global_error(void) { return g_global_err.c_str(); }
 
@@ -979,18 +1010,8 @@ int cl_create(const cl_grid *grid, const cl_options *opts, const cl_angular *ang
         return ctx_fail(ctx, CL_ERR_CUDA);
     }
     f.sms = sm_count();
-    if (const size_t fd = flux_split_doubles(f)) {
-        if (cudaMalloc(&ctx->dFluxF, fd * sizeof(double)) != cudaSuccess ||
-            cudaMalloc(&ctx->dTileRun, (size_t)f.tilesX * f.tilesY * sizeof(int)) != cudaSuccess) {
-            // no room: the direction loops stay whole
-            cudaGetLastError();
-            cudaFree(ctx->dFluxF);
-            ctx->dFluxF = nullptr;
-            ctx->dTileRun = nullptr;
-        }
-        f.F = ctx->dFluxF;
-        f.tileRun = ctx->dTileRun;
-    }
+    if (f.tilesX * f.tilesY > 1)
+        flux_room(ctx);
     if (cudaDeviceSynchronize() != cudaSuccess) {
         ctx->err = std::string("set-up: ") + cudaGetErrorString(cudaGetLastError());
         return ctx_fail(ctx, CL_ERR_CUDA);
@@ -1035,7 +1056,6 @@ void cl_destroy(cl_ctx *ctx)
     cudaFree(ctx->dIters);
     cudaFree(ctx->dAlphaPred);
     cudaFree(ctx->dFluxF);
-    cudaFree(ctx->dTileRun);
     cudaFree(ctx->dP2M);
     cudaFree(ctx->dAlphaP);
     cudaFree(ctx->dCbScratch);
@@ -1254,6 +1274,7 @@ int cl_step_async(cl_ctx *ctx, double dt, double dx, double dy)
             cudaGraphDestroy(ctx->graph);
             ctx->graph = nullptr;
         }
+        flux_room(ctx);
         CUDA_TRY(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         int nk = 0;
         cudaError_t e = enqueue_step(ctx, dt, dx, dy, &nk);
@@ -1281,6 +1302,7 @@ int cl_step_timed(cl_ctx *ctx, double dt, double dx, double dy, float *ms)
 {
     if (!ctx || !ms)
         return CL_ERR_ARG;
+    flux_room(ctx);
     cudaEvent_t ev[7];
     for (int i = 0; i < 7; i++)
         CUDA_TRY(ctx, cudaEventCreate(&ev[i]));
@@ -1348,6 +1370,7 @@ int cl_stage(cl_ctx *ctx, int stage, double dt, double dx, double dy)
 {
     if (!ctx || (stage != 1 && stage != 2))
         return CL_ERR_ARG;
+    flux_room(ctx);
     CUDA_TRY(ctx, cudaMemsetAsync(ctx->dQueue + (stage - 1), 0, sizeof(unsigned), ctx->stream));
     int nk = 0;
     cudaError_t e = enqueue_stage(ctx, stage - 1, dt, dx, dy, false, &nk);
@@ -1363,6 +1386,7 @@ int cl_stage_timed(cl_ctx *ctx, int stage, double dt, double dx, double dy, floa
 {
     if (!ctx || !ms || (stage != 1 && stage != 2))
         return CL_ERR_ARG;
+    flux_room(ctx);
     cudaEvent_t ev[3];
     for (int i = 0; i < 3; i++)
         CUDA_TRY(ctx, cudaEventCreate(&ev[i]));
@@ -1478,6 +1502,7 @@ int cl_step_host(cl_ctx *ctx, double dt, double dx, double dy, double *moments, 
         for (int b = 0; b < kHostBands; b++)
             CUDA_TRY(ctx, cudaEventCreateWithFlags(&ctx->evBand[b], cudaEventDisableTiming));
     }
+    flux_room(ctx);
     cudaStream_t S = ctx->stream, X = ctx->copyStream;
     const size_t n = (size_t)ctx->n, C = (size_t)ctx->C, rowBytes = (size_t)ctx->NY * n * 8;
     const bool periodic = ctx->grid.init_cond == 2;

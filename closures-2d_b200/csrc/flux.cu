@@ -622,7 +622,7 @@ cudaError_t prepare_flux(const FluxArgs &f)
 {
     cudaError_t e = raise_smem_limit(f.paired ? (const void *)flux_kernel<1, 0> : (const void *)flux_kernel<0, 0>,
                                      f.smemBytes);
-    if (e != cudaSuccess)
+    if (e != cudaSuccess || !f.F)
         return e;
     e = raise_smem_limit(f.paired ? (const void *)flux_kernel<1, 1> : (const void *)flux_kernel<0, 1>, f.smemBytes);
     if (e != cudaSuccess)
@@ -650,14 +650,21 @@ static int flux_shares(int tiles, int chunks, int sms)
     return best;
 }
 
+static int flux_chunks(const FluxArgs &f) { return f.nqp / (f.paired ? kQ / 2 : kQ); }
+
 size_t flux_split_doubles(const FluxArgs &f)
 {
     // Splitting pays while the tiles fill less than about two waves (the
     // chunk times saved are then a sizeable share), and F has to stay small.
-    const size_t tiles = (size_t)f.tilesX * f.tilesY;
-    const size_t dirs = (size_t)(f.paired ? 2 : 1) * f.nqp;   // whole chunks of either layout
-    const size_t doubles = tiles * dirs * IC;
-    return (tiles <= 2 * (size_t)f.sms && doubles * sizeof(double) <= kSplitBytes) ? doubles : 0;
+    // A step launches the whole grid, cl_step_host two waves one by one.
+    const int tiles = f.tilesX * f.tilesY, chunks = flux_chunks(f);
+    if (tiles > 2 * f.sms)
+        return 0;
+    int most = flux_shares(tiles, chunks, f.sms) > 1 ? tiles : 0;
+    if (most == 0 && tiles == 2 * f.sms && flux_shares(f.sms, chunks, f.sms) > 1)
+        most = f.sms;
+    const size_t doubles = (size_t)most * chunks * kQ * IC;
+    return doubles * sizeof(double) <= kSplitBytes ? doubles : 0;
 }
 
 cudaError_t launch_flux_tiles(const FluxArgs &f, int first, int count, cudaStream_t stream, int *kernels)
@@ -666,7 +673,9 @@ cudaError_t launch_flux_tiles(const FluxArgs &f, int first, int count, cudaStrea
         return cudaErrorInvalidValue;
     FluxArgs g = f;
     g.tileBase = first;
-    const int shares = (f.F && f.tileRun) ? flux_shares(count, f.nqp / (f.paired ? kQ / 2 : kQ), f.sms) : 1;
+    int shares = f.F ? flux_shares(count, flux_chunks(f), f.sms) : 1;
+    if ((size_t)count * flux_chunks(f) * kQ * IC > f.doublesF)
+        shares = 1;
     if (shares > 1) {
         const dim3 grid((unsigned)count, (unsigned)shares);
         const int pgrid = count * (IC / kProjCells), psmem = project_smem(g);

@@ -35,20 +35,22 @@ struct FluxArgs {
     unsigned long long *tilesRun;   // nullable: tiles that ran the chunk loop (non-uniform)
     int skipUniform;                // 1: uniform tiles apply zero flux without the chunk loop
     // direction loop shared out over CTAs (grids of few tiles): stencil
-    // fluxes [tile][chunk][16][256] and whether each tile ran; null: never
+    // fluxes [tile][chunk][16][256] (doublesF of them) and whether each tile
+    // ran; null: never
     double *F;
+    size_t doublesF;
     int *tileRun;
     int sms;                        // SMs of the device
 };
 
 int plan_flux(FluxArgs &f);
-cudaError_t prepare_flux(const FluxArgs &f);
+cudaError_t prepare_flux(const FluxArgs &f);   // with f.F: the shared-out form too
 // *kernels += the kernels launched.
 cudaError_t launch_flux(const FluxArgs &f, cudaStream_t stream, int *kernels);
 // The tiles first .. first + count - 1 only (one launch of a split stage).
 cudaError_t launch_flux_tiles(const FluxArgs &f, int first, int count, cudaStream_t stream, int *kernels);
-// Doubles of f.F that any launch of this grid may use (0: its direction loop
-// is never shared out); f.tileRun holds one int per tile.
+// Doubles of f.F that the launches of this grid use (0: its direction loop is
+// never shared out); f.tileRun holds one int per tile.
 size_t flux_split_doubles(const FluxArgs &f);
 int flux_tile_rows(const FluxArgs &f);   // interior cells per tile along x
 // duplicateBoundaries (momopt_boundaries.cpp:190-223) on device moments; `prev`:
