@@ -632,17 +632,24 @@ cudaError_t prepare_flux(const FluxArgs &f)
 }
 
 // Shares of the direction loop for `tiles` tiles on `sms` SMs (one CTA each):
-// 1, or the number that takes the fewest chunk times, a CTA's start (staging
-// of alpha) counted as one chunk and the pass over F as half a chunk per wave
-// of tiles.
+// the number that takes the fewest chunk times.  A wave of shares costs its
+// chunks and one more for the CTA's start (staging of alpha); the pass over F
+// 0.08 per chunk of the loop, and as much again per wave of tiles.  Against
+// times of 1 to 25 shares on 1 to 296 tiles at 4 to 144 chunks, the choice is
+// within 1 % of the fastest on average and never slower than the whole loop:
+// 16 tiles at 25 chunks 142 -> 42 us, 74 at 57 310 -> 192, 169 at 57 609 ->
+// 448; whole at 120 tiles and 100 chunks (563 us; 6 shares, which a pass over F
+// taken as half a chunk per wave chose, 591), 112 and 57 (309; 323), 256 and
+// 100 (1116; 1140).
 static int flux_shares(int tiles, int chunks, int sms)
 {
     auto waves = [&](int s) { return (tiles * s + sms - 1) / sms; };
     int best = 1;
     double cost = waves(1) * (chunks + 1.0);
     for (int s = 2; s <= chunks && s <= 64; s++) {
-        const double c = waves(s) * ((chunks + s - 1) / s + 1.0) + 1.5 + 0.5 * tiles / sms;
-        if (c < 0.95 * cost) {
+        const double c =
+            waves(s) * ((chunks + s - 1) / s + 1.0) + 0.5 + 0.08 * chunks * (1.0 + (double)tiles / sms);
+        if (c < cost) {
             cost = c;
             best = s;
         }
