@@ -203,6 +203,9 @@ __device__ __forceinline__ void backward_tile(const BackArgs &a, int block, unsi
             for (int h = 0; h < 4; h++) {
                 const int m = m0 + wm + i * 16 + g + ((h & 2) ? 8 : 0);
                 const int nn = n0 + wn + j * 8 + 2 * t + (h & 1);
+                // the padding columns of the next dZ are operands of its products
+                if (!W && m < M && nn >= N && nn < a.ldn)
+                    a.dZnext[(size_t)m * a.ldn + nn] = __float2bfloat16(0.0f);
                 if (m >= M || nn >= N)
                     continue;
                 if (W) {
@@ -664,7 +667,9 @@ static void mlp_free_work(cl_mlp *m)
     m->cap = 0;
 }
 
-// padding columns stay zero: they are operands of the GEMMs
+// padding columns are zero: they are operands of the GEMMs.  Those of X and Act
+// keep their place and stay as filled; dZ16 holds matrices of several strides
+// in turn, whose writers fill their padding.
 template <class T>
 static bool mlp_zeroed(T **p, size_t cnt)
 {
