@@ -192,18 +192,20 @@ static void quad_directions(int r, int Q, int (&q)[4])
     q[3] = level + Q - 1 - k;
 }
 
-// Whether the weights and all `cols` basis columns have the fourfold symmetry
-// (to 1e-12; the library's own quadrature does to 1.4e-14).
-static bool quad_symmetric(int nq, int cols, int ld, const double *w, const double *p)
+// Whether the weights and all `cols` basis columns have the symmetry of `fold`
+// directions, 4 or (phi and phi + pi only) 2, to 1e-12; the library's own
+// quadrature has the fourfold one to 1.4e-14.
+static bool fold_symmetric(int fold, int nq, int cols, int ld, const double *w, const double *p)
 {
     const int Q = (int)std::lround(std::sqrt((double)nq));
     if (Q * Q != nq || Q % 2 != 0)
         return false;
     const std::vector<int> cls = harmonic_classes(cols);
-    for (int r = 0; r < nq / 4; r++) {
-        int q[4];
-        quad_directions(r, Q, q);
-        for (int h = 1; h < 4; h++) {
+    for (int r = 0; r < nq / fold; r++) {
+        int q[4] = {(r / Q) * 2 * Q + r % Q, (r / Q) * 2 * Q + r % Q + Q};
+        if (fold == 4)
+            quad_directions(r, Q, q);
+        for (int h = 1; h < fold; h++) {
             if (!(std::fabs(w[q[h]] - w[q[0]]) <= 1e-12 * std::fabs(w[q[0]])))
                 return false;
             for (int k = 0; k < cols; k++) {
@@ -240,12 +242,13 @@ cudaError_t build_device_basis(DeviceBasis &B, int n, int n2, int nq, int useGau
     if (Q * Q != nq || Q % 2 != 0)
         paired = fluxPaired = 0;
     // the Gaunt orders 3-6 fold four directions into one (phi -> -phi as
-    // well); tables without that symmetry keep one direction per row
-    const int quad = (paired && useGaunt && newton_quad_supported(n)) ? 1 : 0;
-    if (quad && !quad_symmetric(nq, n2, n2, w, p))
-        paired = 0;
+    // well); tables without that symmetry two, or none
+    B.quad = 0;
+    if (paired && useGaunt && newton_quad_supported(n)) {
+        B.quad = fold_symmetric(4, nq, n2, n2, w, p);
+        paired = B.quad || fold_symmetric(2, nq, n2, n2, w, p);
+    }
     B.paired = paired;
-    B.quad = quad && paired;
     const int K2 = useGaunt ? n2 : n * (n + 1) / 2;
     std::vector<unsigned short> prod(n * (n + 1) / 2);
     product_columns(n, prod.data());

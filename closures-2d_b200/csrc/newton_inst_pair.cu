@@ -1,8 +1,9 @@
 // newton_inst_pair.cu -- Mn instances of the folded layouts.  Direction pairs:
-// one per (column tiles, k-steps, moments) of orders 1 and 2 and the direct
-// orders 3 and 4.  Fourfold directions: the Gaunt orders 3-6, where the four
-// column groups pad to fewer MMAs per direction than two (orders 1 and 2: as
-// many).  The moment count is part of the key: the per-slot logic is unrolled
+// one per (column tiles, k-steps, moments) of orders 1 and 2, the direct
+// orders 3 and 4, and the Gaunt orders 3-6 for tables that have no fourfold
+// symmetry (newton_inst_pair_c.cu).  Fourfold directions: the Gaunt orders
+// 3-6, where the four column groups pad to fewer MMAs per direction than two
+// (orders 1 and 2: as many).  The moment count is part of the key: the per-slot logic is unrolled
 // for exactly that many rows.
 #include "newton_kernel.cuh"
 
@@ -10,8 +11,7 @@ namespace clb {
 
 namespace {
 // (tiles, k-steps, n) of the pair layouts: N = 1, 2 -> (2,2,3) (3,2,6), Gaunt or
-// direct; Gaunt N = 3..6 -> (4,2,10) (7,3,15) (9,4,21) (13,4,28), which run
-// fourfold; direct N = 3, 4 -> (7,2,10) (16,3,15).  The pair instances also
+// direct; Gaunt N = 3..6 -> (4,2,10) (7,3,15) (9,4,21) (13,4,28); direct N = 3, 4 -> (7,2,10) (16,3,15).  The pair instances also
 // carry the even tiles and k-steps: E = sum over even degrees of l + 1 columns,
 // or the products of two moments of one parity, padded to 8.
 constexpr int kPairShapes[][3] = {{2, 2, 3}, {3, 2, 6}, {4, 2, 10}, {7, 2, 10}, {7, 3, 15}, {9, 4, 21}, {13, 4, 28},
@@ -45,7 +45,7 @@ bool newton_run_exact_pair(const NewtonArgs &a, int grid, cudaStream_t s, int mo
     CLB_PAIR(7, 2, 10, 4, 1)
     CLB_PAIR(16, 3, 15, 9, 2)
 #undef CLB_PAIR
-    return false;
+    return newton_run_exact_pair_c(a, grid, s, mode, occ, err);
 }
 
 }  // namespace clb

@@ -8,7 +8,7 @@
 namespace clb {
 
 namespace {
-constexpr int kPair4Shapes[][3] = {{16, 3, 15}};
+constexpr int kPair4Shapes[][3] = {{4, 2, 10}, {7, 3, 15}, {9, 4, 21}, {13, 4, 28}, {16, 3, 15}};
 }  // namespace
 
 bool newton_pair4_supported(int nt, int nbk, int n)
@@ -41,7 +41,7 @@ bool newton_run_exact_pair4(const NewtonArgs &a, int grid, cudaStream_t s, int m
         *err = newton_run<1, 16, 0, 16, 3, 0, 16 * 9 + 2, 8, 15>(a, grid, s, mode, occ);
         return true;
     }
-    return false;
+    return newton_run_exact_pair_c(a, grid, s, mode, occ, err);
 }
 
 }  // namespace clb

@@ -1,14 +1,14 @@
 // newton_inst_screen.cu -- the screening pass of K1 (screen_kernel in
 // newton_kernel.cuh): layout planning and its instances, one per (gradient
-// column tiles, k-steps) of the direction-pair layouts: orders 1, 2 and direct
-// 3 -> (2, 2), direct 4 -> (3, 3); and one per Gaunt order 3-6 (fourfold).
+// column tiles, k-steps) of the direction-pair layouts: orders 1-3 -> (2, 2),
+// 4 -> (3, 3), 5 and 6 -> (4, 4); and one per Gaunt order 3-6 (fourfold).
 #include "newton_kernel.cuh"
 
 #include <algorithm>
 
 namespace clb {
 
-bool screen_supported(int nt, int nbk) { return nt == nbk && nt >= 2 && nt <= 3; }
+bool screen_supported(int nt, int nbk) { return nt == nbk && nt >= 2 && nt <= 4; }
 
 int plan_screen(NewtonArgs &a)
 {
@@ -83,6 +83,8 @@ static cudaError_t screen_dispatch(const NewtonArgs &a, int grid, cudaStream_t s
         return screen_run<2, 2, 0>(a, grid, s, mode, occ);
     case 3:
         return screen_run<3, 3, 0>(a, grid, s, mode, occ);
+    case 4:
+        return screen_run<4, 4, 0>(a, grid, s, mode, occ);
     default:
         return cudaErrorInvalidValue;
     }
