@@ -1863,11 +1863,21 @@ static std::mutex g_tune_mutex;
 static std::map<std::string, std::array<int, 3>> g_tune_cache;
 static bool g_tune_file_read = false;
 
+// The key ends in what the layout "pairs" runs for these tables and in the
+// generation of the kernels that were timed: a choice among other kernels is
+// measured again.
+constexpr int kTunedKernels = 2;
+
 static std::string tune_key(const cl_ctx *ctx)
 {
+    int fold = 2;
+    if (ctx->angGaunt && newton_quad_supported(ctx->angN))
+        for (fold = 4; fold > 1; fold /= 2)
+            if (fold_symmetric(fold, ctx->angNq, ctx->angN2, ctx->angN2, ctx->aw.data(), ctx->ap.data()))
+                break;
     char buf[160];
-    snprintf(buf, sizeof(buf), "n%d_n2%d_nq%d_gaunt%d_mt%d_prec%d_opt%d", ctx->angN, ctx->angN2, ctx->angNq,
-             ctx->angGaunt, ctx->opt.moment_type, ctx->opt.precision, ctx->opt.opt_type);
+    snprintf(buf, sizeof(buf), "n%d_n2%d_nq%d_gaunt%d_mt%d_prec%d_opt%d_fold%d_k%d", ctx->angN, ctx->angN2, ctx->angNq,
+             ctx->angGaunt, ctx->opt.moment_type, ctx->opt.precision, ctx->opt.opt_type, fold, kTunedKernels);
     return buf;
 }
 

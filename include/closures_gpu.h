@@ -223,9 +223,10 @@ int cl_set_last_iterations(cl_ctx *ctx, const int *iters);
  * Every candidate is launched once untimed, then timed three times with
  * CUDA events on the context's stream; the median decides.  The choice is
  * applied to the context and cached per (order, quadrature, Gaunt, closure,
- * precision, optimisation type) in the process, and in the file named by
- * the environment variable CL_TUNE_CACHE when set; with use_cache = 1 a
- * cached choice is applied without timing.  Grids below 16384 cells, batch-only
+ * precision, optimisation type, symmetry of the tables) in the process, and
+ * in the file named by the environment variable CL_TUNE_CACHE when set
+ * (entries of a library with other kernels are not taken); with use_cache = 1
+ * a cached choice is applied without timing.  Grids below 16384 cells, batch-only
  * contexts and the change-of-basis types keep the default shape (nothing is
  * timed; out->ncand = 0).  Every candidate computes the same per-cell sums:
  * the two K1 launch shapes give bit-identical results, the two tile layouts
