@@ -408,7 +408,7 @@ cudaError_t build_device_basis(DeviceBasis &B, int n, int n2, int nq, int useGau
         if ((e = upload(&B.hoff, off)) != cudaSuccess) return e;
         if ((e = upload(&B.hidx, idx)) != cudaSuccess) return e;
         if ((e = upload(&B.hval, val)) != cudaSuccess) return e;
-        const int chunks = gaunt_ell_chunks(n), maxGroups = 16 * chunks;
+        const int chunks = gaunt_ell_chunks(n), maxGroups = gaunt_ell_groups(n, goff);
         std::vector<unsigned short> epair(chunks * 64), eidx((size_t)maxGroups * kEllGroup);
         std::vector<double> eval((size_t)maxGroups * kEllGroup);
         std::vector<int> eoff(chunks + 1);
@@ -1851,7 +1851,7 @@ static int apply_shape(cl_ctx *ctx, int nw, int ncontr, int fcontr)
         ctx->B2.release();
     update_screen(ctx);
     invalidate_graph(ctx);
-    ctx->tuning.newton_warps = nw;
+    ctx->tuning.newton_warps = a.nw;
     ctx->tuning.newton_ctas = ctx->nCtas;
     ctx->tuning.newton_contraction = ncontr;
     ctx->tuning.flux_contraction = fcontr;

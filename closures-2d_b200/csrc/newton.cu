@@ -110,6 +110,18 @@ int plan_newton(NewtonArgs &a)
             a.smemBytes = end * 8;
             return 0;
         }
+        // a Gaunt table too long to be staged beside 32 slots (order 6 with
+        // Q = 12: 26 entry groups instead of 12): 16 slots, whose instances
+        // read it through L1 (32,000 vectors 2.4 ms; unfolded, with the
+        // general contractions, 4.0)
+        if (pb.paired && nw == kWarps) {
+            NewtonArgs b = a;
+            b.nw = 4;
+            if (plan_newton(b) == 0) {
+                a = b;
+                return 0;
+            }
+        }
         a.ntf = 0;
         a.ntExact = a.nbk = 0;
         if (a.mixed)

@@ -91,14 +91,9 @@ extern "C" int cl_solve_batch_noalloc(const cl_angular *ang, const cl_options *o
     off = align_up(off + sizeof(int) * (size_t)(nnz ? nnz : 1), 256);
     const size_t offHval = off;
     off = align_up(off + sizeof(double) * (size_t)(nnz ? nnz : 1), 256);
-    // Gaunt table in lane-major chunks; entry groups bounded by the chunk count
-    // times the longest entry list, which the CSR gives
+    // Gaunt table in lane-major chunks
     const int chunks = gaunt ? gaunt_ell_chunks(n) : 0;
-    int maxPer = 0;
-    if (gaunt)
-        for (int r = 0; r < n * n; r++)
-            maxPer = std::max(maxPer, ang->gaunt_off[r + 1] - ang->gaunt_off[r]);
-    const int maxGroups = chunks * ((maxPer + 3) / 4);
+    const int maxGroups = gaunt ? gaunt_ell_groups(n, ang->gaunt_off) : 0;
     const size_t offEllPair = off;
     off = align_up(off + sizeof(unsigned short) * (size_t)(chunks * 64 + 1), 256);
     const size_t offEllOff = off;

@@ -17,6 +17,8 @@
 //     (momopt_init.cpp:221-259).
 #include "angular.h"
 
+#include <algorithm>
+
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -243,6 +245,19 @@ void product_columns(int n, unsigned short *pairs)
     for (int i = 1; i < n; i++)
         for (int j = 1; j <= i; j++)
             pairs[c++] = (unsigned short)((i << 8) | j);
+}
+
+int gaunt_ell_groups(int n, const int *off)
+{
+    int count[528], m = 0;   // n <= 32
+    for (int i = 0; i < n; i++)
+        for (int j = i; j < n; j++)
+            count[m++] = off[i * n + j + 1] - off[i * n + j];
+    std::sort(count, count + m, [](int x, int y) { return x > y; });
+    int groups = 0;
+    for (int p = 0; p < m; p += 64)
+        groups += (count[p] + 3) / 4;
+    return groups;
 }
 
 int build_gaunt_ell(int n, const int *off, const int *idx, const double *val, unsigned short *pair,

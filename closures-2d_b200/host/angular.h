@@ -35,6 +35,7 @@ namespace clb {
 // pair holds 64 and eoff one entry per chunk (+1 for eoff).
 int build_gaunt_ell(int n, const int *off, const int *idx, const double *val, unsigned short *pair,
                     unsigned short *eidx, double *eval, int *eoff, int maxGroups);
+int gaunt_ell_groups(int n, const int *off);   // the number of groups (no allocation)
 constexpr int kEllGroup = 256;   // entries per group
 inline int gaunt_ell_chunks(int n) { return (n * (n + 1) / 2 + 63) / 64; }
 
