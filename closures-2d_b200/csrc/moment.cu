@@ -407,12 +407,20 @@ __global__ void __launch_bounds__(kParThreads, N <= 6 ? 4 : 2) pn_parity_kernel(
     // every cell of the tile and its halo interior: one rule for all of them
     const bool inner = i0 >= 4 && j0 >= 4 && i0 + kTI + 2 <= a.NX - 2 && j0 + kTJ + 2 <= a.NY - 2;
     constexpr int V = (n % 2 == 0) ? 2 : 1;      // doubles per load (rows of even n start 16-byte aligned)
+    // Loads of a row in flight: all of them, in equal parts where the registers
+    // (128 up to order 6, else 255) do not hold them.  On a grid of few tiles
+    // a stage waits for memory once per part (8 loads a part: P4 36 x 74 29.5 us
+    // a step, all 10 of a row 26.3), and a large one has too few bytes in
+    // flight (800 x 800: P4 217 -> 183 us, P6 332 -> 299, P7 623 -> 509, P8 976 -> 894;
+    // P9 in parts of 18 1280 -> 1446).
+    constexpr int kRowLoads = (RW * n + 32 * V - 1) / (32 * V);
+    constexpr int kMaxBatch = N <= 6 ? 20 / V : N <= 8 ? 18 : 8;
+    constexpr int kParts = (kRowLoads + kMaxBatch - 1) / kMaxBatch, kBatch = (kRowLoads + kParts - 1) / kParts;
     if (a.filter)
         __syncthreads();
     for (int r = warp; r < kTI + 4; r += kParThreads / 32) {
         const bool full = r >= 2 && r < kTI + 2;
         const int c0 = full ? 0 : 2, cells = full ? RW : kTJ, gi = i0 - 2 + r;
-        constexpr int kBatch = 8;
         for (int e0 = lane * V; e0 < cells * n; e0 += kBatch * 32 * V) {
             double v[kBatch][V];
 #pragma unroll
