@@ -4,7 +4,7 @@
 //
 // One kernel per RK stage (pn_parity_kernel; for operators without the
 // harmonics' parity structure pn_tile_kernel on the FP64 tensor cores up to 32
-// moments, pn_stage_kernel above): for each interior cell it applies the moment
+// moments, pn_stage_kernel above, also on small grids of any operators): for each interior cell it applies the moment
 // filter to the stencil values as it loads them (moment_update.cpp:23-40
 // scales the interior in place before the ghost copy, so ghost strips that
 // hold interior copies are filtered too and the physical boundary's are not),
@@ -803,8 +803,14 @@ int cl_pn_create(const cl_grid *grid, const cl_pn_setup *setup, const double *si
     cudaMemcpy(p->U, moments, C * n * 8, cudaMemcpyHostToDevice);
     cudaMemcpy(p->V, moments, C * n * 8, cudaMemcpyHostToDevice);
     p->cur = p->U;
-    // operators with the harmonics' parity structure: pn_parity_kernel
-    for (int N = 1; N <= 9; N++)
+    // Operators with the harmonics' parity structure: pn_parity_kernel.  Above
+    // 32 moments a thread's straight-line code is long, and on a small grid one
+    // tile's time is the stage's; there a warp per cell is faster (a step in
+    // us, warp per cell / parity: order 7 1000 cells 37.7 / 39.1, 2000 41.8 /
+    // 39.8; order 8 1000 45.1 / 56.0, 2000 49.9 / 56.2, 2664 58.2 / 56.6; order 9
+    // 1000 54.0 / 70.1, 2000 60.0 / 72.3, 2664 81.0 / 73.0).
+    const bool warpPerCell = n > 32 && (long long)grid->nx * grid->ny <= 48 * (long long)n;
+    for (int N = 1; N <= 9 && !warpPerCell; N++)
         if ((N + 1) * (N + 2) / 2 == p->n && pn_with_order(N, [&](auto O) {
                 constexpr int order = decltype(O)::value;
                 return pn_parity_coefs<order>(setup->ops, p->coef) &&
