@@ -2252,7 +2252,7 @@ __device__ __noinline__ bool phase_a_rows8(const PhaseA x, bool active, unsigned
             load_chunk(c, c);
     bool ok = wait_full(0);
     double cs[QUAD ? 4 : 2][2];
-    if (active && ok) {
+    if (active && __all_sync(0xffffffffu, ok)) {   // the whole warp or none of it
         gemm1(sP, cs);
         weights(sP, cs);
     }
