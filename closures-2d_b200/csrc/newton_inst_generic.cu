@@ -1,4 +1,7 @@
-// newton_inst_generic.cu -- kernel instances with runtime tile counts: mixed-order launches on the fused path and the general contractions.
+// newton_inst_generic.cu -- kernel instances with runtime tile counts: the fused
+// path for moment sets that end within a degree (a caller's own angular tables;
+// whole orders have exact instances), and the general contractions (direct
+// orders 5 and 6, direct PPn order 4).
 #include "newton_kernel.cuh"
 
 namespace clb {

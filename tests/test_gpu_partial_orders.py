@@ -3,9 +3,11 @@ orders), which the instances of whole orders do not fit: the fused kernels with
 runtime tile counts, Mn and PPn, with the Gaunt table and with products.
 
 The vectors are the moments of known multipliers, which the solves must give
-back: the gradient left at the end is at most tol ||u||, and the multipliers'
-error that over the Hessian's smallest eigenvalue (above 1e-3 for these).  The
-two tables sum the same Hessian, so their solves agree as two layouts do.
+back: the stopping test leaves a gradient of at most tol ||u / u_0||, and the
+multipliers' error is that over the Hessian's smallest eigenvalue (above 1e-3
+for these).  The two tables sum the same Hessian, so their solves agree as two
+layouts do (tol = 1e-6 as in the layouts' tests: at 1e-8 the line search of some
+vectors is decided by the last bit of f).
 """
 import ctypes as C
 
@@ -61,13 +63,14 @@ def test_partial_orders(order, n, closure):
     for gaunt in (1, 0):
         a = _Cut(order, n, 2 * order + 8, gaunt)
         u, alpha = _vectors(a, count, closure, order * 100 + n)
-        ctx = cb.Context.for_batches(a, cb.make_options(moment_type=closure, tol=1e-8))
+        ctx = cb.Context.for_batches(a, cb.make_options(moment_type=closure, tol=1e-6))
         ug, ag = u.copy(), cb.isotropic_alpha(n, count, moment_type=closure)
         it, reg, st = ctx.solve_batch(ug, ag)
         ctx.close()
         assert (st == 0).all() and (reg == 0).all()
-        assert np.max(np.abs(ug - u)) <= 1e-7 * np.max(np.abs(u))
-        assert np.max(np.abs(ag - alpha)) < 1e-4
+        unorm = np.linalg.norm(u / u[:, :1], axis=1)
+        assert np.all(np.linalg.norm(ug - u, axis=1) / u[:, 0] <= 1.001e-6 * unorm)
+        assert np.max(np.abs(ag - alpha)) < 1e-3 * np.max(unorm)
         out.append((ug, it))
     assert np.array_equal(out[0][1], out[1][1])
     assert np.max(np.abs(out[0][0] - out[1][0]) / out[1][0][:, :1]) < 1e-10
