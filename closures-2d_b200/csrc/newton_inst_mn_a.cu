@@ -1,4 +1,6 @@
-// newton_inst_mn_a.cu -- Mn instances specialised to the tile counts of orders 1-2 and Gaunt orders 3-4.
+// newton_inst_mn_a.cu -- Mn instances specialised to the tile counts of orders 1-2
+// and Gaunt orders 3-4, and of moment sets of seven or eight (order 3 cut short:
+// 8000 vectors 861 us with runtime counts, 503 with these).
 #include "newton_kernel.cuh"
 
 namespace clb {
@@ -17,6 +19,14 @@ bool newton_run_exact_mn_a(const NewtonArgs &a, int grid, cudaStream_t s, int mo
     }
     if (a.ntExact == 3 && a.nbk == 1) {
         *err = newton_run<1, 3, 0, 3, 1>(a, grid, s, mode, occ);
+        return true;
+    }
+    if (a.ntExact == 4 && a.nbk == 1) {
+        *err = newton_run<1, 4, 0, 4, 1>(a, grid, s, mode, occ);
+        return true;
+    }
+    if (a.ntExact == 5 && a.nbk == 1) {
+        *err = newton_run<1, 5, 0, 5, 1>(a, grid, s, mode, occ);
         return true;
     }
     if (a.ntExact == 4 && a.nbk == 2) {

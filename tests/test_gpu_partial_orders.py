@@ -56,7 +56,7 @@ def _vectors(a, count, closure, seed):
     return (G * a.w) @ a.p, alpha
 
 
-@pytest.mark.parametrize("order,n", [(2, 4), (2, 5), (3, 7), (3, 9), (4, 12), (5, 16), (5, 20), (6, 25)])
+@pytest.mark.parametrize("order,n", [(2, 4), (2, 5), (3, 7), (3, 8), (3, 9), (4, 12), (5, 16), (5, 20), (6, 25)])
 @pytest.mark.parametrize("closure", [cb.CL_MN, cb.CL_PPN])
 def test_partial_orders(order, n, closure):
     count, out = 150, []
