@@ -81,10 +81,12 @@ __device__ __forceinline__ void ldmatrix4(unsigned (&r)[4], unsigned addr)
 // m16n8k16, the k-steps of one output a single chain; db one addition per
 // row), so the gradients do not depend on the tiling, and training, whose
 // first Adam steps divide gradients by their own size, is reproducible to the
-// bit.  The chains set the time: 256 dependent MMAs for 4096 rows.  So the
-// operands, staged with 16-byte asynchronous copies four stages deep, have to
-// arrive faster than that (through scalar loads the four dW took 1810 us a
-// step at 4096 x 512, the column sums 910, dA 164).
+// bit.  A chain of 256 dependent MMAs (4096 rows) or 4096 additions is some 5
+// to 8 us of a layer's 35; the rest is the 64 stages, about 900 cycles each: a
+// wait for the staged operands, a CTA barrier, sixteen-byte copies by every
+// thread, the fragment loads.  The operands come four stages deep (through
+// scalar loads the four dW took 1810 us a step at 4096 x 512, the column sums
+// 910, dA 164).
 // Row strides (ldin, ldz, ldw) are multiples of 8.
 struct BackArgs {
     const __nv_bfloat16 *in;   // [rows][ldin], K columns
@@ -104,7 +106,7 @@ constexpr int kBackSmem = kBackStages * 2 * kBackTile * 2;
 
 // One 64 x 64 tile, eight warps of 32 x 16.  C [M x N] = A . B over kTot: dW
 // (W): A = in^T, B = dZ, both staged as [k][64]; dA: A = dZ, B = W^T, staged as
-// [64][k].  The chains are latency bound, so what a warp issues per stage
+// [64][k].  A stage is latency bound, so what a warp issues in it
 // counts (addresses are fixed before the loop and advance by one stride), and
 // eight warps hide more than four did (a layer's launch 54 us with addresses
 // formed per piece, 35 us with fixed ones, four warps each).

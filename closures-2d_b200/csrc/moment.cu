@@ -385,7 +385,7 @@ __device__ __forceinline__ void static_for(F &&f)
 // registers.  The new moments go through the tile so that the state, read once
 // and written once, moves in whole lines.  Cells are padded to an odd
 // stride: conflict-free for a thread per cell.
-// P6 800 x 800, stages 1 and 2: 154 and 172 us, dense products on the tensor
+// P6 800 x 800, stages 1 and 2: 147 and 167 us, dense products on the tensor
 // cores (pn_tile_kernel) 342 and 440; the state's 290 and 435 MB take 44 and
 // 65 us.  With fewer CTAs per SM and the old state loaded element by element
 // in stage 2 it took 168 and 254.
