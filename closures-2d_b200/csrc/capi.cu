@@ -102,7 +102,7 @@ cudaError_t upload(T **dst, const std::vector<T> &src)
         return e;
     if (!src.empty())
         e = cudaMemcpy(*dst, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice);
-    return e;
+    return e == cudaSuccess ? uploads_arrived() : e;
 }
 
 // Arrays that go up together: one block of device memory and one copy (twenty
@@ -123,6 +123,8 @@ public:
         cudaError_t e = cudaMalloc(block, host_.size());
         if (e == cudaSuccess)
             e = cudaMemcpy(*block, host_.data(), host_.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess)
+            e = uploads_arrived();
         if (e == cudaSuccess)
             for (const auto &p : places_)
                 *p.first = (char *)*block + p.second;
@@ -1487,6 +1489,7 @@ int cl_set_state(cl_ctx *ctx, const double *moments, const double *alpha)
         CUDA_TRY(ctx, cudaMemcpy(ctx->dMom, moments, bytes, cudaMemcpyHostToDevice));
     if (alpha)
         CUDA_TRY(ctx, cudaMemcpy(ctx->dAlpha, alpha, bytes, cudaMemcpyHostToDevice));
+    CUDA_TRY(ctx, uploads_arrived());
     return CL_OK;
 }
 
@@ -2112,6 +2115,7 @@ int cl_set_last_iterations(cl_ctx *ctx, const int *iters)
         return CL_ERR_ARG;
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     CUDA_TRY(ctx, cudaMemcpy(ctx->dIters, iters, (size_t)ctx->C * sizeof(int), cudaMemcpyHostToDevice));
+    CUDA_TRY(ctx, uploads_arrived());
     return CL_OK;
 }
 
@@ -2460,6 +2464,7 @@ int cl_multi_solve_device_start(cl_multi *m, const int *counts, double *const *d
     if (herr[0]) {
         m->err = error_text(herr[0]);
         cudaMemset(m->dErr, 0, sizeof(herr));
+        uploads_arrived();
         return herr[0];
     }
     return CL_OK;

@@ -19,6 +19,7 @@
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
 
+#include "common.cuh"
 #include "tc_gemm.cuh"
 
 #include <algorithm>
@@ -803,6 +804,7 @@ static int tc_error(cl_mlp *m)
         return CL_ERR_CUDA;
     if (h != 0) {
         cudaMemset(m->tcErr, 0, sizeof(int));
+        clb::uploads_arrived();
         m->err = "tensor-memory GEMM: a bounded wait timed out";
         return CL_ERR_TIMEOUT;
     }
@@ -866,6 +868,7 @@ int cl_mlp_create(int n, int width, int moment_type, double delta_ppn, unsigned 
     m->hstd.assign(n, 1.0f);
     cudaMemcpy(m->mean, m->hmean.data(), n * 4, cudaMemcpyHostToDevice);
     cudaMemcpy(m->stdv, m->hstd.data(), n * 4, cudaMemcpyHostToDevice);
+    clb::uploads_arrived();
     mlp_sync_weights(m);
     cudaStreamSynchronize(m->stream);
     *out = m;
@@ -914,7 +917,7 @@ int cl_mlp_set_output_scaling(cl_mlp *m, const float *mean, const float *stdv)
     m->hstd.assign(stdv, stdv + m->n);
     cudaMemcpy(m->mean, mean, m->n * 4, cudaMemcpyHostToDevice);
     cudaMemcpy(m->stdv, stdv, m->n * 4, cudaMemcpyHostToDevice);
-    return CL_OK;
+    return clb::uploads_arrived() == cudaSuccess ? CL_OK : CL_ERR_CUDA;
 }
 
 // Adam training on pairs (u, alpha) held on the device ([count x n] FP64).
@@ -1160,6 +1163,7 @@ int cl_mlp_loss_and_grads(cl_mlp *m, const double *u, const double *alpha, int r
     cudaMalloc(&ba, (size_t)rows * n * 8);
     cudaMemcpy(bu, u, (size_t)rows * n * 8, cudaMemcpyHostToDevice);
     cudaMemcpy(ba, alpha, (size_t)rows * n * 8, cudaMemcpyHostToDevice);
+    clb::uploads_arrived();
     prep_kernel<<<blocks((size_t)rows * n), 256, 0, m->stream>>>(bu, ba, nullptr, rows, n, round8(n), m->momentType,
                                                                 m->mean, m->stdv, m->X, m->T);
     cudaError_t e = mlp_forward(m, rows);
@@ -1214,6 +1218,7 @@ int cl_mlp_set_params(cl_mlp *m, float *const *W, float *const *b)
         if (b && b[l])
             cudaMemcpy(m->b[l], b[l], m->dims[l + 1] * 4, cudaMemcpyHostToDevice);
     }
+    clb::uploads_arrived();
     mlp_sync_weights(m);
     return cudaStreamSynchronize(m->stream) == cudaSuccess ? CL_OK : CL_ERR_CUDA;
 }
