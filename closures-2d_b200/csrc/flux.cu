@@ -143,7 +143,8 @@ __device__ __forceinline__ void flux_update(const FluxArgs &f, const double (&ac
 // flux_project_kernel projects them, every cell's sum over the directions in
 // the order it has here.  Per stage: 50 x 50 M2, Q = 20 (16 tiles) 165 us
 // before; a whole RK2 step went from 467 to 274 us, 36 x 74 M3, Q = 30 (15
-// tiles) from 854 to 415 us, PP3 from 1487 to 846 us.
+// tiles) from 854 to 415 us, PP3 from 1487 to 846 us, 200 x 200 M4 (169 tiles
+// on 148 SMs) from 3726 to 3547 us.
 template <int PAIR, int SPLIT>
 __global__ void __launch_bounds__(kFluxThreads, 1) flux_kernel(const __grid_constant__ FluxArgs f)
 {
@@ -634,12 +635,12 @@ cudaError_t prepare_flux(const FluxArgs &f)
 // the number that takes the fewest chunk times.  A wave of shares costs its
 // chunks and one more for the CTA's start (staging of alpha); the pass over F
 // 0.08 per chunk of the loop, and as much again per wave of tiles.  Against
-// times of 1 to 57 shares on 1 to 147 tiles at 4 to 144 chunks, the choice is
+// times of 1 to 25 shares on 1 to 296 tiles at 4 to 144 chunks, the choice is
 // within 1 % of the fastest on average and never slower than the whole loop:
-// 16 tiles at 25 chunks 142 -> 42 us, 74 at 57 310 -> 192, 80 at 100 591 -> 427;
-// whole at 120 tiles and 100 chunks (563 us; 6 shares, which a pass over F taken
-// as half a chunk per wave chose, 591), 112 and 57 (309; 323), 128 and 144 (758;
-// 814).
+// 16 tiles at 25 chunks 142 -> 42 us, 74 at 57 310 -> 192, 169 at 57 609 ->
+// 448; whole at 120 tiles and 100 chunks (563 us; 6 shares, which a pass over F
+// taken as half a chunk per wave chose, 591), 112 and 57 (309; 323), 256 and
+// 100 (1116; 1140).
 static int flux_shares(int tiles, int chunks, int sms)
 {
     auto waves = [&](int s) { return (tiles * s + sms - 1) / sms; };
@@ -662,10 +663,14 @@ size_t flux_split_doubles(const FluxArgs &f)
 {
     // Splitting pays while the tiles fill less than about two waves (the
     // chunk times saved are then a sizeable share), and F has to stay small.
-    const int tiles = f.tilesX * f.tilesY, rest = tiles % f.sms, chunks = flux_chunks(f);
-    if (tiles > 2 * f.sms || rest == 0 || flux_shares(rest, chunks, f.sms) == 1)
+    // A step launches the whole grid, cl_step_host two waves one by one.
+    const int tiles = f.tilesX * f.tilesY, chunks = flux_chunks(f);
+    if (tiles > 2 * f.sms)
         return 0;
-    const size_t doubles = (size_t)rest * chunks * kQ * IC;
+    int most = flux_shares(tiles, chunks, f.sms) > 1 ? tiles : 0;
+    if (most == 0 && tiles == 2 * f.sms && flux_shares(f.sms, chunks, f.sms) > 1)
+        most = f.sms;
+    const size_t doubles = (size_t)most * chunks * kQ * IC;
     return doubles * sizeof(double) <= kSplitBytes ? doubles : 0;
 }
 
@@ -675,24 +680,12 @@ cudaError_t launch_flux_tiles(const FluxArgs &f, int first, int count, cudaStrea
         return cudaErrorInvalidValue;
     FluxArgs g = f;
     g.tileBase = first;
-    // a whole wave of tiles takes its loops whole, those left over share them
-    // out: 169 tiles at 57 chunks 396 us (all shared 448, all whole 610), 222 at 25
-    // 239 (255; 279), 240 at 100 1052 (1138; 1179), and F holds the rest only
-    const int chunks = flux_chunks(f), rest = count % f.sms;
-    int shares = (f.F && rest > 0) ? flux_shares(rest, chunks, f.sms) : 1;
-    if ((size_t)rest * chunks * kQ * IC > f.doublesF)
+    int shares = f.F ? flux_shares(count, flux_chunks(f), f.sms) : 1;
+    if ((size_t)count * flux_chunks(f) * kQ * IC > f.doublesF)
         shares = 1;
-    if (const int whole = shares > 1 ? count - rest : count) {
-        if (g.paired)
-            flux_kernel<1, 0><<<whole, kFluxThreads, g.smemBytes, stream>>>(g);
-        else
-            flux_kernel<0, 0><<<whole, kFluxThreads, g.smemBytes, stream>>>(g);
-        g.tileBase += whole;
-        *kernels += 1;
-    }
     if (shares > 1) {
-        const dim3 grid((unsigned)rest, (unsigned)shares);
-        const int pgrid = rest * (IC / kProjCells), psmem = project_smem(g);
+        const dim3 grid((unsigned)count, (unsigned)shares);
+        const int pgrid = count * (IC / kProjCells), psmem = project_smem(g);
         if (g.paired) {
             flux_kernel<1, 1><<<grid, kFluxThreads, g.smemBytes, stream>>>(g);
             flux_project_kernel<1><<<pgrid, kProjWarps * 32, psmem, stream>>>(g);
@@ -701,7 +694,13 @@ cudaError_t launch_flux_tiles(const FluxArgs &f, int first, int count, cudaStrea
             flux_project_kernel<0><<<pgrid, kProjWarps * 32, psmem, stream>>>(g);
         }
         *kernels += 2;
+        return cudaGetLastError();
     }
+    if (g.paired)
+        flux_kernel<1, 0><<<count, kFluxThreads, g.smemBytes, stream>>>(g);
+    else
+        flux_kernel<0, 0><<<count, kFluxThreads, g.smemBytes, stream>>>(g);
+    *kernels += 1;
     return cudaGetLastError();
 }
 
