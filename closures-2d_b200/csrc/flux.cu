@@ -632,24 +632,25 @@ cudaError_t prepare_flux(const FluxArgs &f)
 }
 
 // Shares of the direction loop for `tiles` tiles on `sms` SMs (one CTA each):
-// the number that takes the fewest chunk times.  A wave of shares costs its
-// chunks and one more for the CTA's start (staging of alpha); the pass over F
-// 0.08 per chunk of the loop, and as much again per wave of tiles.  Against
-// times of 1 to 25 shares on 1 to 296 tiles at 4 to 144 chunks, the choice is
-// within 1 % of the fastest on average and never slower than the whole loop:
-// 16 tiles at 25 chunks 142 -> 42 us, 74 at 57 310 -> 192, 169 at 57 609 ->
-// 448; whole at 120 tiles and 100 chunks (563 us; 6 shares, which a pass over F
-// taken as half a chunk per wave chose, 591), 112 and 57 (309; 323), 256 and
-// 100 (1116; 1140).
+// 1, or the number that takes the fewest chunk times, a CTA's start (staging
+// of alpha) counted as one chunk and the pass over F as half a chunk per wave
+// of tiles.  Times per stage, whole / shared: 16 tiles at 25 chunks 142 / 42 us,
+// 74 at 57 310 / 192, 80 at 100 591 / 431, 169 at 57 610 / 472, 222 at 100 1179 /
+// 980.  The pass really costs 0.08 chunks per chunk and wave, so with every tile
+// running, whole loops would be up to 6 % faster in places (120 tiles at 100
+// chunks 530 / 556 us, 112 at 57 309 / 321) and more shares up to 6 % elsewhere
+// (169 at 57: 6 shares 447 us, 3 472); but where tiles are uniform and skip their
+// loops, the few that run have to fill the SMs (half of those 120 uniform 531 /
+// 337 us, three quarters 530 / 247), and a rule on all tiles running took 265 us
+// instead of 249 on 169 tiles half uniform.
 static int flux_shares(int tiles, int chunks, int sms)
 {
     auto waves = [&](int s) { return (tiles * s + sms - 1) / sms; };
     int best = 1;
     double cost = waves(1) * (chunks + 1.0);
     for (int s = 2; s <= chunks && s <= 64; s++) {
-        const double c =
-            waves(s) * ((chunks + s - 1) / s + 1.0) + 0.5 + 0.08 * chunks * (1.0 + (double)tiles / sms);
-        if (c < cost) {
+        const double c = waves(s) * ((chunks + s - 1) / s + 1.0) + 1.5 + 0.5 * tiles / sms;
+        if (c < 0.95 * cost) {
             cost = c;
             best = s;
         }
@@ -663,6 +664,10 @@ size_t flux_split_doubles(const FluxArgs &f)
 {
     // Splitting pays while the tiles fill less than about two waves (the
     // chunk times saved are then a sizeable share), and F has to stay small.
+    // (Of more than a wave, a whole one unshared and only the rest shared is
+    // faster where every tile runs -- 200 x 200 M4 2.79 ms a step against 2.97 --
+    // but not where uniform tiles skip their loops and the others have to be
+    // spread: a 200 x 200 M6 pulse 1.97 ms against 1.76.)
     // A step launches the whole grid, cl_step_host two waves one by one.
     const int tiles = f.tilesX * f.tilesY, chunks = flux_chunks(f);
     if (tiles > 2 * f.sms)

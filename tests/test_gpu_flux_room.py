@@ -46,3 +46,36 @@ def test_reserved_memory(nx, ny, reserved):
         assert used < buffer or used <= 2 * MIB
     ctx.step(1e-3, 0.1, 0.1)
     ctx.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(16 * 5, 16 * 30), (16 * 13 - 3, 16 * 13 - 9), (16 * 8, 16 * 37), (16, 16 * 149)])
+@pytest.mark.parametrize("contraction", [cb.CL_CONTRACT_PAIRS, cb.CL_CONTRACT_SINGLE])
+def test_more_than_a_wave(nx, ny, contraction):
+    """Grids of more than a wave of tiles (150, 169, 296, 149): every tile has the
+    result of the same cells of a grid of few tiles, whose shares are others."""
+    a = cb.Angular(2, 20, 0)
+
+    def step(x0, y0, cells_x, cells_y):
+        # the state of cell (i, j) of the whole grid, ghosts included, from i and j alone
+        i, j = np.meshgrid(np.arange(cells_x + 4) + x0, np.arange(cells_y + 4) + y0, indexing="ij")
+        m = np.zeros(i.shape + (a.n,))
+        m[..., 0] = 1.5 + np.sin(0.37 * i) * np.cos(0.21 * j)
+        for k in range(1, a.n):
+            m[..., k] = 0.1 * np.sin(0.13 * k * i + 0.29 * j)
+        flat = m.reshape(-1, a.n)
+        cells = len(flat)
+        grid = cb.cl_grid(cells_x, cells_y, 2, 0, 0.0, 0.0, 2.0)
+        ctx = cb.Context(grid, cb.make_options(contraction=contraction), a, np.ones(cells), 0.5 * np.ones(cells), flat,
+                         cb.isotropic_alpha(a.n, cells))
+        ctx.step_timed(1e-2, 0.1, 0.1)
+        out = ctx.get_state()[0]
+        ctx.close()
+        return out
+
+    whole = step(0, 0, nx, ny)
+    # a step reaches four cells (two stages of two): the last tile and its
+    # neighbourhood, cut out where the cut is farther away than that
+    cx, cy = min(nx, 40), min(ny, 40)
+    part = step(nx - cx, ny - cy, cx, cy)
+    ix, iy = 2 + (8 if cx < nx else 0), 2 + (8 if cy < ny else 0)
+    assert np.array_equal(part[ix:-2, iy:-2], whole[nx - cx:][ix:-2, (ny - cy) + iy:-2])
