@@ -22,6 +22,7 @@
 #include "flux.cuh"
 #include "newton.cuh"
 #include "readback.h"
+#include "uploads.h"
 
 using namespace clb;
 
@@ -1489,7 +1490,7 @@ int cl_set_state(cl_ctx *ctx, const double *moments, const double *alpha)
         CUDA_TRY(ctx, cudaMemcpy(ctx->dMom, moments, bytes, cudaMemcpyHostToDevice));
     if (alpha)
         CUDA_TRY(ctx, cudaMemcpy(ctx->dAlpha, alpha, bytes, cudaMemcpyHostToDevice));
-    CUDA_TRY(ctx, uploads_arrived());
+    CUDA_TRY(ctx, order_after_uploads(ctx->stream));
     return CL_OK;
 }
 
@@ -2115,7 +2116,7 @@ int cl_set_last_iterations(cl_ctx *ctx, const int *iters)
         return CL_ERR_ARG;
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     CUDA_TRY(ctx, cudaMemcpy(ctx->dIters, iters, (size_t)ctx->C * sizeof(int), cudaMemcpyHostToDevice));
-    CUDA_TRY(ctx, uploads_arrived());
+    CUDA_TRY(ctx, order_after_uploads(ctx->stream));
     return CL_OK;
 }
 

@@ -10,11 +10,6 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kMaxN = 32;            // moments per cell handled by one warp (order <= 6)
 constexpr int kNumReg = 5;
 
-// Waits for the copies and fills made on the legacy stream.  cudaMemcpy from
-// pageable memory returns when the source has been read, before the last bytes
-// have arrived, and the library's own streams do not wait for the legacy one.
-inline cudaError_t uploads_arrived() { return cudaStreamSynchronize(cudaStreamLegacy); }
-
 // Sets a kernel's dynamic shared-memory limit on the current device to `bytes`
 // if it is lower.  Never lowers it: solvers of different orders and tables
 // share kernel instances, each with a plan of its own size, and a launch above

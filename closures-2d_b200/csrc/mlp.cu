@@ -19,8 +19,8 @@
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
 
-#include "common.cuh"
 #include "tc_gemm.cuh"
+#include "uploads.h"
 
 #include <algorithm>
 #include <cmath>
@@ -1163,7 +1163,7 @@ int cl_mlp_loss_and_grads(cl_mlp *m, const double *u, const double *alpha, int r
     cudaMalloc(&ba, (size_t)rows * n * 8);
     cudaMemcpy(bu, u, (size_t)rows * n * 8, cudaMemcpyHostToDevice);
     cudaMemcpy(ba, alpha, (size_t)rows * n * 8, cudaMemcpyHostToDevice);
-    clb::uploads_arrived();
+    clb::order_after_uploads(m->stream);
     prep_kernel<<<blocks((size_t)rows * n), 256, 0, m->stream>>>(bu, ba, nullptr, rows, n, round8(n), m->momentType,
                                                                 m->mean, m->stdv, m->X, m->T);
     cudaError_t e = mlp_forward(m, rows);

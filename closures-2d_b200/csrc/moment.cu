@@ -26,6 +26,7 @@
 #include "common.cuh"
 #include "flux.cuh"
 #include "readback.h"
+#include "uploads.h"
 
 using namespace clb;
 
@@ -981,7 +982,7 @@ int cl_pn_set_state(cl_pn *p, const double *moments)
         return CL_ERR_ARG;
     PN_TRY(p, cudaStreamSynchronize(p->stream));
     PN_TRY(p, cudaMemcpy(p->U, moments, (size_t)p->C * p->n * 8, cudaMemcpyHostToDevice));
-    PN_TRY(p, uploads_arrived());
+    PN_TRY(p, order_after_uploads(p->stream));
     // the second buffer needs the ghost strips; the device copy is cheaper
     // than a second upload
     PN_TRY(p, cudaMemcpyAsync(p->V, p->U, (size_t)p->C * p->n * 8, cudaMemcpyDeviceToDevice, p->stream));
